@@ -364,7 +364,8 @@ typedef enum sc_knn_precision { SC_KNN_FP32 = 0, SC_KNN_BF16 = 1, SC_KNN_FP8 = 2
 typedef struct sc_knn_opts {
     int32_t sigma;        /* sc_knn_sigma; median = reference (neighborhood/mod.rs:105-124, :480-499) */
     int32_t sym;          /* sc_knn_sym;   lower_id = reference (neighborhood/mod.rs:138-163)         */
-    int32_t precision;    /* sc_knn_precision of the candidate distances: BF16 or FP8 e4m3 on the
+    int32_t precision;    /* sc_knn_precision of the candidate distances: 16-bit (BF16; f16, which
+                             rounds finer, where the points' range allows it) or FP8 e4m3 on the
                              tensor cores (norm-expanded contraction, FP32 accumulation), or FP32
                              on the CUDA cores (exact differences, the re-rank's arithmetic)       */
     int32_t rerank_factor;/* candidates kept per row before the exact FP32 re-rank = factor * (k+1)  */

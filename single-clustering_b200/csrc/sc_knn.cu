@@ -1,7 +1,9 @@
 // sc_knn.cu — Gaussian kNN graph builder (src/neighborhood/mod.rs) on sm_100a.
 //
 // 1. k_knn_prep       X (f32) -> A = [-2x, 1, 1, 0..] and B = [x, |x|^2 hi, |x|^2 lo, 0..]
-//                     in BF16, KA = 32 (D <= 30) or 64 (D <= 62) columns.
+//                     in 16 bits, KA = 32 (D <= 30) or 64 (D <= 62) columns: f16,
+//                     scaled by a power of two, where the points' range allows it,
+//                     BF16 otherwise (f16_exp).
 //                     A . B = |c|^2 - 2 q.c = |q - c|^2 - |q|^2: the row-constant
 //                     |q|^2 does not change a row's ranking, so the contraction
 //                     yields ranking scores directly.
@@ -17,11 +19,12 @@
 //                     queries (two M = 128 tiles) stays in shared memory; every
 //                     128-candidate tile of B streams in by TMA (no multicast)
 //                     through a STAGES-deep ring; one thread issues
-//                     tcgen05.mma (M=128, N=128, K=16, BF16 -> FP32) into a
+//                     tcgen05.mma (M=128, N=128, K=16, 16 bit -> FP32) into a
 //                     double-buffered TMEM accumulator (2 x 2 x 128 columns);
-//                     8 epilogue warps read it with tcgen05.ld and keep, per
-//                     query, the R best scores in shared memory (a candidate is
-//                     rejected with one compare against the row's worst kept).
+//                     16 epilogue warps read it with tcgen05.ld and keep scores
+//                     in shared memory. A first scan keeps minima that bound each
+//                     query's (k+1)-th distance, a second one starts from that
+//                     bound and keeps each (query, half)'s 32 best candidates.
 // 3. k_knn_rerank     exact FP32 distances sum (q_d - c_d)^2 of the R candidates
 //                     (no norm expansion, so no cancellation), sorted by
 //                     (distance, self first, index); the first k+1 are kept.
@@ -35,6 +38,7 @@
 // returns; the host turns the status into SC_E_TIMEOUT.
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_fp8.h>
 #include <cudaTypedefs.h>
 
@@ -119,12 +123,14 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
     return d;
 }
 
-// Instruction descriptor, kind::f16: D f32, A/B bf16, both K-major, N = 128, M = 128.
-__host__ __device__ constexpr uint32_t idesc_bf16_128x128() {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TILE >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
+// Instruction descriptor, kind::f16: D f32, A and B both f16 (format 0) or both
+// bf16 (format 1), both K-major, N = 128, M = 128.
+__host__ __device__ constexpr uint32_t idesc_16bit_128x128(bool f16) {
+    return (1u << 4) | (f16 ? 0u : (1u << 7) | (1u << 10)) | ((uint32_t)(TILE >> 3) << 17) |
+           ((uint32_t)(TILE >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+__device__ __forceinline__ void mma_16bit(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -154,102 +160,215 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                  : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-    uint32_t r[32];
+// 64 accumulator columns of this lane's row. The wait stands in the same
+// statement, so no use of the values can be moved before it.
+__device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&v)[64]) {
+    uint32_t r[64];
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        "tcgen05.ld.sync.aligned.32x32b.x64.b32 {"
+        "%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,"
+        "%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,"
+        "%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%64];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
-          "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
-          "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]),
+          "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]),
+          "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]),
+          "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]),
+          "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
+        : "r"(taddr)
+        : "memory");
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// Insert (v, idx) into a query's candidate slots over its current worst slot and
-// return the new worst (value, slot). Kept out of line: it is the rare path,
-// and inlining it into the unrolled filter loop overflows the instruction cache.
-struct Worst {
-    float thr;
-    int slot;
+// A (query, half)'s kept candidates: RCAND slots of shared memory, filled in
+// order; a full row replaces its worst. The search for the worst is kept out of
+// line: inlined into the unrolled filter it overflows the instruction cache.
+struct Kept {
+    float thr;     // scores at or above it are not candidates
+    uint32_t off;  // the slot the next candidate goes to
 };
+constexpr uint32_t SLOT_STRIDE = QT * HALVES * TILE;  // (tile, half, row) owners: one column per owner
 
-// A chunk whose candidates fall in at most this many of a warp's 32 rows is
-// processed by the whole warp, row by row; denser chunks by each lane alone.
-constexpr int COOP_ROWS = 8;
-
-template <int R>
-__device__ __noinline__ Worst cand_insert(float* cs, uint32_t* ci, int qrow, int slot, float v, uint32_t idx) {
-    constexpr int S = QT * HALVES * TILE;
-    cs[slot * S + qrow] = v;
-    ci[slot * S + qrow] = idx;
-    Worst w{-INFINITY, 0};
-    for (int s = 0; s < R; ++s) {
-        const float x = cs[s * S + qrow];
-        if (x > w.thr) {
-            w.thr = x;
-            w.slot = s;
+// The worst of a full row (highest score, lowest slot on ties).
+__device__ __noinline__ Kept row_worst(const float* cs, uint32_t owner) {
+    float worst = -INFINITY;
+    uint32_t at = owner;
+#pragma unroll 8
+    for (int s = 0; s < RCAND; ++s) {
+        const float x = cs[s * SLOT_STRIDE + owner];
+        if (x > worst) {
+            worst = x;
+            at = s * SLOT_STRIDE + owner;
         }
     }
-    return w;
+    return Kept{worst, at};
+}
+
+// A bounding scan keeps scores alone: BOUND_SLOTS per (query, half), cut back to
+// the BOUND_KEEP smallest (ascending, in the first slots) when a row of the warp
+// is nearly full. Returns the largest kept of a row that holds BOUND_KEEP or
+// more, +inf for one that holds fewer. Every lane of the warp calls it.
+constexpr int BOUND_KEEP = 16;
+constexpr int BOUND_SLOTS = 2 * RCAND;  // the candidates' scores and ids in one
+__device__ __noinline__ float bound_cut(float* cs, uint32_t owner, uint32_t cnt) {
+    float best[BOUND_KEEP];
+#pragma unroll
+    for (int i = 0; i < BOUND_KEEP; ++i) best[i] = INFINITY;
+#pragma unroll 1
+    for (uint32_t s = 0; s < (uint32_t)BOUND_SLOTS; ++s) {
+        float v = s < cnt ? cs[s * SLOT_STRIDE + owner] : INFINITY;
+        if (!__any_sync(0xFFFFFFFFu, v < best[BOUND_KEEP - 1])) continue;
+#pragma unroll
+        for (int i = 0; i < BOUND_KEEP; ++i) {  // v takes its place, the rest move up by one
+            const float lo = fminf(best[i], v);
+            v = fmaxf(best[i], v);
+            best[i] = lo;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < BOUND_KEEP; ++i) cs[i * SLOT_STRIDE + owner] = best[i];
+    return best[BOUND_KEEP - 1];
 }
 
 // ------------------------------------------------------------ prep
-template <int KA>
-__global__ void k_knn_prep(const float* __restrict__ X, uint64_t n, uint32_t d, __nv_bfloat16* A,
-                           __nv_bfloat16* B) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const float* x = X + i * d;
-        float nrm = 0.0f;
-        for (uint32_t j = 0; j < d; ++j) nrm = __fmaf_rn(x[j], x[j], nrm);
-        __nv_bfloat16* a = A + i * KA;
-        __nv_bfloat16* b = B + i * KA;
-        for (uint32_t j = 0; j < d; ++j) {
-            __nv_bfloat16 xb = __float2bfloat16_rn(x[j]);
-            a[j] = __float2bfloat16_rn(-2.0f * __bfloat162float(xb));
-            b[j] = xb;
-        }
-        __nv_bfloat16 hi = __float2bfloat16_rn(nrm);
-        __nv_bfloat16 lo = __float2bfloat16_rn(nrm - __bfloat162float(hi));
-        a[d] = __float2bfloat16_rn(1.0f);
-        a[d + 1] = __float2bfloat16_rn(1.0f);
-        b[d] = hi;
-        b[d + 1] = lo;
-        for (uint32_t j = d + 2; j < (uint32_t)KA; ++j) {
-            a[j] = __float2bfloat16_rn(0.0f);
-            b[j] = __float2bfloat16_rn(0.0f);
-        }
-    }
+// What the operand kernels know of the point set (device words, zeroed first;
+// non-negative floats order like their bit patterns, so integer atomics find
+// the largest).
+struct KnnScale {
+    unsigned maxabs;   // max |x_ij|
+    unsigned maxnorm;  // max |x_i|^2
+    unsigned minrow;   // ~bits of the smallest max_j |x_ij| of a point that is not all zeros (atomicMax of ~bits)
+    unsigned rho;      // max |x_i - x^_i| / |x_i|, x^ the 16-bit operand (k_knn_prep)
+};
+
+// The 16-bit operands are f16 where the points' range allows it, BF16 otherwise:
+// both run at the same rate, f16 rounds 8 times finer (11 significant bits), so
+// the score bounds that the scans start from are that much tighter and fewer
+// scores pass them. f16 needs a common power-of-two scale that brings the
+// largest coordinate to [64, 128); a point whose largest coordinate is then
+// 2^-6 or more keeps |x - x^| <= (2^-11 + 2^-16) |x| although its small
+// coordinates may fall below f16's normal range. Points of a wider range (an
+// outlier 2^12 times the rest) keep BF16's relative rounding. Returns the
+// scale's exponent, or INT32_MIN for BF16.
+__device__ __forceinline__ int f16_exp(const KnnScale* k) {
+    const float ma = __uint_as_float(k->maxabs), mr = __uint_as_float(~k->minrow);
+    if (!(ma > 0x1.0p-40f) || !(ma < 0x1.0p40f) || k->minrow == 0u || !(mr * 0x1.0p12f >= ma)) return INT32_MIN;
+    return 6 - ilogbf(ma);
 }
 
-// max |x_ik| and max |x_i|^2 over the point set (non-negative floats order like
-// their bit patterns, so an integer atomicMax finds them).
-__global__ void k_knn_scales(const float* __restrict__ X, uint64_t n, uint32_t d, unsigned* maxabs,
-                             unsigned* maxnorm) {
-    float ma = 0.0f, mn = 0.0f;
+// Rows of X as the contraction's operands, a warp per row (lane j holds columns
+// j and j + 32): A = [-2 x^, c1, c2, 0..], B = [x^, hi, lo, 0..], with c1 hi +
+// c2 lo = |x|^2 to 22 bits in f16 (c1 = 32 and c2 = 2^-5 keep both terms in its
+// range) and to 16 bits in BF16 (c1 = c2 = 1). Also each row's norm and the
+// norm of its rounding error, both rounded up: with the largest relative one
+// (rho) they bound every score's error (score_margin).
+template <int KA>
+__global__ void k_knn_prep(const float* __restrict__ X, uint64_t n, uint32_t d, KnnScale* sc, uint16_t* A,
+                           uint16_t* B, float* __restrict__ nx, float* __restrict__ rx) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const int e = f16_exp(sc);
+    const bool f16 = e != INT32_MIN;
+    const float s = f16 ? ldexpf(1.0f, e) : 1.0f, inv = f16 ? ldexpf(1.0f, -e) : 1.0f;
+    float rho = 0.0f;
+    for (uint64_t i = warp; i < n; i += nwarps) {
+        float x[KA / 32], nrm = 0.0f, res = 0.0f;
+        uint16_t a[KA / 32], b[KA / 32];
+#pragma unroll
+        for (int t = 0; t < KA / 32; ++t) {
+            const uint32_t j = lane + 32 * t;
+            x[t] = j < d ? X[i * d + j] : 0.0f;
+            nrm = __fmaf_rn(x[t], x[t], nrm);
+            float back;  // the operand's value, in the points' units
+            if (f16) {
+                const __half h = __float2half_rn(x[t] * s);
+                back = __half2float(h) * inv;
+                b[t] = __half_as_ushort(h);
+                a[t] = __half_as_ushort(__float2half_rn(-2.0f * __half2float(h)));
+            } else {
+                const __nv_bfloat16 h = __float2bfloat16_rn(x[t]);
+                back = __bfloat162float(h);
+                b[t] = __bfloat16_as_ushort(h);
+                a[t] = __bfloat16_as_ushort(__float2bfloat16_rn(-2.0f * back));
+            }
+            const float df = x[t] - back;
+            res = __fmaf_rn(df, df, res);
+        }
+        for (int o = 16; o; o >>= 1) {
+            nrm += __shfl_xor_sync(FULL, nrm, o);
+            res += __shfl_xor_sync(FULL, res, o);
+        }
+        uint16_t hi, lo, c1, c2;
+        if (f16) {
+            const float v = nrm * s * s * (1.0f / 32.0f);
+            const __half h = __float2half_rn(v);
+            hi = __half_as_ushort(h);
+            lo = __half_as_ushort(__float2half_rn((v - __half2float(h)) * 1024.0f));
+            c1 = __half_as_ushort(__float2half_rn(32.0f));
+            c2 = __half_as_ushort(__float2half_rn(0x1.0p-5f));
+        } else {
+            const __nv_bfloat16 h = __float2bfloat16_rn(nrm);
+            hi = __bfloat16_as_ushort(h);
+            lo = __bfloat16_as_ushort(__float2bfloat16_rn(nrm - __bfloat162float(h)));
+            c1 = c2 = __bfloat16_as_ushort(__float2bfloat16_rn(1.0f));
+        }
+#pragma unroll
+        for (int t = 0; t < KA / 32; ++t) {
+            const uint32_t j = lane + 32 * t;
+            if (j == d) {
+                a[t] = c1;
+                b[t] = hi;
+            } else if (j == d + 1) {
+                a[t] = c2;
+                b[t] = lo;
+            } else if (j > d + 1) {
+                a[t] = b[t] = 0;
+            }
+            A[i * KA + j] = a[t];
+            B[i * KA + j] = b[t];
+        }
+        // FP32 sums of squares of at most 62 terms: 2^-17 covers their rounding
+        const float up = 1.0f + 0x1.0p-16f;
+        if (lane == 0) {
+            nx[i] = sqrtf(nrm) * up;
+            rx[i] = sqrtf(res) * up;
+        }
+        if (nrm > 0.0f) rho = fmaxf(rho, sqrtf(res) / sqrtf(nrm) * (up * up));
+    }
+    if (lane == 0 && rho > 0.0f) atomicMax(&sc->rho, __float_as_uint(rho));
+}
+
+// The point set's ranges (KnnScale).
+__global__ void k_knn_scales(const float* __restrict__ X, uint64_t n, uint32_t d, KnnScale* sc) {
+    float ma = 0.0f, mn = 0.0f, mr = INFINITY;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const float* x = X + i * d;
-        float nrm = 0.0f;
+        float nrm = 0.0f, row = 0.0f;
         for (uint32_t j = 0; j < d; ++j) {
-            ma = fmaxf(ma, fabsf(x[j]));
+            row = fmaxf(row, fabsf(x[j]));
             nrm = __fmaf_rn(x[j], x[j], nrm);
         }
+        ma = fmaxf(ma, row);
+        if (row > 0.0f) mr = fminf(mr, row);
         mn = fmaxf(mn, nrm);
     }
     for (int o = 16; o; o >>= 1) {
         ma = fmaxf(ma, __shfl_xor_sync(0xFFFFFFFFu, ma, o));
         mn = fmaxf(mn, __shfl_xor_sync(0xFFFFFFFFu, mn, o));
+        mr = fminf(mr, __shfl_xor_sync(0xFFFFFFFFu, mr, o));
     }
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(maxabs, __float_as_uint(ma));
-        atomicMax(maxnorm, __float_as_uint(mn));
+        atomicMax(&sc->maxabs, __float_as_uint(ma));
+        atomicMax(&sc->maxnorm, __float_as_uint(mn));
+        if (mr < INFINITY) atomicMax(&sc->minrow, ~__float_as_uint(mr));
     }
 }
 
@@ -262,10 +381,10 @@ __device__ __forceinline__ float from_e4m3(uint8_t b) {
 }
 
 // FP8 operands (64 one-byte columns, D <= 61): see the file comment.
-__global__ void k_knn_prep_f8(const float* __restrict__ X, uint64_t n, uint32_t d, const unsigned* __restrict__ maxabs,
-                              const unsigned* __restrict__ maxnorm, uint8_t* A, uint8_t* B) {
+__global__ void k_knn_prep_f8(const float* __restrict__ X, uint64_t n, uint32_t d, const KnnScale* __restrict__ sc,
+                              uint8_t* A, uint8_t* B) {
     constexpr uint32_t W = 64;
-    const float ma = __uint_as_float(*maxabs), mn = __uint_as_float(*maxnorm);
+    const float ma = __uint_as_float(sc->maxabs), mn = __uint_as_float(sc->maxnorm);
     const float S = ma > 0.0f ? ma / 256.0f : 1.0f;
     const float Sn = mn > 0.0f ? mn / 256.0f : 1.0f;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
@@ -305,7 +424,7 @@ __global__ void k_knn_prep_f8(const float* __restrict__ X, uint64_t n, uint32_t 
 }
 
 // ------------------------------------------------------------ tensor-core candidate search
-template <int KA, int R = RCAND>
+template <int KA>
 struct KnnSmem {
     static constexpr int STAGES = stages_for<KA>();
     static constexpr uint32_t TILE_BYTES = TILE * KA * 2;
@@ -313,14 +432,13 @@ struct KnnSmem {
     static constexpr uint32_t A_OFF = 0;
     static constexpr uint32_t B_OFF = A_OFF + QT * TILE_BYTES;
     static constexpr uint32_t C_OFF = B_OFF + STAGES * TILE_BYTES;               // candidate scores
-    static constexpr uint32_t I_OFF = C_OFF + R * SLOTS * 4;                     // candidate ids
-    static constexpr uint32_t BAR_OFF = I_OFF + R * SLOTS * 4;
+    static constexpr uint32_t I_OFF = C_OFF + RCAND * SLOTS * 4;                 // candidate ids (or more scores)
+    static constexpr uint32_t BAR_OFF = I_OFF + RCAND * SLOTS * 4;
     static constexpr uint32_t NBAR = 2 * STAGES + 4 + 2;
     static constexpr uint32_t MISC_OFF = BAR_OFF + NBAR * 8;
-    static constexpr uint32_t ROW_OFF = MISC_OFF + 64;                       // one staged row chunk per epilogue warp
-    static constexpr uint32_t BYTES = ROW_OFF + NUM_EPI_WARPS * 32 * 4 + 1024;  // + alignment slack
+    static constexpr uint32_t BYTES = MISC_OFF + 64 + 1024;  // + alignment slack
     static_assert(BYTES <= 227 * 1024, "shared memory of the kNN kernel exceeds 227 KB");
-    static_assert(ROW_OFF % 16 == 0, "staged rows must be 16-byte aligned");
+    static_assert(SLOTS == SLOT_STRIDE, "one candidate column per (tile, half, row)");
 };
 
 // The point tiles a query group scans, in order: every tile, or (a pruned
@@ -349,17 +467,34 @@ struct TileWalk {
 // F8: the operands are e4m3 bytes with the row size of BF16 KA columns.
 // rptr / rngs (nullable): the tile ranges of each query group (pruned search).
 // qcap (nullable): per query, a score no kept candidate reaches (a proven
-// bound of the pruned search's second pass); the rows start from it instead
-// of +inf, so far points never enter the insertion path.
-// R: candidates kept per (query, half), RCAND or fewer (a pass that only
-// bounds the (k+1)-th distance); the slots past R are written empty.
-template <int KA, bool F8, int R = RCAND>
+// bound from an earlier pass); the rows start from it instead of +inf, so far
+// points are never candidates.
+// gorder (nullable): the groups in descending order of their tile counts; the
+// CTAs take them forwards and backwards in turn, so the sums of their counts
+// stay close (200k x 50 points: 782 groups of 90 to 500 tiles; taken as they
+// come, an SM idled 29 to 36% of the kernel).
+// BOUND: the scan only bounds each query's (k+1)-th score: bound[q] receives the
+// BOUND_KEEP smallest 8-column minima of either half, ascending. k+1 minima are
+// k+1 points, so their largest is a bound, and nearly the (k+1)-th score itself
+// (two of a query's nearest seldom share 8 columns); no ids, no list to keep in
+// order. Otherwise cand_idx[q] receives the candidates' ids.
+//
+// The epilogue sets the pace (K = 32 or 64 leaves the tensor pipe a quarter to
+// a half busy at best). Per tile a warp reads its 64 columns at once, frees the
+// accumulator, and takes minima of 8 columns; only an 8-column group in which
+// some row's minimum passes that row's threshold is looked at again, all rows
+// of the warp together, a candidate costing two predicated stores. A row is
+// searched for its worst only when it is full; one that starts from a bounding
+// scan's bound (some 20 candidates) hardly ever is. Taking the rows one by one,
+// with a search of the row's slots for every candidate, the two scans of
+// 1M x 50 points took 31.1 and 56.4 ms; they take 8.5 and 16.4 ms.
+template <int KA, bool F8, bool BOUND = false>
 __global__ void __launch_bounds__(KNN_THREADS, 1)
     k_knn_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, uint32_t n,
-             uint32_t nq, float* __restrict__ cand_score, uint32_t* __restrict__ cand_idx, uint32_t* status,
-             uint32_t lim, uint32_t hold_tiles, const uint32_t* __restrict__ rptr, const uint2* __restrict__ rngs,
-             const float* __restrict__ qcap) {
-    using L = KnnSmem<KA, R>;
+             uint32_t nq, uint32_t* __restrict__ cand_idx, float* __restrict__ bound, uint32_t* status, uint32_t lim,
+             uint32_t hold_tiles, const KnnScale* __restrict__ scale, const uint32_t* __restrict__ rptr,
+             const uint2* __restrict__ rngs, const float* __restrict__ qcap, const uint32_t* __restrict__ gorder) {
+    using L = KnnSmem<KA>;
     extern __shared__ __align__(1024) unsigned char raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sA = smem + L::A_OFF;
@@ -379,6 +514,11 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t ntiles = (n + TILE - 1) / TILE;          // point tiles (B)
     const uint32_t ngroups = (nq + QT * TILE - 1) / (QT * TILE);  // query tile groups (A)
+    // the i-th group of this CTA, ngroups when there is none
+    auto group_at = [&](uint32_t i) -> uint32_t {
+        const uint64_t pos = (uint64_t)i * gridDim.x + ((i & 1) && gorder ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+        return pos >= ngroups ? ngroups : (gorder ? gorder[pos] : (uint32_t)pos);
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < L::STAGES; ++s) {
@@ -411,7 +551,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
             uint64_t it = 0;  // global B tile counter (all groups)
             uint32_t gi = 0;
             bool a_in_flight = false;
-            for (uint32_t g = blockIdx.x; g < ngroups && !*abort_flag; g += gridDim.x, ++gi) {
+            for (uint32_t g; (g = group_at(gi)) < ngroups && !*abort_flag; ++gi) {
                 if (gi > 0 && !mbar_wait(aempty, (gi - 1) & 1, lim)) {
                     *abort_flag = 1;
                     break;
@@ -450,10 +590,11 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
     } else if (warp == 1) {
         // ---------------- MMA issuer
         if (lane == 0) {
-            constexpr uint32_t idesc = F8 ? idesc_e4m3_128x128() : idesc_bf16_128x128();
+            const uint32_t idesc =
+                F8 ? idesc_e4m3_128x128() : idesc_16bit_128x128(f16_exp(scale) != INT32_MIN);
             uint64_t it = 0;
             uint32_t gi = 0;
-            for (uint32_t g = blockIdx.x; g < ngroups && !*abort_flag; g += gridDim.x, ++gi) {
+            for (uint32_t g; (g = group_at(gi)) < ngroups && !*abort_flag; ++gi) {
                 if (!mbar_wait(afull, gi & 1, lim)) {
                     *abort_flag = 1;
                     break;
@@ -484,7 +625,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
                                 mma_e4m3(d, smem_desc<KA>(abase + kk * 32), smem_desc<KA>(bbase + kk * 32), idesc,
                                          kk > 0 ? 1u : 0u);
                             else
-                                mma_bf16(d, smem_desc<KA>(abase + kk * 32), smem_desc<KA>(bbase + kk * 32), idesc,
+                                mma_16bit(d, smem_desc<KA>(abase + kk * 32), smem_desc<KA>(bbase + kk * 32), idesc,
                                          kk > 0 ? 1u : 0u);
                         }
                     }
@@ -510,120 +651,92 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
         const int h = combo % HALVES;           // column half
         const int lq = warp & 3;                // lane quarter
         const int row = lq * 32 + lane;         // row within the query tile
-        const int owner = combo * TILE + row;   // candidate-buffer column
-        constexpr int S = L::SLOTS;
-        float* srow = (float*)(smem + L::ROW_OFF) + ew * 32;  // this warp's staged row chunk
+        const uint32_t owner = combo * TILE + row;  // candidate-buffer column
+        constexpr uint32_t S = SLOT_STRIDE;
         uint64_t it = 0;
-        for (uint32_t g = blockIdx.x; g < ngroups && !*abort_flag; g += gridDim.x) {
+        uint32_t gi = 0;
+        for (uint32_t g; (g = group_at(gi)) < ngroups && !*abort_flag; ++gi) {
             const uint64_t qrow = (uint64_t)g * QT * TILE + q * TILE + row;
-            const float capv = (qcap && qrow < nq) ? qcap[qrow] : INFINITY;
-            float thr = capv;
-            int thr_slot = 0;
-            for (int s2 = 0; s2 < R; ++s2) {
-                cs[s2 * S + owner] = INFINITY;
-                ci[s2 * S + owner] = 0xFFFFFFFFu;
-            }
+            const float capv = (!BOUND && qcap && qrow < nq) ? qcap[qrow] : INFINITY;
+            float thr = qrow < nq ? capv : -INFINITY;  // rows past the last query take nothing
+            uint32_t cnt = 0;      // candidates held
+            uint32_t off = owner;  // where the next one goes
             TileWalk walk(rptr, rngs, g, ntiles);
-            const uint32_t cnt = walk.count();
-            for (uint32_t t = 0; t < cnt; ++t, ++it) {
+            const uint32_t tcnt = walk.count();
+            for (uint32_t t = 0; t < tcnt; ++t, ++it) {
                 const uint32_t tile = walk.next();
                 const uint32_t b = (uint32_t)(it & 1);
-                if (!mbar_wait(accfull + b, (uint32_t)((it >> 1) & 1), lim)) {
+                if (!__all_sync(0xFFFFFFFFu, mbar_wait(accfull + b, (uint32_t)((it >> 1) & 1), lim))) {
                     *abort_flag = 1;
                     break;
                 }
                 fence_after();
-                const uint32_t taddr =
-                    tmem + ((uint32_t)(lq * 32) << 16) + b * (QT * TILE) + q * TILE + h * (TILE / HALVES);
-#pragma unroll 1
-                for (int c0 = 0; c0 < TILE / HALVES; c0 += 32) {
-                    float r[32];
-                    tmem_ld32(taddr + c0, r);
-                    // branch-free prefilter: the chunk's minimum against the worst kept
-                    float m[16];
+                float r[64];
+                tmem_ld64(tmem + ((uint32_t)(lq * 32) << 16) + b * (QT * TILE) + q * TILE + h * (TILE / HALVES), r);
+                fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(accempty + b);  // the scores are in registers
+                const uint32_t base_idx = tile * TILE + h * (TILE / HALVES);
+                if (base_idx + 64 > n) {  // the last tile's rows past the points hold zeros, not scores
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) m[j] = fminf(r[j], r[j + 16]);
+                    for (int j = 0; j < 64; ++j)
+                        if (base_idx + j >= n) r[j] = INFINITY;
+                }
+                float m[8];
 #pragma unroll
-                    for (int w2 = 8; w2 >= 1; w2 >>= 1)
+                for (int j8 = 0; j8 < 8; ++j8) {
+                    const float* x = r + j8 * 8;
+                    m[j8] = fminf(fminf(fminf(x[0], x[1]), fminf(x[2], x[3])),
+                                  fminf(fminf(x[4], x[5]), fminf(x[6], x[7])));
+                }
+                const float mall = fminf(fminf(fminf(m[0], m[1]), fminf(m[2], m[3])),
+                                         fminf(fminf(m[4], m[5]), fminf(m[6], m[7])));
+                if (!__any_sync(0xFFFFFFFFu, mall < thr)) continue;
+                if constexpr (BOUND) {
+                    if (__any_sync(0xFFFFFFFFu, cnt > BOUND_SLOTS - 8)) {  // a tile adds up to 8
+                        thr = fminf(thr, bound_cut(cs, owner, cnt));
+                        cnt = cnt < BOUND_KEEP ? cnt : BOUND_KEEP;
+                        off = cnt * S + owner;
+                    }
 #pragma unroll
-                        for (int j = 0; j < w2; ++j) m[j] = fminf(m[j], m[j + w2]);
-                    const uint32_t base_idx = tile * TILE + h * (TILE / HALVES) + c0;
-                    unsigned hits = __ballot_sync(0xFFFFFFFFu, m[0] < thr);
-                    if (__popc(hits) > COOP_ROWS) {
-                        // many rows have candidates: each lane scans its own row
-                        if (m[0] < thr) {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) {
-                                if (r[j] < thr && base_idx + j < n) {
-                                    const Worst w = cand_insert<R>(cs, ci, owner, thr_slot, r[j], base_idx + j);
-                                    thr = fminf(w.thr, capv);
-                                    thr_slot = w.slot;
-                                }
-                            }
+                    for (int j8 = 0; j8 < 8; ++j8) {
+                        if (m[j8] < thr) {
+                            cs[off] = m[j8];
+                            ++cnt;
+                            off += S;
                         }
-                    } else {
-                        // few rows: the warp takes them one at a time, lane j holding
-                        // column j; inserts in ascending column order with a warp argmax
-                        // over the row's kept slots (same operations as the lane path)
-                        while (hits) {
-                            const int L = __ffs(hits) - 1;
-                            hits &= hits - 1;
-                            if (lane == L) {
+                    }
+                } else {
 #pragma unroll
-                                for (int j = 0; j < 32; j += 4)
-                                    *(float4*)(srow + j) = make_float4(r[j], r[j + 1], r[j + 2], r[j + 3]);
-                            }
-                            __syncwarp();
-                            const float v = srow[lane];
-                            __syncwarp();
-                            const int ownerL = owner - lane + L;
-                            float thrL = __shfl_sync(0xFFFFFFFFu, thr, L);
-                            int slotL = __shfl_sync(0xFFFFFFFFu, thr_slot, L);
-                            const float capL = __shfl_sync(0xFFFFFFFFu, capv, L);
-                            const bool inrange = base_idx + lane < n;
-                            unsigned cand = __ballot_sync(0xFFFFFFFFu, inrange && v < thrL);
-                            while (cand) {
-                                const int jc = __ffs(cand) - 1;
-                                if (lane == jc) {
-                                    cs[slotL * S + ownerL] = v;
-                                    ci[slotL * S + ownerL] = base_idx + jc;
-                                }
-                                __syncwarp();
-                                // new worst of the row: highest score, lowest slot on ties
-                                float wv = lane < R ? cs[lane * S + ownerL] : -INFINITY;
-                                int ws = lane;
+                    for (int j8 = 0; j8 < 8; ++j8) {
+                        if (!__any_sync(0xFFFFFFFFu, m[j8] < thr)) continue;
 #pragma unroll
-                                for (int o = 16; o; o >>= 1) {
-                                    const float ov = __shfl_xor_sync(0xFFFFFFFFu, wv, o);
-                                    const int os = __shfl_xor_sync(0xFFFFFFFFu, ws, o);
-                                    if (ov > wv || (ov == wv && os < ws)) {
-                                        wv = ov;
-                                        ws = os;
-                                    }
+                        for (int j = j8 * 8; j < j8 * 8 + 8; ++j) {
+                            if (r[j] < thr) {
+                                cs[off] = r[j];
+                                ci[off] = base_idx + j;
+                                ++cnt;
+                                off += S;
+                                if (cnt >= (uint32_t)RCAND) {
+                                    const Kept kp = row_worst(cs, owner);
+                                    thr = fminf(kp.thr, capv);
+                                    off = kp.off;
                                 }
-                                thrL = fminf(wv, capL);
-                                slotL = ws;
-                                // later columns of this row that still beat the new worst
-                                cand &= ~((2u << jc) - 1u);
-                                cand &= __ballot_sync(0xFFFFFFFFu, inrange && v < thrL);
-                            }
-                            if (lane == L) {
-                                thr = thrL;
-                                thr_slot = slotL;
                             }
                         }
                     }
                 }
-                fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(accempty + b);
             }
-            if (*abort_flag) break;
-            if (qrow < nq) {
-                for (int s2 = 0; s2 < RCAND; ++s2) {
-                    cand_score[qrow * RTOTAL + h * RCAND + s2] = s2 < R ? cs[s2 * S + owner] : INFINITY;
-                    cand_idx[qrow * RTOTAL + h * RCAND + s2] = s2 < R ? ci[s2 * S + owner] : 0xFFFFFFFFu;
-                }
+            if (__any_sync(0xFFFFFFFFu, *abort_flag != 0)) break;
+            if constexpr (BOUND) {
+                bound_cut(cs, owner, cnt);
+                if (qrow < nq)
+                    for (int s2 = 0; s2 < BOUND_KEEP; ++s2)
+                        bound[(qrow * HALVES + h) * BOUND_KEEP + s2] = cs[s2 * S + owner];
+            } else if (qrow < nq) {
+                const uint32_t have = cnt < RCAND ? cnt : RCAND;
+                for (uint32_t s2 = 0; s2 < (uint32_t)RCAND; ++s2)
+                    cand_idx[qrow * RTOTAL + h * RCAND + s2] = s2 < have ? ci[s2 * S + owner] : 0xFFFFFFFFu;
             }
         }
     }
@@ -941,61 +1054,209 @@ CUtensorMap make_map(const void* base, uint64_t n, uint32_t row_bytes, bool byte
     return m;
 }
 
-// Tile ranges of each query group of a pruned search (device arrays).
+// Scores are |y|^2 - 2 x.y from 16-bit operands x^, y^ with FP32 accumulation.
+// A point within Y of the origin scores within a Y + b Y^2 of the exact value:
+// |x.y - x^.y^| <= |x - x^| |y| + |x^| |y - y^|, with |y - y^| <= rho |y| (k_knn_prep
+// measured rho and each |x - x^|), gives a; the norm's two terms and up to 64
+// FP32 accumulations of terms that sum to at most 2 |x| |y| + |y|^2 stay below
+// b = 2^-13. Measured residuals in place of the unit roundoff: on a mixture of
+// 200k x 50 points the margin of the median query is 0.54 (f16) or 3.8 (BF16),
+// from the unit roundoff of BF16 it was 6.8, at a 15th neighbour's squared
+// distance of 83.
+struct ScoreMargin {
+    double a, b;
+};
+__device__ __forceinline__ ScoreMargin score_margin(double nx, double rx, const KnnScale* sc) {
+    const double rho = (double)__uint_as_float(sc->rho);
+    return ScoreMargin{2.0 * (rx + (nx + rx) * rho) * (1.0 + 0x1.0p-20), 0x1.0p-13};
+}
+
+// k + 1 points' squared FP32 distances against any real distance: 2^-16 covers
+// the rounding of either side.
+constexpr double KTH_SLACK = 1.0 + 0x1.0p-14;
+
+__device__ __forceinline__ float up_or_inf(double v) {
+    return v < INFINITY ? __double2float_ru(v) : INFINITY;  // NaN: no bound
+}
+
+// An upper bound on each query's (k+1)-th squared distance from the minima of a
+// bounding scan: the (k+1)-th smallest t of the query's two ascending lists is
+// the score of a point with k others at or below it. Every one of them obeys
+// d^2 <= t + |x|^2 + a Y + b Y^2 with Y = |x| + d; the larger root of that
+// quadratic bounds d. Query r is point q0 + r.
+__global__ void k_bound_kth(const float* __restrict__ minima, uint64_t nq, uint64_t q0, uint32_t k1,
+                            const float* __restrict__ nx, const float* __restrict__ rx,
+                            const KnnScale* __restrict__ sc, float* __restrict__ kb) {
+    const int e = f16_exp(sc);
+    const double unit = e != INT32_MIN ? ldexp(1.0, -2 * e) : 1.0;  // scores in the points' units
+    for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < nq; r += (uint64_t)gridDim.x * blockDim.x) {
+        const float* l0 = minima + r * (HALVES * BOUND_KEEP);
+        const float* l1 = l0 + BOUND_KEEP;
+        uint32_t i = 0, j = 0;
+        float t = INFINITY;
+        for (uint32_t s = 0; s < k1; ++s) {
+            const float a = i < (uint32_t)BOUND_KEEP ? l0[i] : INFINITY, b = j < (uint32_t)BOUND_KEEP ? l1[j] : INFINITY;
+            if (a <= b) ++i;
+            else ++j;
+            t = fminf(a, b);
+        }
+        if (!(t < INFINITY)) {
+            kb[r] = INFINITY;
+            continue;
+        }
+        const double x = nx[q0 + r];
+        const ScoreMargin m = score_margin(x, rx[q0 + r], sc);
+        const double p = m.a + 2.0 * m.b * x, q = (double)t * unit + x * x + m.a * x + m.b * x * x;
+        const double disc = p * p + 4.0 * (1.0 - m.b) * q;  // negative only by rounding, at distance 0
+        const double dist = (p + sqrt(disc > 0.0 ? disc : 0.0)) / (2.0 * (1.0 - m.b));
+        kb[r] = up_or_inf(dist * dist * KTH_SLACK);
+    }
+}
+
+// The same bound where the first scan kept whole lists: their (k+1)-th FP32 distance.
+__global__ void k_list_kth(const float* __restrict__ d2, const uint32_t* __restrict__ perm, uint64_t n, uint32_t k1,
+                           float* __restrict__ kb) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        kb[i] = up_or_inf((double)d2[(uint64_t)perm[i] * k1 + k1 - 1] * KTH_SLACK);
+}
+
+// The score bound the last scan starts from (query r is the point ord[r], or q0
+// + r without ord, and its bound kb[r] then): a point that can reach the
+// query's list lies within d^2 <= kb, so it scores at most kb - |x|^2 plus the
+// margin at Y = |x| + d. Rounded up, and one step more: a candidate's score must
+// be below the cap also where every term is zero (k + 1 points at the origin).
+__global__ void k_score_cap(const float* __restrict__ kb, uint64_t nq, uint64_t q0, const uint32_t* __restrict__ ord,
+                            const float* __restrict__ nx, const float* __restrict__ rx,
+                            const KnnScale* __restrict__ sc, float* __restrict__ cap) {
+    const int e = f16_exp(sc);
+    const double unit = e != INT32_MIN ? ldexp(1.0, 2 * e) : 1.0;
+    for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < nq; r += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t i = ord ? ord[r] : q0 + r;
+        const double d2 = kb[ord ? i : r], x = nx[i], low = x * (1.0 - 0x1.0p-15);
+        const ScoreMargin m = score_margin(x, rx[i], sc);
+        const double Y = x + sqrt(d2);
+        cap[r] = nextafterf(up_or_inf((d2 - low * low + m.a * Y + m.b * Y * Y) * unit), INFINITY);
+    }
+}
+
+// What a scan starts from (device arrays, all nullable).
 struct TileLists {
-    const uint32_t* rptr = nullptr;  // ngroups + 1
-    const uint2* rngs = nullptr;     // (first tile, tile count)
-    const float* cap = nullptr;      // per query (launch order): the score bound of k_knn_tc's qcap
+    const uint32_t* rptr = nullptr;    // the pruned search's tile ranges of each query group: ngroups + 1
+    const uint2* rngs = nullptr;       // (first tile, tile count)
+    const float* cap = nullptr;        // per query (launch order): the score bound of k_knn_tc's qcap
+    const uint32_t* gorder = nullptr;  // the groups by descending tile count
 };
 
-template <int KA, bool F8, int R = RCAND>
-void launch_tc(Ctx& c, const CUtensorMap& ta, const CUtensorMap& tb, uint64_t n, uint64_t nq, float* cand_score,
-               uint32_t* cand_idx, const TileLists& tl = TileLists{}) {
-    using L = KnnSmem<KA, R>;
-    SC_CUDA(cudaFuncSetAttribute(k_knn_tc<KA, F8, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES));
+// Whether the 2 x BOUND_KEEP minima of a bounding scan leave room beside the
+// k + 1 points they bound; otherwise a first scan keeps whole candidate lists.
+bool few_bound(uint32_t k1) { return 2 * BOUND_KEEP >= (int)k1 + 8; }
+
+// A scan of the queries' tiles: candidate ids to cand_idx, or (BOUND) score
+// minima to bound.
+template <int KA, bool F8, bool BOUND>
+void launch_tc(Ctx& c, const CUtensorMap& ta, const CUtensorMap& tb, uint64_t n, uint64_t nq, uint32_t* cand_idx,
+               float* bound, const KnnScale* scale, const TileLists& tl) {
+    using L = KnnSmem<KA>;
+    SC_CUDA(cudaFuncSetAttribute(k_knn_tc<KA, F8, BOUND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES));
     const uint32_t ngroups = (uint32_t)((nq + QT * TILE - 1) / (QT * TILE));
     const unsigned grid = std::min<unsigned>(ngroups, (unsigned)c.sm_count);
-    k_knn_tc<KA, F8, R><<<grid, KNN_THREADS, L::BYTES, c.stream>>>(ta, tb, (uint32_t)n, (uint32_t)nq, cand_score,
-                                                                 cand_idx, c.d_status, c.wait_limit,
-                                                                 c.knn_hold_tiles, tl.rptr, tl.rngs, tl.cap);
+    k_knn_tc<KA, F8, BOUND><<<grid, KNN_THREADS, L::BYTES, c.stream>>>(
+        ta, tb, (uint32_t)n, (uint32_t)nq, cand_idx, bound, c.d_status, c.wait_limit, c.knn_hold_tiles, scale, tl.rptr,
+        tl.rngs, tl.cap, tl.gorder);
     SC_LAUNCH_CHECK();
     c.launches++;
 }
 
-// Candidates of the queries q0 .. q0 + nq - 1 against all n points. A is the
-// query operand: its tensor map starts at row q0 (KA * 2 bytes per row, a
-// multiple of 16, so every row start is a legal TMA base).
-template <int KA>
-void candidates(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint64_t q0, uint64_t nq, float* cand_score,
+// The contraction's operands of the points X. The query operand's tensor map
+// starts at row q0 (64 or 128 bytes per row, so every row start is a legal TMA
+// base) and has nq rows.
+struct TcOperands {
+    DBuf<uint8_t> A, B;
+    DBuf<float> nx, rx;  // 16-bit: each row's norm and rounding error (k_knn_prep)
+    CUtensorMap ta{}, tb{};
+    int kind = 0;  // 0: 16-bit KA = 32, 1: 16-bit KA = 64, 2: e4m3
+    const KnnScale* scale = nullptr;
+    uint32_t row_bytes() const { return kind == 1 ? 128u : 64u; }
+};
+
+// scale: the point set's ranges (k_knn_scales has run).
+void prep_operands(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint64_t q0, uint64_t nq, int precision,
+                   KnnScale* scale, TcOperands& op) {
+    op.kind = precision == SC_KNN_FP8 ? 2 : d <= 30 ? 0 : 1;
+    op.scale = scale;
+    const uint64_t rb = op.row_bytes();
+    op.A.alloc(c, n * rb);
+    op.B.alloc(c, n * rb);
+    if (op.kind == 2) {
+        k_knn_prep_f8<<<grid_for(n, 256), 256, 0, c.stream>>>(dX, n, d, scale, op.A.get(), op.B.get());
+    } else {
+        op.nx.alloc(c, n);
+        op.rx.alloc(c, n);
+        uint16_t *A = (uint16_t*)op.A.get(), *B = (uint16_t*)op.B.get();
+        const unsigned grid = grid_for(n * 32, 256, 148u * 8u);
+        if (op.kind == 0) k_knn_prep<32><<<grid, 256, 0, c.stream>>>(dX, n, d, scale, A, B, op.nx.get(), op.rx.get());
+        else k_knn_prep<64><<<grid, 256, 0, c.stream>>>(dX, n, d, scale, A, B, op.nx.get(), op.rx.get());
+    }
+    SC_LAUNCH_CHECK();
+    c.launches++;
+    op.ta = make_map(op.A.get() + q0 * rb, nq, (uint32_t)rb, op.kind == 2);
+    op.tb = make_map(op.B.get(), n, (uint32_t)rb, op.kind == 2);
+}
+
+void launch_keep(Ctx& c, const TcOperands& op, uint64_t n, uint64_t nq, uint32_t* cidx, const TileLists& tl) {
+    if (op.kind == 2) launch_tc<32, true, false>(c, op.ta, op.tb, n, nq, cidx, nullptr, op.scale, tl);
+    else if (op.kind == 0) launch_tc<32, false, false>(c, op.ta, op.tb, n, nq, cidx, nullptr, op.scale, tl);
+    else launch_tc<64, false, false>(c, op.ta, op.tb, n, nq, cidx, nullptr, op.scale, tl);
+}
+
+// Bounds every query's (k+1)-th squared distance (kb, query order) by a scan of
+// 16-bit scores. minima: 2 x BOUND_KEEP words per query.
+void launch_bound(Ctx& c, const TcOperands& op, uint64_t n, uint64_t q0, uint64_t nq, uint32_t k1, float* minima,
+                  const TileLists& tl, float* kb) {
+    if (op.kind == 0) launch_tc<32, false, true>(c, op.ta, op.tb, n, nq, nullptr, minima, op.scale, tl);
+    else launch_tc<64, false, true>(c, op.ta, op.tb, n, nq, nullptr, minima, op.scale, tl);
+    k_bound_kth<<<grid_for(nq, 256), 256, 0, c.stream>>>(minima, nq, q0, k1, op.nx.get(), op.rx.get(), op.scale, kb);
+    SC_LAUNCH_CHECK();
+    c.launches++;
+}
+
+// Candidates of the queries q0 .. q0 + nq - 1 against all n points. 16-bit
+// operands take two scans, as the pruned search does: the first bounds each
+// query's (k+1)-th distance, the second starts from that bound, so its rows
+// hold some twenty candidates instead of taking 32 (1 + ln(n / 64)) one after
+// another. One scan from +inf took 1.33 ms at 5,003 x 30 points, the two take
+// 0.15 ms. One scan for lists too long for the bounding scan's minima (k > 23)
+// and for e4m3, whose scores are too coarse for a useful bound.
+void candidates(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t k, uint64_t q0, uint64_t nq, int precision,
                 uint32_t* cand_idx) {
-    DBuf<__nv_bfloat16> A(c, n * KA), B(c, n * KA);
-    k_knn_prep<KA><<<grid_for(n, 256), 256, 0, c.stream>>>(dX, n, d, A.get(), B.get());
+    DBuf<KnnScale> scale(c, 1);
+    zero(c, scale.get(), 1);
+    k_knn_scales<<<grid_for(n, 256), 256, 0, c.stream>>>(dX, n, d, scale.get());
     SC_LAUNCH_CHECK();
     c.launches++;
-    CUtensorMap ta = make_map(A.get() + q0 * KA, nq, KA * 2, false), tb = make_map(B.get(), n, KA * 2, false);
-    launch_tc<KA, false>(c, ta, tb, n, nq, cand_score, cand_idx);
-}
-
-// The same search with e4m3 operands (64-byte rows, the geometry of BF16 KA = 32).
-void candidates_f8(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint64_t q0, uint64_t nq, float* cand_score,
-                   uint32_t* cand_idx) {
-    DBuf<uint8_t> A(c, n * 64), B(c, n * 64);
-    DBuf<unsigned> mx(c, 2);
-    zero(c, mx.get(), 2);
-    k_knn_scales<<<grid_for(n, 256), 256, 0, c.stream>>>(dX, n, d, mx.get(), mx.get() + 1);
-    k_knn_prep_f8<<<grid_for(n, 256), 256, 0, c.stream>>>(dX, n, d, mx.get(), mx.get() + 1, A.get(), B.get());
-    SC_LAUNCH_CHECK();
-    c.launches += 2;
-    CUtensorMap ta = make_map(A.get() + q0 * 64, nq, 64, true), tb = make_map(B.get(), n, 64, true);
-    launch_tc<32, true>(c, ta, tb, n, nq, cand_score, cand_idx);
+    TcOperands op;
+    prep_operands(c, dX, n, d, q0, nq, precision, scale.get(), op);
+    TileLists tl;
+    DBuf<float> kb, cap;
+    if (op.kind != 2 && few_bound(k + 1)) {
+        kb.alloc(c, nq);
+        cap.alloc(c, nq);
+        launch_bound(c, op, n, q0, nq, k + 1, (float*)cand_idx, tl, kb.get());
+        k_score_cap<<<grid_for(nq, 256), 256, 0, c.stream>>>(kb.get(), nq, q0, nullptr, op.nx.get(), op.rx.get(),
+                                                             op.scale, cap.get());
+        SC_LAUNCH_CHECK();
+        c.launches++;
+        tl.cap = cap.get();
+    }
+    launch_keep(c, op, n, nq, cand_idx, tl);
 }
 
 // ------------------------------------------------------------ exact pruning
 // Points are grouped by a deterministic k-means (fixed-point sums, ties to the
 // lower centroid) and sorted by group, so every 128-row tile is spatially
-// coherent. A query group first scans the tiles of its own clusters; the exact
-// FP32 re-rank of those candidates bounds each query's (k+1)-th distance from
-// above. A cluster b can hold a closer point only if a lower bound on
+// coherent. A query group first scans the tiles of its own clusters; the k + 1
+// smallest score minima bound each query's (k+1)-th distance from above
+// (k_bound_kth). A cluster b can hold a closer point only if a lower bound on
 // |q - x| over x in b is at most that distance: the ball bound |q - c_b| - r_b
 // and the slab bound of the direction u from the query's cluster centre to
 // c_b (every x in b projects into [lo, hi] on u, so |q - x| >= the distance
@@ -1003,10 +1264,10 @@ void candidates_f8(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint64_t q0,
 // every cluster some query of the group cannot exclude, narrowed to the fine
 // cells (~256 points) a ball bound cannot exclude; skipped points are provably
 // farther than the query's (k+1)-th neighbour, so the result is the full
-// search's. The first pass keeps fewer candidates (it only yields the bound)
+// search's. The first pass keeps score minima alone (it only yields the bound)
 // and walks each group's nearest cells first; the second starts every query's
 // candidate rows from a proven score bound derived from the first pass's
-// distance (k_pass2_cap). Both passes take their tile lists from the device.
+// bound (k_score_cap). Both passes take their tile lists from the device.
 constexpr int KM_ITERS = 8;
 constexpr uint32_t KM_SAMPLE = 65536;  // points the Lloyd steps run on
 
@@ -1281,8 +1542,8 @@ __global__ void k_cluster_extent(const float* __restrict__ Xs, uint32_t d, const
 // rounding of a projection or a distance (a few ulps of the largest |x| times
 // d), so every bound used is below the exact one.
 __global__ void k_cluster_needs(const float* __restrict__ Xs, uint32_t d, const Chunk* __restrict__ chunks,
-                                const uint32_t* __restrict__ perm, const float* __restrict__ d2k, uint32_t k1,
-                                const float* __restrict__ cent, const unsigned* __restrict__ rad,
+                                const float* __restrict__ kb, const float* __restrict__ cent,
+                                const unsigned* __restrict__ rad,
                                 const float* __restrict__ Ua, const unsigned* __restrict__ lo,
                                 const unsigned* __restrict__ hi, uint32_t K, float eps, uint32_t words,
                                 unsigned long long* mask) {
@@ -1311,7 +1572,7 @@ __global__ void k_cluster_needs(const float* __restrict__ Xs, uint32_t d, const 
         float x[64];
 #pragma unroll
         for (int j = 0; j < 64; ++j) x[j] = (uint32_t)j < d ? Xs[ii * d + j] : 0.0f;
-        const float kd2 = d2k[(uint64_t)perm[ii] * k1 + (k1 - 1)];
+        const float kd2 = kb[ii];
         // no (k+1)-th neighbour among the own clusters: every cluster is needed
         const float kth = isfinite(kd2) ? sqrtf(kd2) * (1.0f + 1e-5f) + eps : INFINITY;
         unsigned long long m[4] = {0ull, 0ull, 0ull, 0ull};
@@ -1414,8 +1675,8 @@ __global__ void k_cell_radius(const float* __restrict__ Xs, uint64_t n, uint32_t
 // |g - c_f| - r_g - r_f > max kth; only the remaining cells are tested per
 // query. Both tests carry the same rounding margins, the group test twice.
 __global__ void k_group_cells(const float* __restrict__ Xs, uint64_t n, uint32_t d, const uint32_t* __restrict__ ord,
-                              const uint32_t* __restrict__ perm, const float* __restrict__ d2k, uint32_t k1,
-                              const unsigned long long* __restrict__ gmask, const uint32_t* __restrict__ gown,
+                              const float* __restrict__ kb, const unsigned long long* __restrict__ gmask,
+                              const uint32_t* __restrict__ gown,
                               uint32_t words, uint32_t K, const uint32_t* __restrict__ fbase,
                               const float* __restrict__ fcent, const unsigned* __restrict__ crad, float eps,
                               uint32_t cwords, const unsigned long long* __restrict__ qmask,
@@ -1427,7 +1688,7 @@ __global__ void k_group_cells(const float* __restrict__ Xs, uint64_t n, uint32_t
     float x[64];
 #pragma unroll
     for (int j = 0; j < 64; ++j) x[j] = (uint32_t)j < d ? Xs[sq * d + j] : 0.0f;
-    const float kd2 = d2k[(uint64_t)perm[sq] * k1 + (k1 - 1)];
+    const float kd2 = kb[sq];
     const float kth = isfinite(kd2) ? sqrtf(kd2) * (1.0f + 1e-5f) + eps : INFINITY;
     extern __shared__ unsigned s_bits[];  // cwords: the result, then cwords: cells the group ball keeps
     unsigned* s_maybe = s_bits + cwords;
@@ -1595,11 +1856,11 @@ __global__ void k_u64_to_u32(const uint64_t* __restrict__ in, uint64_t n, uint32
 // [cstart[first], cstart[last + 1]); those become tile ranges, merged where
 // they touch or overlap.
 // Without rptr it counts the ranges into cnt; with it, it writes them from
-// rptr[g] and adds the group's tile count to *tiles.
+// rptr[g], adds the group's tile count to *tiles and leaves its sort key.
 __global__ void k_group_ranges(const unsigned* __restrict__ gcell, uint32_t cwords, uint32_t F,
                                const uint64_t* __restrict__ cstart, uint64_t ngroups,
                                const uint32_t* __restrict__ rptr, uint64_t* cnt, uint2* rngs,
-                               unsigned long long* tiles) {
+                               unsigned long long* tiles, uint32_t* gkey) {
     for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < ngroups;
          g += (uint64_t)gridDim.x * blockDim.x) {
         const unsigned* bits = gcell + g * cwords;
@@ -1644,38 +1905,12 @@ __global__ void k_group_ranges(const unsigned* __restrict__ gcell, uint32_t cwor
             }
         }
         if (open) emit(cur_b, cur_e);
-        if (rptr) atomicAdd(tiles, (unsigned long long)sum);
-        else cnt[g] = k;
-    }
-}
-
-// The pass-2 score bound of every query (row r of the pass-2 order is the
-// sorted query ord[r]). Scores are |y|^2 - 2 x.y from BF16 operands with FP32
-// accumulation. A point that can reach the final list has an FP32 distance of
-// at most d21 (the query's (k+1)-th FP32 distance from pass 1), so |y| <= Y =
-// |x| + sqrt(d21), and its score lies within 2^-6 (1 + 2^-6) |x| Y + 2^-14 Y^2
-// of d^2 - |x|^2. The terms: the BF16 roundings of x and y (unit roundoff
-// u = 2^-8 each) move 2 x.y by at most (4u + 2u^2) |x| |y| (Cauchy-Schwarz
-// over the products); the FP32 norm split into two BF16 terms and up to 64
-// FP32 accumulations add under 2^-15 (|x| |y| + |y|^2). 2^-16 (d21 + |x|^2)
-// covers the FP32 distances and norm; the sum is rounded up.
-__global__ void k_pass2_cap(const float* __restrict__ Xs, uint64_t n, uint32_t d, const uint32_t* __restrict__ ord,
-                            const uint32_t* __restrict__ perm, const float* __restrict__ d21, uint32_t k1,
-                            float* __restrict__ cap) {
-    for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t sq = ord[r];
-        const float* x = Xs + sq * d;
-        float nx2 = 0.0f;
-        for (uint32_t t = 0; t < d; ++t) nx2 = __fmaf_rn(x[t], x[t], nx2);
-        const float dk = d21[(uint64_t)perm[sq] * k1 + k1 - 1];
-        if (!(dk < INFINITY)) {
-            cap[r] = INFINITY;
-            continue;
+        if (rptr) {
+            atomicAdd(tiles, (unsigned long long)sum);
+            gkey[g] = ~(uint32_t)sum;  // ascending keys: descending tile counts
+        } else {
+            cnt[g] = k;
         }
-        const double nx = sqrt((double)nx2), Y = nx + sqrt((double)dk);
-        const double margin = ldexp(nx * Y, -6) * (1.0 + 0x1.0p-6) + ldexp(Y * Y, -14) +
-                              ldexp((double)dk + (double)nx2, -16);
-        cap[r] = __double2float_ru((double)dk - (double)nx2 + 1.01 * margin);
     }
 }
 
@@ -1742,55 +1977,6 @@ uint32_t prune_clusters(const Ctx& c, uint64_t n) {
     return (uint32_t)std::min<uint64_t>(256, std::max<uint64_t>(16, n / 8192));
 }
 
-// BF16 or FP8 operands of the points X (rows = queries = candidates).
-struct TcOperands {
-    DBuf<uint8_t> A, B;
-    CUtensorMap ta{}, tb{};
-    int kind = 0;  // 0: BF16 KA = 32, 1: BF16 KA = 64, 2: e4m3
-};
-
-void prep_operands(Ctx& c, const float* dX, uint64_t n, uint32_t d, int precision, TcOperands& op) {
-    if (precision == SC_KNN_FP8) {
-        op.kind = 2;
-        op.A.alloc(c, n * 64);
-        op.B.alloc(c, n * 64);
-        DBuf<unsigned> mx(c, 2);
-        zero(c, mx.get(), 2);
-        k_knn_scales<<<grid_for(n, 256), 256, 0, c.stream>>>(dX, n, d, mx.get(), mx.get() + 1);
-        k_knn_prep_f8<<<grid_for(n, 256), 256, 0, c.stream>>>(dX, n, d, mx.get(), mx.get() + 1, op.A.get(),
-                                                              op.B.get());
-        SC_LAUNCH_CHECK();
-        c.launches += 2;
-        op.ta = make_map(op.A.get(), n, 64, true);
-        op.tb = make_map(op.B.get(), n, 64, true);
-        return;
-    }
-    const uint32_t KA = d <= 30 ? 32 : 64;
-    op.kind = KA == 32 ? 0 : 1;
-    op.A.alloc(c, n * KA * 2);
-    op.B.alloc(c, n * KA * 2);
-    __nv_bfloat16* A = (__nv_bfloat16*)op.A.get();
-    __nv_bfloat16* B = (__nv_bfloat16*)op.B.get();
-    if (KA == 32) k_knn_prep<32><<<grid_for(n, 256), 256, 0, c.stream>>>(dX, n, d, A, B);
-    else k_knn_prep<64><<<grid_for(n, 256), 256, 0, c.stream>>>(dX, n, d, A, B);
-    SC_LAUNCH_CHECK();
-    c.launches++;
-    op.ta = make_map(A, n, KA * 2, false);
-    op.tb = make_map(B, n, KA * 2, false);
-}
-
-// few: keep PASS1_CAND candidates per (query, half) instead of RCAND (BF16;
-// for a pass whose lists only bound the (k+1)-th distance).
-constexpr int PASS1_CAND = 16;
-void launch_operands(Ctx& c, const TcOperands& op, uint64_t n, float* cscore, uint32_t* cidx, const TileLists& tl,
-                     bool few = false) {
-    if (op.kind == 2) launch_tc<32, true>(c, op.ta, op.tb, n, n, cscore, cidx, tl);
-    else if (op.kind == 0 && few) launch_tc<32, false, PASS1_CAND>(c, op.ta, op.tb, n, n, cscore, cidx, tl);
-    else if (op.kind == 0) launch_tc<32, false>(c, op.ta, op.tb, n, n, cscore, cidx, tl);
-    else if (few) launch_tc<64, false, PASS1_CAND>(c, op.ta, op.tb, n, n, cscore, cidx, tl);
-    else launch_tc<64, false>(c, op.ta, op.tb, n, n, cscore, cidx, tl);
-}
-
 // The exact k+1 nearest points of every point by the pruned search (see
 // "exact pruning" above); the same lists as the full scan.
 // Device time between events recorded on the context's stream.
@@ -1822,18 +2008,16 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     StageTimer tm(c);
     tm.mark();
     // 1. deterministic k-means: K centroids from evenly spaced points, KM_ITERS Lloyd steps
-    DBuf<unsigned> mx(c, 2);
-    zero(c, mx.get(), 2);
-    k_knn_scales<<<grid_for(n, 256), 256, 0, c.stream>>>(dX, n, d, mx.get(), mx.get() + 1);
+    DBuf<KnnScale> scale_words(c, 1);
+    zero(c, scale_words.get(), 1);
+    k_knn_scales<<<grid_for(n, 256), 256, 0, c.stream>>>(dX, n, d, scale_words.get());
     SC_LAUNCH_CHECK();
     c.launches++;
-    unsigned hmx[2];
-    d2h(c, hmx, mx.get(), 2);
     DBuf<float> cent(c, (uint64_t)K * d);
-    sync(c);
+    const KnnScale hmx = to_host(c, scale_words.get());
     float maxabs, maxnorm;
-    std::memcpy(&maxabs, &hmx[0], 4);
-    std::memcpy(&maxnorm, &hmx[1], 4);
+    std::memcpy(&maxabs, &hmx.maxabs, 4);
+    std::memcpy(&maxnorm, &hmx.maxnorm, 4);
     // sums of n coordinates of magnitude <= maxabs stay below 2^62 in fixed point
     const double span = std::max(1e-30, (double)maxabs * (double)n);
     const int e = std::min(40, (int)std::floor(62.0 - std::log2(span)) - 1);
@@ -1999,35 +2183,38 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     c.launches++;
     // 5. operands of the sorted points
     TcOperands op;
-    prep_operands(c, Xs.get(), n, d, precision, op);
+    prep_operands(c, Xs.get(), n, d, 0, n, precision, scale_words.get(), op);
     tm.mark();  // 3: extents and operands
     auto own = [&](uint64_t g, std::vector<std::pair<uint64_t, uint64_t>>& pts) {
         const uint32_t a0 = h_cl[g * QT * TILE], a1 = h_cl[std::min<uint64_t>(n, (g + 1) * QT * TILE) - 1];
         pts.emplace_back(start[a0], start[a1 + 1]);
         return std::make_pair(a0, a1);
     };
-    DBuf<float> cscore(c, n * RTOTAL);
     DBuf<uint32_t> cidx(c, n * RTOTAL);
-    // queries in the order `ord` (nullable: the sorted order), operand `o`
-    // a scan and its re-rank, the tile lists on the device
-    auto run_pass_dev = [&](const TcOperands& o, const uint32_t* ord, const uint32_t* d_rptr, const uint2* d_rngs,
-                            uint32_t* out_idx, float* out_d2, const float* qcap, bool few) {
-        launch_operands(c, o, n, cscore.get(), cidx.get(), TileLists{d_rptr, d_rngs, qcap}, few);
+    // the candidates' exact re-rank, queries in the order `ord` (nullable: the sorted order)
+    auto rerank = [&](const uint32_t* ord, uint32_t* out_idx, float* out_d2) {
         k_knn_rerank_sorted<<<grid_for(n * 32, 256), 256, 0, c.stream>>>(Xs.get(), n, d, k, ord, perm.get(),
                                                                         cidx.get(), out_idx, out_d2);
         SC_LAUNCH_CHECK();
         c.launches++;
     };
+    // query groups by descending tile count (stable), from their negated counts
+    DBuf<uint32_t> gkey(c, ngroups), gkey_s(c, ngroups), giota(c, ngroups), gorder(c, ngroups);
+    k_iota_u32<<<grid_for(ngroups, 256), 256, 0, c.stream>>>(giota.get(), ngroups);
+    SC_LAUNCH_CHECK();
+    c.launches++;
+    auto order_groups = [&]() {
+        sort_pairs(c, gkey.get(), gkey_s.get(), giota.get(), gorder.get(), ngroups, 32);
+    };
     // 6. pass 1: every query group against its own clusters, nearest cells first
     // (k_order_tiles: the rows' thresholds tighten within the first tiles, so
-    // fewer later scores take the insertion path; pass 1 only yields the
-    // bounds of pass 2)
+    // fewer later scores are kept; pass 1 only yields the bounds of pass 2: kb,
+    // each sorted query's (k+1)-th squared distance from above)
     std::vector<uint32_t> rptr(ngroups + 1, 0);
     uint64_t tiles1 = 0;
-    DBuf<uint32_t> idx1(c, n * k1);
-    DBuf<float> d21(c, n * k1);
+    DBuf<float> kb(c, n);
     {
-        std::vector<uint32_t> h_tb(ngroups), h_te(ngroups);
+        std::vector<uint32_t> h_tb(ngroups), h_te(ngroups), h_key(ngroups);
         std::vector<std::pair<uint64_t, uint64_t>> pts;
         for (uint64_t g = 0; g < ngroups; ++g) {
             pts.clear();
@@ -2035,6 +2222,7 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
             h_tb[g] = (uint32_t)(pts[0].first / TILE);
             h_te[g] = (uint32_t)((pts[0].second + TILE - 1) / TILE);
             tiles1 += h_te[g] - h_tb[g];
+            h_key[g] = ~(h_te[g] - h_tb[g]);
             if (tiles1 > 0xFFFFFFFFull)
                 fail(SC_E_UNSUPPORTED, "pruned kNN lists exceed 2^32 tiles: use more clusters or the full scan");
             rptr[g + 1] = (uint32_t)tiles1;
@@ -2054,10 +2242,20 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
                                                                fcent.get(), d_rp.get(), d_rg.get());
         SC_LAUNCH_CHECK();
         c.launches++;
-        // pass 1 only bounds the (k+1)-th distance: fewer kept candidates suffice
-        // (any k + 1 real points give a bound; 2 x PASS1_CAND of them are kept)
-        run_pass_dev(op, nullptr, d_rp.get(), d_rg.get(), idx1.get(), d21.get(), nullptr,
-                     2 * PASS1_CAND >= (int)k1 + 8);
+        h2d(c, gkey.get(), h_key.data(), ngroups);
+        order_groups();
+        const TileLists tl{d_rp.get(), d_rg.get(), nullptr, gorder.get()};
+        if (op.kind != 2 && few_bound(k1)) {
+            launch_bound(c, op, n, 0, n, k1, (float*)cidx.get(), tl, kb.get());
+        } else {
+            DBuf<uint32_t> idx1(c, n * k1);
+            DBuf<float> d21(c, n * k1);
+            launch_keep(c, op, n, n, cidx.get(), tl);
+            rerank(nullptr, idx1.get(), d21.get());
+            k_list_kth<<<grid_for(n, 256), 256, 0, c.stream>>>(d21.get(), perm.get(), n, k1, kb.get());
+            SC_LAUNCH_CHECK();
+            c.launches++;
+        }
         sync(c);  // the host arrays above must outlive the copies
     }
     tm.mark();  // 4: pass 1
@@ -2072,8 +2270,8 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     const size_t sm_need = (size_t)K * d * 8 + (size_t)K * 12;
     SC_CUDA(cudaFuncSetAttribute(k_cluster_needs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_need));
     k_cluster_needs<<<(unsigned)ch_need.size(), QT * TILE, sm_need, c.stream>>>(
-        Xs.get(), d, d_ch_need.get(), perm.get(), d21.get(), k1, cent.get(), rad.get(), d_Ua.get(), lo.get(), hi.get(),
-        K, eps, words, mask.get());
+        Xs.get(), d, d_ch_need.get(), kb.get(), cent.get(), rad.get(), d_Ua.get(), lo.get(), hi.get(), K, eps, words,
+        mask.get());
     SC_LAUNCH_CHECK();
     c.launches++;
     // pass-2 order: by own cluster, then by need set; groups of 256 in that order
@@ -2099,7 +2297,7 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     DBuf<unsigned> gcell(c, ngroups * cwords);
     zero(c, gcell.get(), ngroups * cwords);
     SC_CUDA(cudaFuncSetAttribute(k_group_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(cwords * 8)));
-    k_group_cells<<<(unsigned)ngroups, QT * TILE, cwords * 8, c.stream>>>(Xs.get(), n, d, ord.get(), perm.get(), d21.get(), k1,
+    k_group_cells<<<(unsigned)ngroups, QT * TILE, cwords * 8, c.stream>>>(Xs.get(), n, d, ord.get(), kb.get(),
                                                                 gmask.get(), gown.get(), words, K, d_fbase.get(),
                                                                 fcent.get(), crad.get(), eps, cwords, mask.get(),
                                                                 cl_s.get(), gcell.get());
@@ -2109,8 +2307,9 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     // the query operand in pass-2 order
     TcOperands op2;
     {
-        const uint32_t row_bytes = op.kind == 1 ? 128u : 64u;
+        const uint32_t row_bytes = op.row_bytes();
         op2.kind = op.kind;
+        op2.scale = op.scale;
         op2.A.alloc(c, n * row_bytes);
         k_gather_operand_rows<<<grid_for(n * row_bytes / 16, 256), 256, 0, c.stream>>>(
             (const uint4*)op.A.get(), ord.get(), n, row_bytes / 16, (uint4*)op2.A.get());
@@ -2119,20 +2318,18 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
         op2.ta = make_map(op2.A.get(), n, row_bytes, op.kind == 2);
         op2.tb = op.tb;
     }
-    // score bounds of the BF16 search from the pass-1 distances (FP8 scores
+    // score bounds of the 16-bit search from the pass-1 bounds (FP8 scores
     // carry too coarse an error for a useful bound: none)
     DBuf<float> qcap;
     if (op.kind != 2) {
         qcap.alloc(c, n);
-        k_pass2_cap<<<grid_for(n, 256), 256, 0, c.stream>>>(Xs.get(), n, d, ord.get(), perm.get(), d21.get(), k1,
-                                                            qcap.get());
+        k_score_cap<<<grid_for(n, 256), 256, 0, c.stream>>>(kb.get(), n, 0, ord.get(), op.nx.get(), op.rx.get(),
+                                                            op.scale, qcap.get());
         SC_LAUNCH_CHECK();
         c.launches++;
     }
     sync(c);
     tm.mark();  // 9: bounds
-    idx1.release();
-    d21.release();
     mask.release();
     // 8. pass 2: every cell a query of the group cannot exclude (cells in point
     // order), the tile lists built on the device from the cell bitmaps
@@ -2144,7 +2341,7 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     DBuf<unsigned long long> d_tiles2(c, 1);
     zero(c, d_tiles2.get(), 1);
     k_group_ranges<<<grid_for(ngroups, 128), 128, 0, c.stream>>>(gcell.get(), cwords, F, d_cstart.get(), ngroups,
-                                                                 nullptr, gcnt.get(), nullptr, nullptr);
+                                                                 nullptr, gcnt.get(), nullptr, nullptr, nullptr);
     exclusive_sum(c, gcnt.get(), r64.get(), ngroups + 1);
     const uint64_t nranges = to_host(c, r64.get() + ngroups);
     if (nranges > 0xFFFFFFFFull)
@@ -2153,12 +2350,14 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     DBuf<uint2> d_rngs2(c, std::max<uint64_t>(nranges, 1));
     k_group_ranges<<<grid_for(ngroups, 128), 128, 0, c.stream>>>(gcell.get(), cwords, F, d_cstart.get(), ngroups,
                                                                  d_rptr2.get(), nullptr, d_rngs2.get(),
-                                                                 d_tiles2.get());
+                                                                 d_tiles2.get(), gkey.get());
     SC_LAUNCH_CHECK();
     c.launches += 3;
     const uint64_t tiles2 = to_host(c, d_tiles2.get());
     tm.mark();  // 10: lists built
-    run_pass_dev(op2, ord.get(), d_rptr2.get(), d_rngs2.get(), idx, d2, qcap.get(), false);
+    order_groups();
+    launch_keep(c, op2, n, n, cidx.get(), TileLists{d_rptr2.get(), d_rngs2.get(), qcap.get(), gorder.get()});
+    rerank(ord.get(), idx, d2);
     tm.mark();  // 11: pass 2
     c.knn_stats.ms_cluster = tm.ms(0, 3);
     c.knn_stats.ms_pass1 = tm.ms(3, 4);
@@ -2200,18 +2399,10 @@ void knn_search_device(Ctx& c, const float* dX, uint64_t n, uint64_t d, uint64_t
         const uint64_t groups = (nq + QT * TILE - 1) / (QT * TILE), tiles = (n + TILE - 1) / TILE;
         c.knn_stats.tiles_scanned = c.knn_stats.tiles_full = groups * tiles;
     }
-    DBuf<float> cscore(c, precision == SC_KNN_FP32 ? 0 : nq * RTOTAL);
     DBuf<uint32_t> cidx(c, nq * RTOTAL);
-    if (precision == SC_KNN_FP32) {
-        if (d <= 32) candidates_fp32<32>(c, dX, n, (uint32_t)d, q0, nq, cidx.get());
-        else candidates_fp32<64>(c, dX, n, (uint32_t)d, q0, nq, cidx.get());
-    } else if (precision == SC_KNN_FP8) {
-        candidates_f8(c, dX, n, (uint32_t)d, q0, nq, cscore.get(), cidx.get());
-    } else if (d <= 30) {
-        candidates<32>(c, dX, n, (uint32_t)d, q0, nq, cscore.get(), cidx.get());
-    } else {
-        candidates<64>(c, dX, n, (uint32_t)d, q0, nq, cscore.get(), cidx.get());
-    }
+    if (precision != SC_KNN_FP32) candidates(c, dX, n, (uint32_t)d, (uint32_t)k, q0, nq, precision, cidx.get());
+    else if (d <= 32) candidates_fp32<32>(c, dX, n, (uint32_t)d, q0, nq, cidx.get());
+    else candidates_fp32<64>(c, dX, n, (uint32_t)d, q0, nq, cidx.get());
     k_knn_rerank<<<grid_for(nq * 32, 256), 256, 0, c.stream>>>(dX, n, (uint32_t)d, (uint32_t)k, q0, nq,
                                                                 cidx.get(), idx, d2);
     SC_LAUNCH_CHECK();

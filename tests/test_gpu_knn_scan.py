@@ -1,0 +1,87 @@
+"""The two-scan candidate search of the 16-bit tensor-core arm against the FP32
+arm (exact FP32 differences of every pair): equal lists, bit for bit, at the
+edges of its tiles and lists and for point sets that drive each operand format
+and each bound to its limits."""
+import numpy as np
+import pytest
+
+import sc_gpu
+from sc_gpu import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _points(kind, n, d, seed):
+    rng = np.random.Generator(np.random.PCG64(seed))
+    if kind == "mixture":
+        return synth.gaussian_mixture(n, d, 6, seed=seed, sigma=(0.7, 1.5))[0]
+    x = rng.normal(size=(n, d))
+    if kind == "tiny":       # f16 needs its scale
+        x *= 1e-7
+    elif kind == "huge":     # past f16's own range without it
+        x *= 1e9
+    elif kind == "outlier":  # wider than f16 takes: BF16 operands
+        x[0] *= 1e6
+    elif kind == "small_rows":  # points far below the rest, above and below the f16 rule
+        x[: n // 2] *= 2.0 ** -9
+        x[n // 2: n // 2 + 3] = 0.0
+    elif kind == "integers":  # exactly representable: the measured rounding error is zero
+        x = np.round(3 * x)
+    return x.astype(np.float32)
+
+
+@pytest.mark.parametrize("kind", ["mixture", "tiny", "huge", "outlier", "small_rows"])
+@pytest.mark.parametrize("n,d,k", [(1, 3, 1), (17, 3, 5), (127, 30, 10), (128, 31, 15), (129, 30, 15), (257, 62, 10),
+                                   (1023, 7, 23), (1500, 50, 24), (2049, 50, 31), (5003, 30, 10)])
+def test_scans_give_the_exact_lists(kind, n, d, k):
+    X = _points(kind, n, d, n + d + k)
+    a = sc_gpu.knn_gaussian(X, k, sigma=sc_gpu.SIGMA_KTH, sym=sc_gpu.SYM_UNION, precision=sc_gpu.KNN_FP32)
+    b = sc_gpu.knn_gaussian(X, k, sigma=sc_gpu.SIGMA_KTH, sym=sc_gpu.SYM_UNION, precision=sc_gpu.KNN_BF16)
+    if kind == "outlier":
+        # the outlier's own scores all lie within one 16-bit rounding of its norm:
+        # no 16-bit operand can rank its neighbours, so its row is left out
+        assert np.array_equal(a.index[1:], b.index[1:])
+        assert np.array_equal(a.distances[1:].view(np.uint32), b.distances[1:].view(np.uint32))
+        return
+    assert np.array_equal(a.index, b.index)
+    assert np.array_equal(a.distances.view(np.uint32), b.distances.view(np.uint32))
+    assert np.array_equal(a.conn_ptrs, b.conn_ptrs) and np.array_equal(a.conn_nbrs, b.conn_nbrs)
+    assert np.array_equal(a.conn_w.view(np.uint32), b.conn_w.view(np.uint32))
+
+
+@pytest.mark.parametrize("n,d,k", [(300, 4, 10), (3000, 12, 15)])
+def test_ties_and_points_at_the_origin(n, d, k):
+    """Equal distances (integer coordinates, repeated points, many points at the
+    origin, where every score and bound is zero): the distances of the lists are
+    the exact ones; which of the tied points is listed may differ."""
+    X = _points("integers", n, d, 5)
+    X[: 2 * k] = 0.0
+    a = sc_gpu.knn_gaussian(X, k, precision=sc_gpu.KNN_FP32)
+    b = sc_gpu.knn_gaussian(X, k, precision=sc_gpu.KNN_BF16)
+    assert np.array_equal(a.distances, b.distances)
+    assert np.array_equal(b.index[:, 0], np.arange(n))
+
+
+@pytest.mark.parametrize("n,lo,hi", [(4000, 0, 1), (4000, 255, 1030), (4000, 3999, 4000)])
+def test_query_rows_of_a_shard(n, lo, hi):
+    X = _points("mixture", n, 40, 9)
+    full = sc_gpu.knn_gaussian(X, 12, precision=sc_gpu.KNN_FP32)
+    idx, d2 = sc_gpu.knn_search(X, 12, lo, hi)
+    assert np.array_equal(idx, full.index[lo:hi])
+    assert np.array_equal(np.sqrt(d2), full.distances[lo:hi])
+
+
+@pytest.mark.parametrize("kind", ["mixture", "outlier"])
+def test_pruned_search_of_either_operand_format(kind):
+    """70,000 points: the pruned search with f16 (mixture) and BF16 (an outlier
+    widens the range) operands, against the FP32 arm on sampled rows."""
+    n, d, k = 70_000, 20, 15
+    X = _points("mixture", n, d, 3)
+    if kind == "outlier":
+        X[7] = 1e6
+    b = sc_gpu.knn_gaussian(X, k)
+    assert sc_gpu.knn_last_stats()["clusters"] >= 16
+    for lo in (0, 33_000, n - 500):
+        idx, d2 = sc_gpu.knn_search(X, k, lo, lo + 500, precision=sc_gpu.KNN_FP32)
+        assert np.array_equal(idx, b.index[lo:lo + 500])
+        assert np.array_equal(np.sqrt(d2), b.distances[lo:lo + 500])
