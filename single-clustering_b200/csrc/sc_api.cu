@@ -577,6 +577,7 @@ sc_status sc_leiden_batch_ex(sc_ctx* ctx, const sc_graph* const* graphs, const s
         sc_error_info first_err{};
         auto worker = [&]() {
             sc::Ctx w;
+            w.staged_downloads = false;
             sc_status st = init_ctx(w, c.device, W <= 8);
             if (st != SC_OK) {
                 std::lock_guard<std::mutex> lk(mu);

@@ -96,20 +96,44 @@ struct Ctx {
     // (bucket counts, counters, sizes): copies into it are truly asynchronous, so
     // several can be queued and completed by one stream synchronisation
     uint8_t* mailbox = nullptr;
-    // pinned staging lanes of large host -> device uploads (created on first use)
+    // pinned staging lanes of large copies to and from pageable memory (created on first use)
     struct Staging* staging = nullptr;
+    // large results come back through the staging lanes; not on the contexts of
+    // a batch's workers, which live for one call and run beside each other
+    bool staged_downloads = true;
 };
 constexpr int SIDE_STREAMS = 3;
 constexpr size_t MAILBOX_BYTES = 4096;
-constexpr int STAGE_LANES = 4;                     // host threads of a staged upload
-constexpr size_t STAGE_CHUNK = size_t(4) << 20;     // bytes per pinned buffer (two per lane)
+constexpr int STAGE_LANES = 8;                     // host threads of a staged copy
+constexpr size_t STAGE_CHUNK = size_t(2) << 20;     // bytes per pinned buffer (two per lane)
 constexpr size_t STAGE_MIN_BYTES = size_t(16) << 20;  // smaller uploads use one plain copy
+constexpr size_t DOWNLOAD_MIN_BYTES = size_t(4) << 20;  // smaller results come back in plain copies
 
 // Host -> device copy of `bytes` from pageable `src`, ordered on the context's
 // stream (large copies go through the pinned staging lanes); src may be reused
 // when it returns.
 void upload(Ctx& c, void* dst, const void* src, size_t bytes);
 void release_staging(Ctx& c);
+// Device -> host copies into pageable buffers, ordered after what the context's
+// stream has queued at start(). Large ones run on the staging lanes' own threads
+// and streams until finish(), which also waits for the context's stream; the
+// sources must stay as they are until then.
+class Download {
+   public:
+    explicit Download(Ctx& ctx);
+    ~Download();
+    Download(const Download&) = delete;
+    Download& operator=(const Download&) = delete;
+    void add(void* dst, const void* src, size_t bytes);  // a null dst or no bytes: nothing to copy
+    void start();
+    void finish();
+
+   private:
+    struct State;
+    void join();
+    Ctx& c;
+    std::unique_ptr<State> st;
+};
 // The device's pool of user-graph arrays (created on first use, kept until exit).
 cudaMemPool_t user_graph_pool(int device);
 // u32 device labels -> u64 host labels (widened on the device, one copy)

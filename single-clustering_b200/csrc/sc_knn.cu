@@ -2412,10 +2412,12 @@ void knn_search_device(Ctx& c, const float* dX, uint64_t n, uint64_t d, uint64_t
 
 // Gaussian connectivities (neighborhood/mod.rs:105-163, :480-544) from the
 // device k+1 lists of all n points (squared distances): sigma per point,
-// weights, symmetrisation, duplicate removal, CSR.
+// weights, symmetrisation, duplicate removal, CSR. earlier: a download that
+// still runs on the context's staging lanes.
 void knn_connectivities_device(Ctx& c, const uint32_t* idx, const float* d2, uint64_t n, uint64_t k,
                                const sc_knn_opts& opts, uint64_t* conn_ptrs, uint32_t* conn_nbrs, float* conn_w,
-                               uint64_t conn_cap, uint64_t* conn_nnz, DevGraph** graph_out) {
+                               uint64_t conn_cap, uint64_t* conn_nnz, DevGraph** graph_out,
+                               Download* earlier = nullptr) {
     DBuf<float> sigma(c, n);
     DBuf<unsigned long long> keys(c, 2 * n * k + 1), keys_s(c, 2 * n * k + 1);
     DBuf<float> w(c, 2 * n * k + 1), w_s(c, 2 * n * k + 1);
@@ -2456,27 +2458,35 @@ void knn_connectivities_device(Ctx& c, const uint32_t* idx, const float* d2, uin
     SC_LAUNCH_CHECK();
     c.launches++;
     if (conn_nnz) *conn_nnz = M;
+    Download csr(c);  // while the graph is built
+    if (earlier) earlier->finish();  // the lanes serve one download at a time
     if (conn_ptrs) {
         if (M > conn_cap) fail(SC_E_INVALID_ARGUMENT, "conn_capacity %llu < %llu entries",
                                (unsigned long long)conn_cap, (unsigned long long)M);
-        d2h(c, conn_ptrs, ptr.get(), n + 1);
-        if (conn_nbrs) d2h(c, conn_nbrs, cols.get(), M);
-        if (conn_w) d2h(c, conn_w, uw.get(), M);
+        csr.add(conn_ptrs, ptr.get(), ptr.bytes());
+        csr.add(conn_nbrs, cols.get(), M * sizeof(uint32_t));
+        csr.add(conn_w, uw.get(), M * sizeof(float));
+        csr.start();
     }
-    if (graph_out) *graph_out = graph_from_csr(c, ptr.get(), n + 1, cols.get(), M, uw.get(), M, nullptr, 0, true);
-    sync(c);
+    std::unique_ptr<DevGraph> graph;
+    if (graph_out) graph.reset(graph_from_csr(c, ptr.get(), n + 1, cols.get(), M, uw.get(), M, nullptr, 0, true));
+    csr.finish();
+    if (graph_out) *graph_out = graph.release();
 }
 
-void copy_lists_out(Ctx& c, const uint32_t* idx, const float* d2, uint64_t rows, uint64_t k, int squared,
-                    uint32_t* knn_index, float* knn_dist) {
-    if (knn_index) d2h(c, knn_index, idx, rows * (k + 1));
-    if (knn_dist) {
-        std::vector<float> h(rows * (k + 1));
-        d2h(c, h.data(), d2, rows * (k + 1));
-        sync(c);
-        for (uint64_t i = 0; i < h.size(); ++i) knn_dist[i] = squared ? h[i] : std::sqrt(h[i]);
-    }
-    sync(c);
+__global__ void k_sqrt(const float* __restrict__ a, uint64_t n, float* b) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        b[i] = sqrtf(a[i]);
+}
+
+// The distances a caller sees: the squared ones, or their roots in `roots`.
+const float* distances_out(Ctx& c, const float* d2, uint64_t count, int squared, bool wanted, DBuf<float>& roots) {
+    if (squared || !wanted || !count) return d2;
+    roots.alloc(c, count);
+    k_sqrt<<<grid_for(count, 256), 256, 0, c.stream>>>(d2, count, roots.get());
+    SC_LAUNCH_CHECK();
+    c.launches++;
+    return roots.get();
 }
 
 }  // namespace
@@ -2491,10 +2501,16 @@ void knn_gaussian(Ctx& c, const float* X, uint64_t n, uint64_t d, uint64_t k, co
     DBuf<uint32_t> idx(c, n * (k + 1));
     DBuf<float> d2(c, n * (k + 1));
     knn_search_device(c, dX.get(), n, d, k, 0, n, opts.precision, idx.get(), d2.get());
-    copy_lists_out(c, idx.get(), d2.get(), n, k, opts.squared_kiddo, knn_index, knn_dist);
-    if (!conn_ptrs && !graph_out) return;
-    knn_connectivities_device(c, idx.get(), d2.get(), n, k, opts, conn_ptrs, conn_nbrs, conn_w, conn_cap, conn_nnz,
-                              graph_out);
+    DBuf<float> roots;
+    const float* dist = distances_out(c, d2.get(), n * (k + 1), opts.squared_kiddo, knn_dist != nullptr, roots);
+    Download lists(c);  // while the connectivities are built
+    lists.add(knn_index, idx.get(), idx.bytes());
+    lists.add(knn_dist, dist, d2.bytes());
+    lists.start();
+    if (conn_ptrs || graph_out)
+        knn_connectivities_device(c, idx.get(), d2.get(), n, k, opts, conn_ptrs, conn_nbrs, conn_w, conn_cap, conn_nnz,
+                                  graph_out, &lists);
+    lists.finish();
 }
 
 // Times the search of all rows of X under candidate cluster counts (1: the
@@ -2562,7 +2578,11 @@ void knn_search(Ctx& c, const float* X, uint64_t n, uint64_t d, uint64_t k, uint
     DBuf<uint32_t> idx(c, nq * (k + 1));
     DBuf<float> d2(c, nq * (k + 1));
     knn_search_device(c, dX.get(), n, d, k, q0, nq, opts.precision, idx.get(), d2.get());
-    copy_lists_out(c, idx.get(), d2.get(), nq, k, 1, knn_index, knn_d2);
+    Download lists(c);
+    lists.add(knn_index, idx.get(), idx.bytes());
+    lists.add(knn_d2, d2.get(), d2.bytes());
+    lists.start();
+    lists.finish();
 }
 
 // Connectivities from gathered host lists (all n rows, squared distances).
