@@ -755,87 +755,156 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
 // sum_t (q_t - c_t)^2, the re-rank's own operations in the same order
 // (dimensions past d are zero on both sides and add exactly nothing), so the
 // candidates are the exact FP32 nearest points, with no norm expansion and no
-// reduced-precision operand. One thread per query, 256 queries per block, the
-// query's coordinates in registers; points stream through shared memory in
-// tiles of F32_TILE (every thread reads the same point: broadcast loads). Each
-// query keeps its RCAND best (distance, id) in shared memory, the worst kept
-// is the rejection threshold, so most points cost one compare after the
-// distance. The other RCAND candidate slots are written empty.
-constexpr int F32_THREADS = 256;
+// reduced-precision operand. A thread holds F32_Q queries' coordinates in
+// registers; points stream through shared memory in tiles of F32_TILE (every
+// thread reads the same point: broadcast loads).
+//
+// Bound by FP32 issue: 2 DP operations a pair (DP: d rounded up to 4, a register
+// array's size). One query a thread left it bound by the broadcast loads
+// instead (a 16-byte load feeds 8 operations, and holds the SM's one load
+// pipe as long as these take): 8.7 ms at 30,011 x 50, 6.3 with two queries and
+// two points at a time (four independent sums). Each half of
+// the points has blocks of its own (blockIdx.y) and keeps its RCAND best in its
+// half of the candidate slots, so small blocks spread evenly (470 of them
+// there). A candidate is two predicated stores into the query's F32_SLOTS
+// slots; when a row of the warp is nearly full, all rows are cut back to their
+// RCAND best together. The floor is 2.5 ms of FP32 operations; one query a thread,
+// a search of the row for every insertion and DP = 64 for all d > 32 took 9.1 ms.
+constexpr int F32_THREADS = 64;
+constexpr int F32_Q = 2;  // queries a thread
+constexpr int F32_QUERIES = F32_THREADS * F32_Q;
 constexpr int F32_TILE = 64;
+constexpr int F32_SLOTS = 40;
+constexpr int F32_GROUP = 2;  // points taken together: four independent sums a thread
+
+// Cuts a row of `cnt` candidates to its RCAND best (the last one takes the worst
+// one's slot until RCAND are left); returns the worst kept, or thr with fewer.
+__device__ __noinline__ float f32_cut(float* cs, uint32_t* ci, uint32_t cnt, float thr) {
+    while (cnt >= (uint32_t)RCAND) {
+        float worst = -INFINITY;
+        uint32_t at = 0;
+#pragma unroll 8
+        for (uint32_t s = 0; s < cnt; ++s) {
+            const float x = cs[s * F32_QUERIES];
+            if (x > worst) {
+                worst = x;
+                at = s;
+            }
+        }
+        thr = worst;
+        if (cnt == (uint32_t)RCAND) break;
+        --cnt;
+        cs[at * F32_QUERIES] = cs[cnt * F32_QUERIES];
+        ci[at * F32_QUERIES] = ci[cnt * F32_QUERIES];
+    }
+    return thr;
+}
 
 template <int DP>
 __global__ void __launch_bounds__(F32_THREADS) k_knn_fp32(const float* __restrict__ X, uint64_t n, uint32_t d,
                                                           uint64_t q0, uint64_t nq, uint32_t* __restrict__ cand_idx) {
     extern __shared__ __align__(16) unsigned char smem[];
-    float* tile = (float*)smem;                           // [F32_TILE][DP]
-    float* cs = tile + F32_TILE * DP;                     // [RCAND][F32_THREADS]
-    uint32_t* ci = (uint32_t*)(cs + RCAND * F32_THREADS);  // [RCAND][F32_THREADS]
+    float* tile = (float*)smem;                                // [F32_TILE][DP]
+    float* cs = tile + F32_TILE * DP + threadIdx.x;            // [F32_SLOTS][F32_QUERIES], this thread's columns
+    uint32_t* ci = (uint32_t*)(cs + F32_SLOTS * F32_QUERIES);  // at 0 and F32_THREADS; the ids beside them
     const uint32_t t = threadIdx.x;
-    const uint64_t lq = (uint64_t)blockIdx.x * F32_THREADS + t;
-    const bool have = lq < nq;
-    float q[DP];
+    const uint64_t lq0 = (uint64_t)blockIdx.x * F32_QUERIES + t;
+    float q[F32_Q][DP], thr[F32_Q];
+    uint32_t cnt[F32_Q];
 #pragma unroll
-    for (int j = 0; j < DP; ++j) q[j] = (have && (uint32_t)j < d) ? X[(q0 + lq) * d + j] : 0.0f;
-    for (int s2 = 0; s2 < RCAND; ++s2) {
-        cs[s2 * F32_THREADS + t] = INFINITY;
-        ci[s2 * F32_THREADS + t] = 0xFFFFFFFFu;
+    for (int u = 0; u < F32_Q; ++u) {
+        const uint64_t lq = lq0 + u * F32_THREADS;
+#pragma unroll
+        for (int j = 0; j < DP; ++j) q[u][j] = (lq < nq && (uint32_t)j < d) ? X[(q0 + lq) * d + j] : 0.0f;
+        thr[u] = lq < nq ? INFINITY : -INFINITY;
+        cnt[u] = 0;
     }
-    float thr = INFINITY;
-    int thr_slot = 0;
-    for (uint64_t base = 0; base < n; base += F32_TILE) {
+    // this half's points, whole tiles
+    const uint64_t tiles = (n + F32_TILE - 1) / F32_TILE, mid = (tiles + 1) / 2 * F32_TILE;
+    const uint64_t p0 = blockIdx.y ? mid : 0, p1 = blockIdx.y ? n : (mid < n ? mid : n);
+    for (uint64_t base = p0; base < p1; base += F32_TILE) {
         __syncthreads();  // the previous tile is no longer read
         for (uint32_t e = t; e < (uint32_t)(F32_TILE * DP); e += F32_THREADS) {
             const uint32_t p = e / DP, j = e % DP;
-            tile[e] = (base + p < n && j < d) ? X[(base + p) * d + j] : 0.0f;
+            tile[e] = (base + p < p1 && j < d) ? X[(base + p) * d + j] : 0.0f;
         }
         __syncthreads();
-        const uint32_t cnt = (n - base < (uint64_t)F32_TILE) ? (uint32_t)(n - base) : (uint32_t)F32_TILE;
-        for (uint32_t p = 0; p < cnt; ++p) {
-            const float4* c4 = (const float4*)(tile + p * DP);
-            float acc = 0.0f;
+        const uint32_t points = (p1 - base < (uint64_t)F32_TILE) ? (uint32_t)(p1 - base) : (uint32_t)F32_TILE;
+        for (uint32_t g = 0; g < points; g += F32_GROUP) {
+#pragma unroll
+            for (int u = 0; u < F32_Q; ++u) {
+                if (__any_sync(0xFFFFFFFFu, cnt[u] > F32_SLOTS - F32_GROUP)) {
+                    thr[u] = f32_cut(cs + u * F32_THREADS, ci + u * F32_THREADS, cnt[u], thr[u]);
+                    cnt[u] = cnt[u] < (uint32_t)RCAND ? cnt[u] : (uint32_t)RCAND;
+                }
+            }
+            // rows past the last point are zeros in the tile: computed, not taken
+            float acc[F32_GROUP][F32_Q];
+#pragma unroll
+            for (int v = 0; v < F32_GROUP; ++v)
+#pragma unroll
+                for (int u = 0; u < F32_Q; ++u) acc[v][u] = 0.0f;
+            const float4* c4 = (const float4*)(tile + g * DP);
 #pragma unroll
             for (int j4 = 0; j4 < DP / 4; ++j4) {
-                const float4 c = c4[j4];
-                float df = __fsub_rn(q[4 * j4], c.x);
-                acc = __fmaf_rn(df, df, acc);
-                df = __fsub_rn(q[4 * j4 + 1], c.y);
-                acc = __fmaf_rn(df, df, acc);
-                df = __fsub_rn(q[4 * j4 + 2], c.z);
-                acc = __fmaf_rn(df, df, acc);
-                df = __fsub_rn(q[4 * j4 + 3], c.w);
-                acc = __fmaf_rn(df, df, acc);
+#pragma unroll
+                for (int v = 0; v < F32_GROUP; ++v) {
+                    const float4 c = c4[v * (DP / 4) + j4];
+#pragma unroll
+                    for (int u = 0; u < F32_Q; ++u) {
+                        float df = __fsub_rn(q[u][4 * j4], c.x);
+                        acc[v][u] = __fmaf_rn(df, df, acc[v][u]);
+                        df = __fsub_rn(q[u][4 * j4 + 1], c.y);
+                        acc[v][u] = __fmaf_rn(df, df, acc[v][u]);
+                        df = __fsub_rn(q[u][4 * j4 + 2], c.z);
+                        acc[v][u] = __fmaf_rn(df, df, acc[v][u]);
+                        df = __fsub_rn(q[u][4 * j4 + 3], c.w);
+                        acc[v][u] = __fmaf_rn(df, df, acc[v][u]);
+                    }
+                }
             }
-            if (acc < thr) {
-                cs[thr_slot * F32_THREADS + t] = acc;
-                ci[thr_slot * F32_THREADS + t] = (uint32_t)(base + p);
-                thr = -INFINITY;
-                for (int s2 = 0; s2 < RCAND; ++s2) {
-                    const float x = cs[s2 * F32_THREADS + t];
-                    if (x > thr) {
-                        thr = x;
-                        thr_slot = s2;
+#pragma unroll
+            for (int v = 0; v < F32_GROUP; ++v) {
+#pragma unroll
+                for (int u = 0; u < F32_Q; ++u) {
+                    if (acc[v][u] < thr[u] && g + v < points) {
+                        cs[cnt[u] * F32_QUERIES + u * F32_THREADS] = acc[v][u];
+                        ci[cnt[u] * F32_QUERIES + u * F32_THREADS] = (uint32_t)(base + g + v);
+                        ++cnt[u];
                     }
                 }
             }
         }
     }
-    if (have) {
-        for (int s2 = 0; s2 < RCAND; ++s2) {
-            cand_idx[lq * RTOTAL + s2] = ci[s2 * F32_THREADS + t];
-            cand_idx[lq * RTOTAL + RCAND + s2] = 0xFFFFFFFFu;
-        }
+#pragma unroll
+    for (int u = 0; u < F32_Q; ++u) {
+        const uint64_t lq = lq0 + u * F32_THREADS;
+        f32_cut(cs + u * F32_THREADS, ci + u * F32_THREADS, cnt[u], thr[u]);
+        if (lq >= nq) continue;
+        const uint32_t kept = cnt[u] < (uint32_t)RCAND ? cnt[u] : (uint32_t)RCAND;
+        uint32_t* out = cand_idx + lq * RTOTAL + blockIdx.y * RCAND;
+        for (uint32_t s2 = 0; s2 < (uint32_t)RCAND; ++s2)
+            out[s2] = s2 < kept ? ci[s2 * F32_QUERIES + u * F32_THREADS] : 0xFFFFFFFFu;
     }
 }
 
 template <int DP>
-void candidates_fp32(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint64_t q0, uint64_t nq, uint32_t* cand_idx) {
-    const size_t sm = (size_t)F32_TILE * DP * 4 + (size_t)RCAND * F32_THREADS * 8;
+void candidates_fp32_dp(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint64_t q0, uint64_t nq, uint32_t* cand_idx) {
+    const size_t sm = (size_t)F32_TILE * DP * 4 + (size_t)F32_SLOTS * F32_QUERIES * 8;
     SC_CUDA(cudaFuncSetAttribute(k_knn_fp32<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    const uint64_t blocks = (nq + F32_THREADS - 1) / F32_THREADS;
-    k_knn_fp32<DP><<<(unsigned)blocks, F32_THREADS, sm, c.stream>>>(dX, n, d, q0, nq, cand_idx);
+    const uint64_t blocks = (nq + F32_QUERIES - 1) / F32_QUERIES;
+    k_knn_fp32<DP><<<dim3((unsigned)blocks, HALVES), F32_THREADS, sm, c.stream>>>(dX, n, d, q0, nq, cand_idx);
     SC_LAUNCH_CHECK();
     c.launches++;
+}
+
+// DP = d rounded up to a multiple of 4.
+template <int DP = 4>
+void candidates_fp32(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint64_t q0, uint64_t nq, uint32_t* cand_idx) {
+    if constexpr (DP < 64) {
+        if (d > (uint32_t)DP) return candidates_fp32<DP + 4>(c, dX, n, d, q0, nq, cand_idx);
+    }
+    candidates_fp32_dp<DP>(c, dX, n, d, q0, nq, cand_idx);
 }
 
 // ------------------------------------------------------------ exact re-rank
@@ -2380,7 +2449,7 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
 // Exact (brute-force) k+1 nearest points of the queries q0 .. q0 + nq - 1
 // among all n points of the device array dX: 64 candidates per query (the 32
 // best of each half of the candidate columns) from the BF16 or FP8 tensor-core
-// scores, or the 32 best exact FP32 distances from the CUDA cores, ranked
+// scores, or the 32 best exact FP32 distances of either half of the points from the CUDA cores, ranked
 // exactly in FP32. idx/d2 are nq x (k+1), self first, then ascending squared
 // distance, ties by lower index.
 void knn_search_device(Ctx& c, const float* dX, uint64_t n, uint64_t d, uint64_t k, uint64_t q0, uint64_t nq,
@@ -2401,8 +2470,7 @@ void knn_search_device(Ctx& c, const float* dX, uint64_t n, uint64_t d, uint64_t
     }
     DBuf<uint32_t> cidx(c, nq * RTOTAL);
     if (precision != SC_KNN_FP32) candidates(c, dX, n, (uint32_t)d, (uint32_t)k, q0, nq, precision, cidx.get());
-    else if (d <= 32) candidates_fp32<32>(c, dX, n, (uint32_t)d, q0, nq, cidx.get());
-    else candidates_fp32<64>(c, dX, n, (uint32_t)d, q0, nq, cidx.get());
+    else candidates_fp32(c, dX, n, (uint32_t)d, q0, nq, cidx.get());
     k_knn_rerank<<<grid_for(nq * 32, 256), 256, 0, c.stream>>>(dX, n, (uint32_t)d, (uint32_t)k, q0, nq,
                                                                 cidx.get(), idx, d2);
     SC_LAUNCH_CHECK();

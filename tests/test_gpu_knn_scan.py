@@ -85,3 +85,21 @@ def test_pruned_search_of_either_operand_format(kind):
         idx, d2 = sc_gpu.knn_search(X, k, lo, lo + 500, precision=sc_gpu.KNN_FP32)
         assert np.array_equal(idx, b.index[lo:lo + 500])
         assert np.array_equal(np.sqrt(d2), b.distances[lo:lo + 500])
+
+
+@pytest.mark.parametrize("d", [1, 4, 5, 31, 50, 62])
+@pytest.mark.parametrize("n,k", [(2, 1), (64, 10), (65, 31), (129, 15), (200, 31), (4097, 31)])
+def test_fp32_halves_against_fp64(n, d, k):
+    """The FP32 arm splits the points at a whole tile (n around 64 and 128: an
+    empty, a ragged and a full second half) and keeps 32 per half: its squared
+    distances equal the FP64 search's within FP32 rounding (62 terms, 2^-18)."""
+    X = _points("mixture", n, d, n + d)
+    idx, d2 = sc_gpu.knn_search(X, k, 0, n, precision=sc_gpu.KNN_FP32)
+    X64 = X.astype(np.float64)
+    full = np.stack([((X64 - x) ** 2).sum(1) for x in X64])
+    full[np.arange(n), np.arange(n)] = -1.0
+    want = np.maximum(np.sort(full, axis=1)[:, :k + 1], 0.0)
+    m = min(k + 1, n)
+    assert np.array_equal(idx[:, 0], np.arange(n))
+    assert np.all(np.isinf(d2[:, m:])) and np.all(idx[:, m:] == 0xFFFFFFFF)
+    assert np.all(np.abs(d2[:, :m] - want[:, :m]) <= 2.0 ** -18 * want[:, :m] + 1e-30)
