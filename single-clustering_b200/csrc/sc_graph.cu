@@ -1695,6 +1695,23 @@ void finish_aggregate(Ctx& c, DevGraph& out) {
     out.sym_state.store(1, std::memory_order_relaxed);
 }
 
+DevGraph* graph_from_contraction(Ctx& c, uint64_t n, uint64_t E, const uint64_t* ptr, const uint32_t* nbr,
+                                 const float* w, const double* node_w) {
+    std::unique_ptr<DevGraph> g(new DevGraph());
+    galloc(c, *g, n, E);
+    d2d(c, g->ptr, ptr, n + 1);
+    d2d(c, g->nbr, nbr, E);
+    d2d(c, g->w, w, E);
+    d2d(c, g->node_w, node_w, n);
+    if (E) {
+        k_fill_erow<<<grid_for(n * 32, TB), TB, 0, c.stream>>>(g->ptr, n, g->erow);
+        SC_LAUNCH_CHECK();
+        c.launches++;
+    }
+    finish_aggregate(c, *g);
+    return g.release();
+}
+
 DevGraph* graph_aggregate(Ctx& c, const DevGraph& g, const uint32_t* d_grp, uint32_t G) {
     const uint64_t n = g.n, E = g.E;
     std::unique_ptr<DevGraph> out(new DevGraph());

@@ -318,6 +318,9 @@ DevGraph* graph_from_edges(Ctx& c, uint64_t n, const uint64_t* from, const uint6
 DevGraph* graph_aggregate(Ctx& c, const DevGraph& g, const uint32_t* d_grp, uint32_t n_groups);
 // disjoint union of `count` graphs, instance i's node ids shifted past instance i-1's
 DevGraph* graph_union(Ctx& c, const DevGraph* const* gs, uint64_t count);
+// a graph of a run from the device arrays of a contraction (clean, symmetric rows)
+DevGraph* graph_from_contraction(Ctx& c, uint64_t n, uint64_t E, const uint64_t* ptr, const uint32_t* nbr,
+                                 const float* w, const double* node_w);
 void graph_validate_symmetry(Ctx& c, const DevGraph& g);
 bool graph_bitwise_symmetric(Ctx& c, const DevGraph& g);
 void graph_copy_csr(Ctx& c, const DevGraph& g, uint64_t* ptr, uint32_t* nbr, float* w);
