@@ -25,15 +25,45 @@ namespace sc {
 
 namespace {
 
+// The counters of a decide kernel (entries, candidates, nodes) from its threads'
+// sums: one global atomic per counter and block. Every warp adding its own made
+// the three addresses the bound of a large launch.
+__device__ __forceinline__ void flush_counters(unsigned long long* counters, unsigned long long sdeg,
+                                               unsigned long long scand, unsigned long long snodes) {
+    __shared__ unsigned long long s_sum[3][32];
+    const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    unsigned long long x[3] = {sdeg, scand, snodes};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        for (int o = 16; o; o >>= 1) x[k] += __shfl_xor_sync(0xFFFFFFFFu, x[k], o);
+        if (lane == 0) s_sum[k][wid] = x[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        unsigned long long t = 0;
+        for (unsigned w = 0; w < nw; ++w) t += s_sum[threadIdx.x][w];
+        if (t) atomicAdd(counters + 1 + threadIdx.x, t);
+    }
+}
+
 // ------------------------------------------------------------ small-degree decide
 // REFINE=false: local moving. REFINE=true: refinement (singletons only, inside
 // the constraint, randomised choice among non-negative candidates).
+//
+// Bound by instructions and the latency of the gathers about equally (1M-point
+// kNN graph: 29 warps an SM, issue slots 36% busy before). What it no longer does:
+// sum a community's entries with 64-bit shared atomics, which retry once per lane
+// on the same community (peer_sum folds them in at most log2 G shuffle rounds);
+// evaluate the gain of the own, the joined and the fresh community one after
+// another, a division each (two lanes without a candidate take the own and the
+// fresh one); start a block per handful of nodes, so that the prefetch below never
+// ran and every warp ended with three atomics on the same counters. The first
+// batch of a 1M x 30 graph: 210 -> 167 us (G = 16) and 174 -> 105 us (G = 32).
 template <int G, bool REFINE, bool MULTI>
 __global__ void __launch_bounds__(TB, 4) k_decide_small(Params p, const uint32_t* __restrict__ list,
                                                         const uint64_t* __restrict__ lbeg,
                                                         const uint32_t* __restrict__ ldeg, uint32_t count) {
     const unsigned FULL = 0xFFFFFFFFu;
-    __shared__ unsigned long long s_acc[TB];
     const int lane = threadIdx.x & 31;
     const int sub = lane & (G - 1);
     const int gw = lane / G;  // group within warp
@@ -76,6 +106,7 @@ __global__ void __launch_bounds__(TB, 4) k_decide_small(Params p, const uint32_t
         fetch(wb + step);
         const NodeCfg q = node_cfg<MULTI>(p, v);
         const uint32_t own = have ? ro(p.memb + (v)) : 0;
+        const uint32_t fresh = (uint32_t)(p.S0 + v);
         bool eligible = have;
         if (REFINE && have) eligible = ro(p.csize + (own)) == 1;  // refine.rs:60-62
         bool valid = eligible && sub < deg;
@@ -84,66 +115,83 @@ __global__ void __launch_bounds__(TB, 4) k_decide_small(Params p, const uint32_t
         valid = valid && u != v;
         if (REFINE && valid) valid = ro(p.constraint + (u)) == ro(p.constraint + (v));
         const uint32_t cu = valid ? ro(p.memb + (u)) : NONE32;
-        const long long wf = valid ? to_fix((double)wt, p.inv_scale) : 0;
-        const uint64_t key = valid ? (((uint64_t)gw << 32) | cu) : (0xFFFFFFFF00000000ull | (uint64_t)lane);
-        const unsigned mm = __match_any_sync(FULL, key);
-        const bool leader = valid && (__ffs(mm) - 1 == lane);
-        // per-community sums: every lane adds into its group leader's shared slot
-        // (integer adds, so the order does not matter); only leaders read theirs
-        s_acc[threadIdx.x] = 0ull;
-        __syncwarp();
-        if (valid) atomicAdd(&s_acc[(threadIdx.x & ~31u) + (unsigned)(__ffs(mm) - 1)], (unsigned long long)wf);
-        __syncwarp();
-        const long long acc = (long long)s_acc[threadIdx.x];
-        __syncwarp();
         // node quantities (identical in all lanes of the group)
         long long kf = 0, af = 0;
         double sl = 0.0;
+        bool try_fresh = false;
         if (eligible) {
             kf = to_fix(ro(p.strength + (v)), p.inv_scale);
             af = to_fix(ro(p.node_w + (v)), p.inv_nscale);
             sl = ro(p.self_loop + (v));
+            // one empty community per node (local_move.rs:92-100)
+            if (!REFINE) try_fresh = fresh != own && ro(p.csize + (own)) > 1 && ro(p.csize + (fresh)) == 0;
         }
         const double k = from_fix(kf, p.scale), a = from_fix(af, p.nscale);
+        if (!REFINE) try_fresh = try_fresh && (!p.has_limit || a <= p.limit);
+        const uint64_t key = valid ? (((uint64_t)gw << 32) | cu) : (0xFFFFFFFF00000000ull | (uint64_t)lane);
+        const unsigned mm = __match_any_sync(FULL, key);
+        const bool leader = valid && (__ffs(mm) - 1 == lane);
+        const long long acc = peer_sum(mm, valid ? to_fix((double)wt, p.inv_scale) : 0ll);
         // weight to the own community
-        unsigned ob = __ballot_sync(FULL, leader && cu == own) & gmask;
+        const unsigned ob = __ballot_sync(FULL, leader && cu == own) & gmask;
         long long wof = __shfl_sync(FULL, acc, ob ? (__ffs(ob) - 1) : lane);
         if (!ob) wof = 0;
-        double base = 0.0;
-        if (eligible) {
-            base = gain_of(p, q, from_fix(wof, p.scale), sl, k, from_fix(ro(p.Kf + (own)) - kf, p.scale), a,
-                           (p.need_nc ? from_fix(ro(p.Wf + (own)) - af, p.nscale) : 0.0));
+        // candidates are held by leader lanes; two other lanes of the group take
+        // the own and the fresh community
+        const bool other = leader && cu != own;
+        scand += other ? 1ull : 0ull;
+        const unsigned idle = gmask & ~__ballot_sync(FULL, other), idle2 = idle & (idle - 1);
+        double gain = 0.0, base, ge;
+        if (__all_sync(FULL, idle2 != 0u || !eligible)) {
+            const int ol = idle ? __ffs(idle) - 1 : lane, fl = idle2 ? __ffs(idle2) - 1 : lane;
+            if (eligible && (other || lane == ol || (!REFINE && lane == fl))) {
+                const bool is_own = lane == ol, is_fresh = !other && !is_own;
+                const uint32_t cc = other ? cu : own;
+                const double kc = is_fresh ? 0.0 : from_fix(ro(p.Kf + cc) - (is_own ? kf : 0ll), p.scale);
+                const double nc =
+                    p.need_nc && !is_fresh ? from_fix(ro(p.Wf + cc) - (is_own ? af : 0ll), p.nscale) : 0.0;
+                const double wto = is_fresh ? 0.0 : from_fix(is_own ? wof : acc, p.scale);
+                gain = gain_of(p, q, wto, sl, k, kc, a, nc);
+                // max_community_weight: a candidate past the cap is none
+                if (other && p.has_limit && !(__dadd_rn(nc, a) <= p.limit)) gain = -INFINITY;
+            }
+            base = __shfl_sync(FULL, gain, ol);
+            ge = __shfl_sync(FULL, gain, fl);
+        } else {
+            // a group whose every lane holds a candidate: the two before the others
+            base = ge = 0.0;
+            if (eligible) {
+                const bool is_own = !(sub & 1);
+                const double kc = is_own ? from_fix(ro(p.Kf + own) - kf, p.scale) : 0.0;
+                const double nc = p.need_nc && is_own ? from_fix(ro(p.Wf + own) - af, p.nscale) : 0.0;
+                gain = gain_of(p, q, is_own ? from_fix(wof, p.scale) : 0.0, sl, k, kc, a, nc);
+            }
+            base = __shfl_sync(FULL, gain, gbase);
+            ge = __shfl_sync(FULL, gain, gbase + 1);
+            if (other) {
+                const double nc = (p.need_nc ? from_fix(ro(p.Wf + (cu)), p.nscale) : 0.0);
+                gain = gain_of(p, q, from_fix(acc, p.scale), sl, k, from_fix(ro(p.Kf + (cu)), p.scale), a, nc);
+                if (p.has_limit && !(__dadd_rn(nc, a) <= p.limit)) gain = -INFINITY;
+            }
         }
-        // candidates held by leader lanes
         double g = -INFINITY;
         uint32_t c = NONE32, cu_member = NONE32;
-        bool cand = false;
-        if (leader && cu != own) {
-            double nc = (p.need_nc ? from_fix(ro(p.Wf + (cu)), p.nscale) : 0.0);
-            if (!p.has_limit || __dadd_rn(nc, a) <= p.limit) {
-                g = gain_of(p, q, from_fix(acc, p.scale), sl, k, from_fix(ro(p.Kf + (cu)), p.scale), a, nc);
-                if (REFINE) {
-                    double rel = __dsub_rn(g, base);
-                    if (rel >= 0.0) {  // `>=` takes ties (refine.rs:91-95)
-                        cand = true;
-                        g = refine_key(p, q, rel, v - q.base, cu - q.base);
-                    } else {
-                        g = -INFINITY;
-                    }
-                } else {
-                    cand = true;
-                }
-                if (cand) {
-                    c = cu;
-                    cu_member = u;
-                }
+        if (other && gain != -INFINITY) {
+            g = gain;
+            if (REFINE) {
+                const double rel = __dsub_rn(gain, base);
+                // `>=` takes ties (refine.rs:91-95)
+                g = rel >= 0.0 ? refine_key(p, q, rel, v - q.base, cu - q.base) : -INFINITY;
+            }
+            if (!REFINE || g != -INFINITY) {
+                c = cu;
+                cu_member = u;
             }
         }
         if (sub == 0 && eligible) {
             snodes += 1;
             sdeg += (unsigned long long)deg;
         }
-        scand += (leader && cu != own) ? 1ull : 0ull;
         // argmax over the group: higher key, then lower id
 #pragma unroll
         for (int o = G / 2; o; o >>= 1) {
@@ -164,15 +212,9 @@ __global__ void __launch_bounds__(TB, 4) k_decide_small(Params p, const uint32_t
                     best = c;
                     bg = g;
                 }
-                // one empty community per node (local_move.rs:92-100)
-                const uint32_t fresh = (uint32_t)(p.S0 + v);
-                if (fresh != own && ro(p.csize + (own)) > 1 && ro(p.csize + (fresh)) == 0 &&
-                    (!p.has_limit || a <= p.limit)) {
-                    double ge = gain_of(p, q, 0.0, sl, k, 0.0, a, 0.0);
-                    if (better(ge, fresh, bg, best)) {
-                        best = fresh;
-                        bg = ge;
-                    }
+                if (try_fresh && better(ge, fresh, bg, best)) {
+                    best = fresh;
+                    bg = ge;
                 }
                 double d = __dsub_rn(bg, base);
                 if (best != own && d > q.thr) {
@@ -191,11 +233,10 @@ __global__ void __launch_bounds__(TB, 4) k_decide_small(Params p, const uint32_t
             p.epoch[v] = p.cur;
         }
     }
-    warp_add(p.counters + 1, sdeg);
-    warp_add(p.counters + 2, scand);
-    warp_add(p.counters + 3, snodes);
+    flush_counters(p.counters, sdeg, scand, snodes);
 }
 
+// ------------------------------------------------------------ large-degree decide
 // One warp per node of degree 33..WARP_DEGREE: an open-addressing hash of
 // neighbour communities in this warp's slice of shared memory, gains scored
 // by every lane over its slots, warp argmax.
@@ -266,24 +307,41 @@ __global__ void __launch_bounds__(32 * WARPS_PER_BLOCK) k_decide_warp(Params p, 
         if (lane == 0) s_cnt[wib] = 0;
         __syncwarp();
         const uint32_t cv = REFINE ? ro(p.constraint + (v)) : 0;
-        for (uint64_t base0 = b; base0 < e; base0 += 32) {  // warp-uniform trip count
-            const uint64_t j = base0 + lane;
-            const bool first = base0 == b;
-            bool ok = j < e;
-            uint32_t u = 0;
-            float wj = 0.0f;
-            if (ok) {
-                u = first ? u_first : ro(p.nbr + (j));
-                wj = first ? w_first : ro(p.w + (j));
+        // four chunks' gathers are in flight before any of them enters the table:
+        // one chunk at a time, each waited for two round trips of its own
+        for (uint64_t base0 = b; base0 < e; base0 += 128) {  // warp-uniform trip count
+            uint32_t u[4], cu[4];
+            float w[4];
+            bool ok[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const uint64_t j = base0 + 32 * t + lane;
+                ok[t] = j < e;
+                u[t] = v;
+                w[t] = 0.0f;
+                if (t == 0 && base0 == b) {
+                    u[t] = ok[t] ? u_first : v;
+                    w[t] = w_first;
+                } else if (ok[t]) {
+                    u[t] = ro(p.nbr + (j));
+                    w[t] = ro(p.w + (j));
+                }
             }
-            ok = ok && u != v;
-            if (REFINE && ok) ok = ro(p.constraint + (u)) == cv;
-            const uint32_t cu = ok ? ro(p.memb + (u)) : 0u;
-            const uint64_t key = ok ? (uint64_t)cu : (0xFFFFFFFF00000000ull | lane);
-            const unsigned peers = __match_any_sync(FULL, key);
-            const long long x = peer_sum(peers, ok ? to_fix((double)wj, p.inv_scale) : 0ll);
-            if (ok && __ffs(peers) - 1 == lane)
-                hinsert_listed(keys, vals, mask, cu, x, p.status, s_list[wib], &s_cnt[wib], WARP_DEGREE);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                ok[t] = ok[t] && u[t] != v;
+                if (REFINE && ok[t]) ok[t] = ro(p.constraint + (u[t])) == cv;
+                cu[t] = ok[t] ? ro(p.memb + (u[t])) : 0u;
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                if (base0 + 32 * t >= e) break;  // warp-uniform
+                const uint64_t key = ok[t] ? (uint64_t)cu[t] : (0xFFFFFFFF00000000ull | lane);
+                const unsigned peers = __match_any_sync(FULL, key);
+                const long long x = peer_sum(peers, ok[t] ? to_fix((double)w[t], p.inv_scale) : 0ll);
+                if (ok[t] && __ffs(peers) - 1 == lane)
+                    hinsert_listed(keys, vals, mask, cu[t], x, p.status, s_list[wib], &s_cnt[wib], WARP_DEGREE);
+            }
         }
         fetch_chunk();
         __syncwarp();
@@ -374,9 +432,7 @@ __global__ void __launch_bounds__(32 * WARPS_PER_BLOCK) k_decide_warp(Params p, 
         }
         __syncwarp();
     }
-    warp_add(p.counters + 1, sdeg);
-    warp_add(p.counters + 2, scand);
-    warp_add(p.counters + 3, snodes);
+    flush_counters(p.counters, sdeg, scand, snodes);
 }
 
 // One block per node. HUB = false: degree <= HUB_DEGREE, hash table in shared
@@ -431,18 +487,33 @@ __global__ void __launch_bounds__(TB) k_decide_block(Params p, const uint32_t* _
         const uint32_t cv = REFINE ? ro(p.constraint + (v)) : 0;
         {
             const unsigned lane = threadIdx.x & 31u;
-            // each warp walks its own 32-entry chunks: trip counts are warp-uniform
-            for (uint64_t base0 = b + (threadIdx.x & ~31u); base0 < e; base0 += blockDim.x) {
-                const uint64_t j = base0 + lane;
-                bool ok = j < e;
-                const uint32_t u = ok ? ro(p.nbr + (j)) : 0u;
-                ok = ok && u != v;
-                if (REFINE && ok) ok = ro(p.constraint + (u)) == cv;
-                const uint32_t cu = ok ? ro(p.memb + (u)) : 0u;
-                const uint64_t key = ok ? (uint64_t)cu : (0xFFFFFFFF00000000ull | lane);
-                const unsigned peers = __match_any_sync(0xFFFFFFFFu, key);
-                const long long x = peer_sum(peers, ok ? to_fix((double)ro(p.w + (j)), p.inv_scale) : 0ll);
-                if (ok && __ffs(peers) - 1 == (int)lane) hinsert(keys, vals, mask, cu, x, p.status);
+            // each warp walks its own 32-entry chunks, four in flight: trip counts are warp-uniform
+            const uint64_t stride = blockDim.x;
+            for (uint64_t base0 = b + (threadIdx.x & ~31u); base0 < e; base0 += 4 * stride) {
+                uint32_t u[4], cu[4];
+                float w[4];
+                bool ok[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const uint64_t j = base0 + t * stride + lane;
+                    ok[t] = j < e;
+                    u[t] = ok[t] ? ro(p.nbr + (j)) : v;
+                    w[t] = ok[t] ? ro(p.w + (j)) : 0.0f;
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    ok[t] = ok[t] && u[t] != v;
+                    if (REFINE && ok[t]) ok[t] = ro(p.constraint + (u[t])) == cv;
+                    cu[t] = ok[t] ? ro(p.memb + (u[t])) : 0u;
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    if (base0 + t * stride >= e) break;  // warp-uniform
+                    const uint64_t key = ok[t] ? (uint64_t)cu[t] : (0xFFFFFFFF00000000ull | lane);
+                    const unsigned peers = __match_any_sync(0xFFFFFFFFu, key);
+                    const long long x = peer_sum(peers, ok[t] ? to_fix((double)w[t], p.inv_scale) : 0ll);
+                    if (ok[t] && __ffs(peers) - 1 == (int)lane) hinsert(keys, vals, mask, cu[t], x, p.status);
+                }
             }
         }
         __syncthreads();
@@ -524,12 +595,7 @@ __global__ void __launch_bounds__(TB) k_decide_block(Params p, const uint32_t* _
         }
         __syncthreads();
     }
-    // block-level counter flush (thread 0 holds the node and degree counts)
-    atomicAdd(p.counters + 2, scand);
-    if (threadIdx.x == 0) {
-        atomicAdd(p.counters + 1, sdeg);
-        atomicAdd(p.counters + 3, snodes);
-    }
+    flush_counters(p.counters, sdeg, scand, snodes);
 }
 
 // ------------------------------------------------------------ commit
@@ -572,49 +638,76 @@ __global__ void k_apply(Params p, const uint32_t* __restrict__ list, uint32_t co
 // commit, so every membership it reads is final.
 // A node enters the next sweep's list once: its stamp is raised to `mark` (the
 // next sweep's number + 1) and only the lane that raised it appends it.
-// Half a warp per node (k-NN rows hold 10-30 entries, so a whole warp per row
-// would leave most lanes idle); both halves walk max(their chunk counts) chunks
-// so that the ballot and the shuffle see every lane.
-__global__ void k_activate(Params p, const uint32_t* __restrict__ list, uint32_t count, uint32_t* stamp,
-                           uint32_t mark, uint32_t* next_list, uint32_t* next_count) {
+// A warp takes `window` list entries, a lane each, and then the rows of those
+// that moved, two at a time (k-NN rows hold 10-30 entries, so half a warp a row).
+// What it appends gathers in a queue of its own in shared memory and goes out
+// with one atomic per some hundred entries: one returning atomic on the one
+// counter for every 16 entries of a row was what bound it (318 us for the first
+// batch of a 1M x 30 graph, 156 now).
+constexpr int ACT_QUEUE = 320;  // entries of a warp's queue: a step adds up to 32
+__global__ void __launch_bounds__(TB) k_activate(Params p, const uint32_t* __restrict__ list, uint32_t count,
+                                                 uint32_t window, uint32_t* stamp, uint32_t mark, uint32_t* next_list,
+                                                 uint32_t* next_count) {
+    __shared__ uint32_t s_queue[TB / 32][ACT_QUEUE];
     const unsigned FULL = 0xFFFFFFFFu;
     const unsigned lane = threadIdx.x & 31u, half = lane >> 4, sub = lane & 15u;
+    uint32_t* queue = s_queue[threadIdx.x >> 5];
+    uint32_t queued = 0;  // warp-uniform
+    auto flush = [&]() {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(next_count, queued);
+        base = __shfl_sync(FULL, base, 0);
+        for (uint32_t i = lane; i < queued; i += 32) next_list[base + i] = queue[i];
+        __syncwarp();
+        queued = 0;
+    };
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i0 = warp * 2; i0 < count; i0 += nwarps * 2) {  // warp-uniform
-        const uint64_t i = i0 + half;
-        uint32_t v = 0, t = 0;
-        uint64_t b = 0, e = 0;
-        if (i < count) {
-            v = list[i];
-            if (p.moved[v] == p.cur) {
-                t = p.memb[v];
-                b = p.ptr[v];
-                e = p.ptr[v + 1];
+    for (uint64_t i0 = warp * window; i0 < count; i0 += nwarps * window) {  // warp-uniform
+        const uint64_t i = i0 + lane;
+        uint32_t mv = 0, mt = 0, md = 0;
+        uint64_t mb = 0;
+        bool moved = false;
+        if (lane < window && i < count) {
+            mv = list[i];
+            moved = p.moved[mv] == p.cur;
+            if (moved) {
+                mt = p.memb[mv];
+                mb = p.ptr[mv];
+                md = (uint32_t)(p.ptr[mv + 1] - mb);
             }
         }
-        const uint64_t my_chunks = (e - b + 15) >> 4;
-        const uint64_t chunks = max(my_chunks, __shfl_xor_sync(FULL, my_chunks, 16));
-        for (uint64_t ch = 0; ch < chunks; ++ch) {
-            const uint64_t j = b + ch * 16 + sub;
-            uint32_t u = 0;
-            bool add = false;
-            if (j < e) {
-                u = p.nbr[j];
-                // a plain read first: a node already queued for the next sweep
-                // (the common case once many of its neighbours moved) costs no atomic
-                add = u != v && p.memb[u] != t && stamp[u] < mark && atomicMax(stamp + u, mark) < mark;
-            }
-            const unsigned bal = __ballot_sync(FULL, add);
-            if (bal) {
-                const int leader = __ffs(bal) - 1;
-                uint32_t base = 0;
-                if ((int)lane == leader) base = atomicAdd(next_count, (uint32_t)__popc(bal));
-                base = __shfl_sync(FULL, base, leader);
-                if (add) next_list[base + __popc(bal & ((1u << lane) - 1u))] = u;
+        unsigned todo = __ballot_sync(FULL, moved);
+        while (todo) {  // the lowest two of the moved nodes, half a warp each
+            const unsigned rest = todo & (todo - 1);
+            const int L0 = __ffs(todo) - 1, L1 = rest ? __ffs(rest) - 1 : L0;
+            todo = rest & (rest - 1);
+            const int L = half ? L1 : L0;
+            const uint32_t v = __shfl_sync(FULL, mv, L), t = __shfl_sync(FULL, mt, L);
+            uint32_t d = __shfl_sync(FULL, md, L);
+            const uint64_t b = __shfl_sync(FULL, mb, L);
+            if (half && !rest) d = 0;
+            const uint32_t most = max(d, __shfl_xor_sync(FULL, d, 16));
+            for (uint32_t j0 = 0; j0 < most; j0 += 16) {
+                uint32_t u = 0;
+                bool add = false;
+                if (j0 + sub < d) {
+                    u = p.nbr[b + j0 + sub];
+                    // a plain read first: a node already queued for the next sweep
+                    // (the common case once many of its neighbours moved) costs no atomic
+                    add = u != v && p.memb[u] != t && stamp[u] < mark && atomicMax(stamp + u, mark) < mark;
+                }
+                const unsigned bal = __ballot_sync(FULL, add);
+                if (bal) {
+                    if (add) queue[queued + __popc(bal & ((1u << lane) - 1u))] = u;
+                    queued += __popc(bal);
+                    __syncwarp();
+                    if (queued > ACT_QUEUE - 32) flush();
+                }
             }
         }
     }
+    if (queued) flush();
 }
 
 template <bool MULTI>
@@ -672,41 +765,64 @@ __global__ void k_bucket_count(const uint64_t* __restrict__ ptr, const uint32_t*
         if (sc[t]) atomicAdd(counts + t, sc[t]);
 }
 
-// One warp-aggregated atomic per distinct (batch, bucket) per warp.
+// SCATTER_ITEMS entries a thread: their places inside the block's share of each
+// (batch, bucket) list come from counters in shared memory, the share from one
+// atomic per list and block (one per distinct list and warp kept the dozen
+// cursors busy: 3.4 ms of a 4M-point run, 1.0 now).
+constexpr int SCATTER_ITEMS = 4;
 template <bool MULTI>
-__global__ void k_bucket_scatter(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ alist,
-                                 const uint32_t* __restrict__ acount, uint64_t n, uint64_t seed, uint32_t sweep,
-                                 int B, Route route, uint32_t* cursor, uint32_t* list, uint64_t* lbeg,
-                                 uint32_t* ldeg, const uint32_t* inst, const InstCfg* icfg) {
+__global__ void __launch_bounds__(TB)
+    k_bucket_scatter(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ alist,
+                     const uint32_t* __restrict__ acount, uint64_t n, uint64_t seed, uint32_t sweep, int B, Route route,
+                     uint32_t* cursor, uint32_t* list, uint64_t* lbeg, uint32_t* ldeg, const uint32_t* inst,
+                     const InstCfg* icfg) {
+    __shared__ uint32_t s_cnt[MAX_SLOTS], s_base[MAX_SLOTS];
     const unsigned lane = threadIdx.x & 31u;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const int slots = B * NBUCKET;
     const uint64_t m = alist ? *acount : n;
-    for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) - lane; base < m; base += stride) {
-        const uint64_t i = base + lane;
-        const uint64_t v = i < m ? (alist ? alist[i] : i) : 0;
-        int slot = -1;
-        uint64_t rb = 0;
-        uint32_t deg = 0;
-        if (i < m) {
-            const int b = batch_of<MULTI>(seed, sweep, v, B, inst, icfg);
-            if (b >= 0) {
-                rb = ptr[v];
-                deg = (uint32_t)(ptr[v + 1] - rb);
-                int k = bucket_of(deg, route);
-                slot = b * NBUCKET + k;
+    for (uint64_t base = blockIdx.x * (uint64_t)(TB * SCATTER_ITEMS); base < m;
+         base += (uint64_t)gridDim.x * (TB * SCATTER_ITEMS)) {  // block-uniform
+        for (int t = threadIdx.x; t < slots; t += TB) s_cnt[t] = 0;
+        __syncthreads();
+        uint32_t v[SCATTER_ITEMS], deg[SCATTER_ITEMS], rank[SCATTER_ITEMS];
+        uint64_t rb[SCATTER_ITEMS];
+        int slot[SCATTER_ITEMS];
+#pragma unroll
+        for (int t = 0; t < SCATTER_ITEMS; ++t) {
+            const uint64_t i = base + t * TB + threadIdx.x;
+            slot[t] = -1;
+            v[t] = deg[t] = 0;
+            rb[t] = 0;
+            if (i < m) {
+                v[t] = alist ? alist[i] : (uint32_t)i;
+                const int b = batch_of<MULTI>(seed, sweep, v[t], B, inst, icfg);
+                if (b >= 0) {
+                    rb[t] = ptr[v[t]];
+                    deg[t] = (uint32_t)(ptr[v[t] + 1] - rb[t]);
+                    slot[t] = b * NBUCKET + bucket_of(deg[t], route);
+                }
             }
         }
-        const unsigned mm = __match_any_sync(0xFFFFFFFFu, slot < 0 ? 1000 + (int)lane : slot);
-        const int leader = __ffs(mm) - 1;
-        uint32_t pos0 = 0;
-        if (slot >= 0 && (int)lane == leader) pos0 = atomicAdd(cursor + slot, (uint32_t)__popc(mm));
-        pos0 = __shfl_sync(0xFFFFFFFFu, pos0, leader);
-        if (slot >= 0) {
-            const uint32_t pos = pos0 + __popc(mm & ((1u << lane) - 1u));
-            list[pos] = (uint32_t)v;
-            lbeg[pos] = rb;
-            ldeg[pos] = deg;
+#pragma unroll
+        for (int t = 0; t < SCATTER_ITEMS; ++t) {
+            const unsigned mm = __match_any_sync(0xFFFFFFFFu, slot[t] < 0 ? 1000 + (int)lane : slot[t]);
+            const int leader = __ffs(mm) - 1;
+            uint32_t first = 0;
+            if (slot[t] >= 0 && (int)lane == leader) first = atomicAdd(&s_cnt[slot[t]], (uint32_t)__popc(mm));
+            rank[t] = __shfl_sync(0xFFFFFFFFu, first, leader) + __popc(mm & ((1u << lane) - 1u));
         }
+        __syncthreads();
+        for (int t = threadIdx.x; t < slots; t += TB) s_base[t] = s_cnt[t] ? atomicAdd(cursor + t, s_cnt[t]) : 0u;
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < SCATTER_ITEMS; ++t) {
+            if (slot[t] < 0) continue;
+            const uint32_t pos = s_base[slot[t]] + rank[t];
+            list[pos] = v[t];
+            lbeg[pos] = rb[t];
+            ldeg[pos] = deg[t];
+        }
+        __syncthreads();  // s_cnt and s_base are reused
     }
 }
 
@@ -888,17 +1004,23 @@ void launch_decide(Ctx& c, Params& p, Workspace& ws, int k, uint32_t off, uint32
     const uint32_t* list = ws.list.get() + off;
     const uint64_t* lbeg = ws.lbeg.get() + off;
     const uint32_t* ldeg = ws.ldeg.get() + off;
+    // twice what the SMs hold at once: the warps go on to their next node, whose
+    // row they have prefetched, and a late block still finds work. Level 0 of a 4M
+    // graph, local moving: 40.8 / 39.0 / 38.8 / 40.1 ms with 4 / 8 / 16 / 64 blocks
+    // an SM of the lane-group kernels, 39.7 / 39.0 / 38.7 with 7 / 14 / 64 of the
+    // warp kernel (its refinement 4.6 / 4.4 / 4.6).
+    const unsigned small_grid = (unsigned)c.sm_count * 8u, warp_grid = (unsigned)c.sm_count * 14u;
     if (k == 0) {
         unsigned warps = (cnt + 3) / 4;
-        k_decide_small<8, REFINE, MULTI><<<grid_for((uint64_t)warps * 32, TB, 148u * 64u), TB, 0, st>>>(p, list, lbeg, ldeg, cnt);
+        k_decide_small<8, REFINE, MULTI><<<grid_for((uint64_t)warps * 32, TB, small_grid), TB, 0, st>>>(p, list, lbeg, ldeg, cnt);
     } else if (k == 1) {
         unsigned warps = (cnt + 1) / 2;
-        k_decide_small<16, REFINE, MULTI><<<grid_for((uint64_t)warps * 32, TB, 148u * 64u), TB, 0, st>>>(p, list, lbeg, ldeg, cnt);
+        k_decide_small<16, REFINE, MULTI><<<grid_for((uint64_t)warps * 32, TB, small_grid), TB, 0, st>>>(p, list, lbeg, ldeg, cnt);
     } else if (k == 2) {
-        k_decide_small<32, REFINE, MULTI><<<grid_for((uint64_t)cnt * 32, TB, 148u * 64u), TB, 0, st>>>(p, list, lbeg, ldeg, cnt);
+        k_decide_small<32, REFINE, MULTI><<<grid_for((uint64_t)cnt * 32, TB, small_grid), TB, 0, st>>>(p, list, lbeg, ldeg, cnt);
     } else if (k == 3) {
         const uint64_t warps = cnt;
-        k_decide_warp<REFINE, MULTI><<<grid_for(warps * 32, 32 * WARPS_PER_BLOCK, 148u * 64u), 32 * WARPS_PER_BLOCK, 0,
+        k_decide_warp<REFINE, MULTI><<<grid_for(warps * 32, 32 * WARPS_PER_BLOCK, warp_grid), 32 * WARPS_PER_BLOCK, 0,
                                 st>>>(p, list, lbeg, ldeg, cnt);
     } else if (k == 4) {
         size_t sm = HCAP_SMEM * (sizeof(long long) + sizeof(uint32_t));
@@ -1001,11 +1123,11 @@ void launch_bucket_scatter(Ctx& c, const Params& p, const DevGraph& g, const uin
                            Workspace& ws) {
     const uint64_t n = g.n;
     if (p.inst)
-        k_bucket_scatter<true><<<grid_for(work, TB), TB, 0, c.stream>>>(g.ptr, alist, acount, n, seed, sweep, B,
+        k_bucket_scatter<true><<<grid_for(work, TB * SCATTER_ITEMS), TB, 0, c.stream>>>(g.ptr, alist, acount, n, seed, sweep, B,
                                                                         route_of(c), ws.cursor.get(), ws.list.get(),
                                                                         ws.lbeg.get(), ws.ldeg.get(), p.inst, p.icfg);
     else
-        k_bucket_scatter<false><<<grid_for(work, TB), TB, 0, c.stream>>>(g.ptr, alist, acount, n, seed, sweep, B,
+        k_bucket_scatter<false><<<grid_for(work, TB * SCATTER_ITEMS), TB, 0, c.stream>>>(g.ptr, alist, acount, n, seed, sweep, B,
                                                                          route_of(c), ws.cursor.get(), ws.list.get(),
                                                                          ws.lbeg.get(), ws.ldeg.get(), nullptr, nullptr);
     SC_LAUNCH_CHECK();
@@ -1159,8 +1281,11 @@ MoveResult local_move(Ctx& c, const DevGraph& g, Workspace& ws, uint32_t* memb, 
                 SC_CUDA(cudaStreamWaitEvent(c.aux, c.ev_aux_start, 0));
                 as = c.aux;
             }
-            k_activate<<<grid_for((uint64_t)(hi - lo) * 16, TB, 148u * 64u), TB, 0, as>>>(
-                p, ws.list.get() + lo, hi - lo, ws.stamp.get(), sweep + 2, ws.nlist.get(), ws.ncount.get());
+            // two entries a warp while that leaves warps idle, up to 32
+            const uint32_t act_warps = (uint32_t)c.sm_count * 32u;
+            const uint32_t window = std::min<uint32_t>(32, std::max<uint32_t>(2, (hi - lo) / act_warps));
+            k_activate<<<grid_for((uint64_t)((hi - lo + window - 1) / window) * 32, TB, 148u * 32u), TB, 0, as>>>(
+                p, ws.list.get() + lo, hi - lo, window, ws.stamp.get(), sweep + 2, ws.nlist.get(), ws.ncount.get());
             if (overlap) {
                 SC_CUDA(cudaEventRecord(c.ev_aux_done, c.aux));
                 act_pending = true;
