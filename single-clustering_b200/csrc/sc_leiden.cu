@@ -733,16 +733,6 @@ __device__ __forceinline__ int bucket_of(uint32_t deg, Route r) {
     return deg <= r.g8 ? 0 : deg <= r.g16 ? 1 : deg <= r.g32 ? 2 : deg <= WARP_DEGREE ? 3 : deg <= HUB_DEGREE ? 4 : 5;
 }
 
-// The hash batch of node v in a sweep, or -1 for a node of a frozen instance.
-template <bool MULTI>
-__device__ __forceinline__ int batch_of(uint64_t seed, uint32_t sweep, uint64_t v, int B, const uint32_t* inst,
-                                        const InstCfg* icfg) {
-    if (!MULTI) return (int)(hash3(seed, sweep, v) % (uint64_t)B);
-    const InstCfg& c = icfg[inst[v]];
-    if (c.frozen) return -1;
-    return (int)(hash3(c.seed, sweep, v - c.base) % (uint64_t)B);
-}
-
 // The nodes of a sweep: alist[0 .. *acount) or, with alist == nullptr, all n.
 template <bool MULTI>
 __global__ void k_bucket_count(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ alist,
@@ -1222,6 +1212,7 @@ MoveResult local_move(Ctx& c, const DevGraph& g, Workspace& ws, uint32_t* memb, 
     unsigned long long last_ctr[4] = {0, 0, 0, 0};
     long long last_gacc = 0;
     bool read_fresh = false;  // last_ctr / last_gacc hold the counters' current values
+    const uint32_t tail = tail_limit(c, g, cfg);
     for (uint32_t sweep = 0; sweep < (uint32_t)MAX_SWEEPS; ++sweep) {
         zero(c, ws.counts.get(), B * NBUCKET);
         zero(c, ws.ncount.get(), 1);
@@ -1252,6 +1243,25 @@ MoveResult local_move(Ctx& c, const DevGraph& g, Workspace& ws, uint32_t* memb, 
         moves_before = ctr[0];
         if (offs[B * NBUCKET] == 0) break;
         read_fresh = false;
+        // few enough active nodes for the team: a sweep of them costs a dozen
+        // launches and a read-back here, 20 to 40 us there
+        if (offs[B * NBUCKET] <= tail && (!all_active || n <= tail)) {
+            uint32_t* const lists[2] = {ws.alist.get(), ws.nlist.get()};
+            uint32_t* const cnts[2] = {ws.acount.get(), ws.ncount.get()};
+            const TailResult t = tail_run(c, &p, (uint32_t)n, alist, lists, cnts, ws.stamp.get(), sweep, epoch,
+                                          moves_before, budget);
+            r.sweeps += t.swept;
+            if (t.done) break;
+            if (t.swapped) {
+                std::swap(ws.alist, ws.nlist);
+                std::swap(ws.acount, ws.ncount);
+            }
+            all_active = false;
+            epoch = t.epoch;
+            moves_before = t.moves_before;
+            sweep = t.sweep - 1;
+            continue;
+        }
         h2d(c, ws.cursor.get(), offs, B * NBUCKET);
         launch_bucket_scatter(c, p, g, alist, ws.acount.get(), all_active ? n : offs[B * NBUCKET], seed, sweep, B,
                               ws);
@@ -1299,7 +1309,7 @@ MoveResult local_move(Ctx& c, const DevGraph& g, Workspace& ws, uint32_t* memb, 
         all_active = false;
         r.sweeps++;
     }
-    if (!read_fresh) {  // the sweep limit ended the loop after launching a sweep
+    if (!read_fresh) {  // the team, or the sweep limit after launching a sweep, ended the loop
         Mailbox mb(c);
         const unsigned long long* hk = mb.get(ws.counters.get(), 4);
         const long long* hg = mb.get(ws.gain_acc.get(), 1);

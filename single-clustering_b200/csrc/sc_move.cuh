@@ -168,6 +168,16 @@ __device__ __forceinline__ double refine_key(const Params& p, const NodeCfg& q, 
     return __dadd_rn(__ddiv_rn(rel, q.theta), -log(-log(u)));
 }
 
+// The hash batch of node v in a sweep, or -1 for a node of a frozen instance.
+template <bool MULTI>
+__device__ __forceinline__ int batch_of(uint64_t seed, uint32_t sweep, uint64_t v, int B, const uint32_t* inst,
+                                        const InstCfg* icfg) {
+    if (!MULTI) return (int)(hash3(seed, sweep, v) % (uint64_t)B);
+    const InstCfg& c = icfg[inst[v]];
+    if (c.frozen) return -1;
+    return (int)(hash3(c.seed, sweep, v - c.base) % (uint64_t)B);
+}
+
 // Read-only load (ld.global.nc): the decide kernels never write the graph, the
 // membership or the community aggregates they read; only the commit kernels do.
 template <class T>

@@ -33,6 +33,7 @@ constexpr uint32_t TEAM_CLUSTER = 16;
 // block cost less than the cluster's (64 against 16: 0.74 and 0.78 ms there).
 constexpr uint32_t SOLO_NODES = 64;
 constexpr uint64_t SOLO_ENTRIES = 4096;
+constexpr uint32_t TAIL_NODES_PER_BLOCK = 384;  // active nodes a block, up to which the last sweeps are the team's
 constexpr uint32_t TEAM_BIG = TEAM_MAX_NODES / 8;  // rows past a warp's table, per block (8 blocks at least, or one of SOLO_NODES)
 constexpr uint32_t GROUPS = 4;  // nodes a block decides side by side (decide_group)
 constexpr uint32_t SLOTS_MAX = 2 * TEAM_MAX_NODES;  // community ids of a level: the partition's and one fresh per node
@@ -122,7 +123,7 @@ struct TeamSmem {
     };
     uint32_t big[TEAM_BIG];
     uint4 item[TEAM_BIG];  // node, row start, degree, community
-    uint32_t nbig, nitem, next;
+    uint32_t nbig, bigmax, nitem, next;
     uint32_t wcnt[TEAM_WARPS];
     unsigned long long wsum[TEAM_WARPS];
     unsigned long long total;
@@ -238,7 +239,7 @@ __device__ __forceinline__ double key_of(const Params& p, const NodeCfg& q, uint
                                          double base) {
     if (!REFINE) return gain;
     const double rel = __dsub_rn(gain, base);
-    return rel >= 0.0 ? refine_key(p, q, rel, v, cu) : -INFINITY;
+    return rel >= 0.0 ? refine_key(p, q, rel, v - q.base, cu - q.base) : -INFINITY;
 }
 
 // The choice from the best candidate (g, c): the target, or NONE32; *gain its
@@ -278,12 +279,12 @@ __device__ __forceinline__ void warp_best(double& g, uint32_t& c) {
 
 // One warp decides node v (row at b, deg <= WARP_DEGREE). Returns the number of
 // candidate communities (the same in every lane).
-template <bool REFINE>
+template <bool REFINE, bool MULTI>
 __device__ uint32_t decide_warp(const Params& p, uint32_t v, uint64_t b, uint32_t deg, uint32_t own, WarpTable& t,
                                 uint32_t* s_cnt) {
     const unsigned FULL = 0xFFFFFFFFu;
     const unsigned lane = threadIdx.x & 31u;
-    const NodeCfg q = node_cfg<false>(p, v);
+    const NodeCfg q = node_cfg<MULTI>(p, v);
     const uint32_t cv = REFINE ? p.constraint[v] : 0u;
     double g = -INFINITY;
     uint32_t c = NONE32, ncand;
@@ -422,31 +423,45 @@ __device__ uint32_t decide_warp(const Params& p, uint32_t v, uint64_t b, uint32_
     return ncand;
 }
 
-// A group of warps decides node v (any degree) with one accumulator per
-// community id (ids < slots): no probing, no table size to fit, and stored
-// weights are positive, so a zero sum means no entry. A quarter of the block
-// where a quarter of the accumulators hold the level's ids, so that four nodes'
-// latencies overlap, else the whole block.
+// A group of warps decides node v (longer rows than a warp takes): a quarter of
+// the block, so that four nodes' latencies overlap, or the whole block. With
+// DENSE it keeps one accumulator per community id (ids < slots): no probing, no
+// table size to fit, and stored weights are positive, so a zero sum means no
+// entry; a quarter of the block holds a quarter of the ids. Without (the ids of
+// a large level) a hash table twice the degree.
 struct Group {
     uint32_t id, threads;  // named barrier 1 + id; threads of the group
     __device__ uint32_t tid() const { return threadIdx.x % threads; }
     __device__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(1 + id), "r"(threads) : "memory"); }
 };
+constexpr uint32_t GROUP_BYTES = SLOTS_MAX / GROUPS * sizeof(long long);
+constexpr uint32_t GROUP_DEGREE = 1024;  // longest row of a quarter's table, and of the block's
+constexpr uint32_t BLOCK_DEGREE = 4096;
+static_assert(2 * GROUP_DEGREE * 12 <= GROUP_BYTES && 2 * BLOCK_DEGREE * 12 <= GROUPS * GROUP_BYTES,
+              "a table of twice the degree fits the accumulators' memory");
 
-template <bool REFINE>
+template <bool REFINE, bool MULTI, bool DENSE>
 __device__ uint32_t decide_group(const Params& p, uint32_t v, uint32_t slots, TeamSmem& s, const Group& grp) {
     const unsigned FULL = 0xFFFFFFFFu;
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t tid = grp.tid(), warps = grp.threads / 32;
-    long long* dense = s.dense + grp.id * (SLOTS_MAX / GROUPS);
     double* red_g = s.red_g + grp.id * (32 / GROUPS);  // a group of the whole block has id 0
     uint32_t* red_c = s.red_c + grp.id * (32 / GROUPS);
     const uint64_t b = p.ptr[v], e = p.ptr[v + 1];
     const uint32_t own = p.memb[v];
-    const NodeCfg q = node_cfg<false>(p, v);
+    const NodeCfg q = node_cfg<MULTI>(p, v);
     const NodeSide side = node_side<REFINE>(p, v, own);
     const uint32_t cv = REFINE ? p.constraint[v] : 0u;
-    for (uint32_t i = tid; i < slots; i += grp.threads) dense[i] = 0;
+    if (!DENSE) {
+        slots = 64;
+        while (slots < 2 * (uint32_t)(e - b)) slots <<= 1;
+    }
+    long long* sums = s.dense + grp.id * (SLOTS_MAX / GROUPS);
+    uint32_t* keys = reinterpret_cast<uint32_t*>(sums + slots);  // !DENSE only
+    for (uint32_t i = tid; i < slots; i += grp.threads) {
+        sums[i] = 0;
+        if (!DENSE) keys[i] = EMPTYK;
+    }
     if (tid == 0) s.member[grp.id] = NONE32;
     grp.sync();
     // four chunks' gathers in flight, as in decide_warp
@@ -472,22 +487,22 @@ __device__ uint32_t decide_group(const Params& p, uint32_t v, uint32_t slots, Te
             if (j0 + k * grp.threads >= e) break;  // warp-uniform
             const unsigned peers = __match_any_sync(FULL, ok[k] ? (uint64_t)cu[k] : (0xFFFFFFFF00000000ull | lane));
             const long long x = peer_sum(peers, ok[k] ? to_fix((double)w[k], p.inv_scale) : 0ll);
-            if (ok[k] && __ffs(peers) - 1 == (int)lane)
-                atomicAdd((unsigned long long*)(dense + cu[k]), (unsigned long long)x);
+            if (!ok[k] || __ffs(peers) - 1 != (int)lane) continue;
+            if (DENSE) atomicAdd((unsigned long long*)(sums + cu[k]), (unsigned long long)x);
+            else hinsert(keys, sums, slots - 1, cu[k], x, p.status);
         }
     }
     grp.sync();
-    // lanes 0 and 1 of every warp take the own and the fresh community beside
-    // the first candidates of the other lanes
     double g = -INFINITY, base = 0.0, ge = 0.0;
     uint32_t c = NONE32, mine = 0;
-    const long long wof = dense[own];
+    const long long wof = DENSE ? sums[own] : hlookup(keys, sums, slots - 1, own);
     if (lane < 2) base = gain_as(p, q, side, lane == 0 ? OWN : FRESH, own, wof);
     ge = __shfl_sync(FULL, base, 1);
     base = __shfl_sync(FULL, base, 0);
-    for (uint32_t cu = tid; cu < slots; cu += grp.threads) {
-        const long long acc = dense[cu];
-        if (acc == 0 || cu == own) continue;
+    for (uint32_t i = tid; i < slots; i += grp.threads) {
+        const uint32_t cu = DENSE ? i : keys[i];
+        const long long acc = sums[i];
+        if ((DENSE ? acc == 0 : cu == EMPTYK) || cu == own) continue;
         ++mine;
         const double gg = key_of<REFINE>(p, q, v, cu, gain_as(p, q, side, JOIN, cu, acc), base);
         if (gg != -INFINITY && better(gg, cu, g, c)) {
@@ -573,14 +588,14 @@ __device__ __forceinline__ void for_picked(const Team& team, TeamSmem& s, const 
 }
 
 // Decisions of the nodes of one batch among list[0 .. m): those whose hash batch is b.
-template <bool REFINE>
+template <bool REFINE, bool MULTI, bool DENSE>
 __device__ void decide_batch(const Params& p, const Team& team, TeamSmem& s, const uint32_t* list, uint32_t m,
                              uint32_t sweep, int B, int b, uint32_t slots, Tally& tally) {
     const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     for_picked(
         team, s, list, m,
         [&](uint32_t v, uint4& it) {
-            if ((int)(hash3(p.seed, sweep, v) % (uint64_t)B) != b) return false;
+            if (batch_of<MULTI>(p.seed, sweep, v, B, p.inst, p.icfg) != b) return false;
             const uint32_t own = p.memb[v];
             if (REFINE && p.csize[own] != 1) return false;  // refine.rs:60-62
             const uint64_t rb = p.ptr[v];
@@ -589,10 +604,11 @@ __device__ void decide_batch(const Params& p, const Team& team, TeamSmem& s, con
             const uint32_t at = atomicAdd(&s.nbig, 1u);
             if (at < TEAM_BIG) s.big[at] = v;
             else atomicOr(p.status, DEV_OVERFLOW);
+            if (!DENSE) atomicMax(&s.bigmax, it.z);
             return false;
         },
         [&](const uint4& it) {
-            const uint32_t nc = decide_warp<REFINE>(p, it.x, it.y, it.z, it.w, s.table[wid], &s.wcnt[wid]);
+            const uint32_t nc = decide_warp<REFINE, MULTI>(p, it.x, it.y, it.z, it.w, s.table[wid], &s.wcnt[wid]);
             if (lane == 0) {
                 tally.deg += it.z;
                 tally.cand += nc;
@@ -600,30 +616,32 @@ __device__ void decide_batch(const Params& p, const Team& team, TeamSmem& s, con
             }
         });
     const uint32_t nbig = min(s.nbig, TEAM_BIG);
-    const uint32_t parts = slots <= SLOTS_MAX / GROUPS ? GROUPS : 1u;
+    const bool quarters = DENSE ? slots <= SLOTS_MAX / GROUPS : s.bigmax <= GROUP_DEGREE;
+    const uint32_t parts = quarters ? GROUPS : 1u;
     const Group grp{threadIdx.x / (TEAM_THREADS / parts), TEAM_THREADS / parts};
     for (uint32_t i = grp.id; i < nbig; i += parts) {
         const uint32_t v = s.big[i];
-        tally.cand += decide_group<REFINE>(p, v, slots, s, grp);
+        tally.cand += decide_group<REFINE, MULTI, DENSE>(p, v, slots, s, grp);
         if (grp.tid() == 0) {
             tally.deg += p.ptr[v + 1] - p.ptr[v];
             tally.nodes += 1;
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) s.nbig = 0;
+    if (threadIdx.x == 0) s.nbig = s.bigmax = 0;
 }
 
 // Commits the decisions of epoch p.cur among list[0 .. m).
-template <bool REFINE>
-__device__ void apply_batch(const Params& p, const Team& team, const uint32_t* list, uint32_t m, TeamCtl* ctl) {
+template <bool REFINE, bool MULTI>
+__device__ void apply_batch(const Params& p, const Team& team, const uint32_t* list, uint32_t m,
+                            unsigned long long* moves, long long* gain) {
     unsigned long long nmoves = 0;
     long long gsum = 0;
     for (uint32_t i0 = team.rank * TEAM_THREADS; i0 < m; i0 += team.size * TEAM_THREADS) {
         const uint32_t i = i0 + threadIdx.x;
         if (i >= m) continue;
         const uint32_t v = list ? list[i] : i;
-        if (p.epoch[v] != p.cur || cancelled<false>(p, v)) continue;
+        if (p.epoch[v] != p.cur || cancelled<MULTI>(p, v)) continue;
         const uint32_t t = p.tgt[v], old = p.from[v];
         const long long kf = to_fix(p.strength[v], p.inv_scale);
         p.memb[v] = t;
@@ -638,13 +656,18 @@ __device__ void apply_batch(const Params& p, const Team& team, const uint32_t* l
         atomicAdd(p.csize + t, 1u);
         if (!REFINE) {
             nmoves++;
-            gsum += p.dgain[v];
+            if (MULTI) {
+                if (p.dgain[v])
+                    atomicAdd((unsigned long long*)(p.gain_inst + p.inst[v]), (unsigned long long)p.dgain[v]);
+            } else {
+                gsum += p.dgain[v];
+            }
             p.moved[v] = p.cur;
         }
     }
     if (REFINE) return;
-    warp_add(&ctl->moves, nmoves);
-    warp_add((unsigned long long*)&ctl->gain, (unsigned long long)gsum);
+    warp_add(moves, nmoves);
+    if (!MULTI) warp_add((unsigned long long*)gain, (unsigned long long)gsum);
 }
 
 // Queues the neighbours of the nodes that moved in epoch p.cur and now sit in
@@ -825,7 +848,7 @@ __global__ void __launch_bounds__(TEAM_THREADS, 1) k_team(const __grid_constant_
     const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     Team team{blockIdx.x, gridDim.x};  // the grid is one cluster
     TeamCtl* ctl = a.ctl;
-    if (threadIdx.x == 0) s.nbig = s.nitem = s.next = 0;
+    if (threadIdx.x == 0) s.nbig = s.bigmax = s.nitem = s.next = 0;
     __syncthreads();
 
     TeamBuf cur = a.in;
@@ -950,10 +973,10 @@ __global__ void __launch_bounds__(TEAM_THREADS, 1) k_team(const __grid_constant_
             unsigned* ncount = &ctl->acount[(sweep + 1) & 1];
             for (int b = 0; b < LM_BATCHES; ++b) {
                 p.cur = ++epoch;
-                decide_batch<false>(p, team, s, list, m, sweep, LM_BATCHES, b, slots, tally);
+                decide_batch<false, false, true>(p, team, s, list, m, sweep, LM_BATCHES, b, slots, tally);
                 team.sync();
                 if (b == 0 && g0 == 0) *ncount = 0;  // last read a sweep ago; first written after the next barrier
-                apply_batch<false>(p, team, list, m, ctl);
+                apply_batch<false, false>(p, team, list, m, &ctl->moves, &ctl->gain);
                 team.sync();
                 // beside the next batch's decisions: it writes only the next sweep's list
                 activate_batch(p, team, s, list, m, a.stamp, sweep + 2, next, ncount);
@@ -993,9 +1016,9 @@ __global__ void __launch_bounds__(TEAM_THREADS, 1) k_team(const __grid_constant_
             team.sync();
             for (int b = 0; b < RF_BATCHES; ++b) {
                 p.cur = (uint32_t)(b + 1);
-                decide_batch<true>(p, team, s, nullptr, n, 0xFFFFFFFFu, RF_BATCHES, b, n, rt);
+                decide_batch<true, false, true>(p, team, s, nullptr, n, 0xFFFFFFFFu, RF_BATCHES, b, n, rt);
                 team.sync();
-                apply_batch<true>(p, team, nullptr, n, ctl);
+                apply_batch<true, false>(p, team, nullptr, n, nullptr, nullptr);
                 team.sync();
             }
             warp_add(a.refine_ctr + 0, rt.nodes);
@@ -1185,6 +1208,100 @@ __global__ void __launch_bounds__(TEAM_THREADS, 1) k_team(const __grid_constant_
     }
 }
 
+// ------------------------------------------------------------ the last sweeps of a larger level
+struct TailCtl {
+    unsigned done, which, sweep, epoch, swept, pad;
+    unsigned long long moves_before;
+};
+struct TailArgs {
+    Params p;
+    const uint32_t* first;  // the first sweep's list (null: all of [0, n))
+    uint32_t* list[2];      // later lists: sweep k of this launch reads list[k & 1]
+    unsigned* count[2];
+    uint32_t* stamp;
+    uint32_t n, sweep, epoch, limit;
+    unsigned long long moves_before, budget;
+    TailCtl* ctl;
+};
+
+// Local moving from sweep a.sweep on, whose list the host has counted, until
+// the level is done or a sweep has more than a.limit active nodes.
+template <bool MULTI>
+__global__ void __launch_bounds__(TEAM_THREADS, 1) k_move_tail(const __grid_constant__ TailArgs a) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    TeamSmem& s = *reinterpret_cast<TeamSmem*>(raw);
+    const Team team{blockIdx.x, gridDim.x};
+    const bool lead = team.rank == 0 && threadIdx.x == 0;
+    if (threadIdx.x == 0) s.nbig = s.bigmax = s.nitem = s.next = 0;
+    __syncthreads();
+    Params p = a.p;
+    Tally tally{0, 0, 0};
+    uint32_t sweep = a.sweep, epoch = a.epoch, swept = 0, which = 0;
+    unsigned long long moves_before = a.moves_before;
+    bool done = true;
+    for (; sweep < (uint32_t)MAX_SWEEPS; ++sweep) {
+        const uint32_t* list = swept || !a.first ? a.list[which] : a.first;
+        if (!swept && !a.first) list = nullptr;
+        const uint32_t m = swept || a.first ? *a.count[which] : a.n;
+        const unsigned long long moves = p.counters[0];
+        if (swept) {  // the host has checked the first sweep
+            if (moves == moves_before || moves >= a.budget || m == 0) break;
+            if (m > a.limit) {
+                done = false;
+                break;
+            }
+            moves_before = moves;
+        }
+        unsigned* ncount = a.count[which ^ 1];
+        uint32_t* next = a.list[which ^ 1];
+        for (int b = 0; b < LM_BATCHES; ++b) {
+            p.cur = ++epoch;
+            decide_batch<false, MULTI, false>(p, team, s, list, m, sweep, LM_BATCHES, b, 0, tally);
+            team.sync();
+            if (b == 0 && lead) *ncount = 0;
+            apply_batch<false, MULTI>(p, team, list, m, p.counters, p.gain_acc);
+            team.sync();
+            activate_batch(p, team, s, list, m, a.stamp, sweep + 2, next, ncount);
+        }
+        team.sync();
+        which ^= 1u;
+        ++swept;
+    }
+    warp_add(p.counters + 1, tally.deg);
+    warp_add(p.counters + 2, tally.cand);
+    warp_add(p.counters + 3, tally.nodes);
+    if (lead) {
+        a.ctl->done = done;
+        a.ctl->which = which;
+        a.ctl->sweep = sweep;
+        a.ctl->epoch = epoch;
+        a.ctl->swept = swept;
+        a.ctl->moves_before = moves_before;
+    }
+}
+
+// A launch of one cluster of `blocks` blocks with the team's shared memory.
+template <class K, class A>
+void launch_team(Ctx& c, K kernel, uint32_t blocks, const A& args) {
+    SC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TeamSmem)));
+    SC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(blocks);
+    lc.blockDim = dim3(TEAM_THREADS);
+    lc.dynamicSmemBytes = sizeof(TeamSmem);
+    lc.stream = c.stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    SC_CUDA(cudaLaunchKernelEx(&lc, kernel, args));
+    c.launches++;
+}
+
+uint32_t team_blocks(const Ctx& c) { return c.side[0] ? TEAM_CLUSTER : TEAM_CLUSTER / 2; }
+
 }  // namespace
 
 bool team_takes(Ctx& c, const DevGraph& g, const sc_leiden_config& cfg) {
@@ -1260,22 +1377,8 @@ void team_run(Ctx& c, const DevGraph& g, uint32_t* memb, uint64_t C, const sc_le
     a.max_levels = cfg.max_levels;
 
     const bool solo = n <= SOLO_NODES && E <= SOLO_ENTRIES;
-    const uint32_t blocks = solo ? 1u : c.side[0] ? TEAM_CLUSTER : TEAM_CLUSTER / 2;
-    SC_CUDA(cudaFuncSetAttribute(k_team, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TeamSmem)));
-    SC_CUDA(cudaFuncSetAttribute(k_team, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(blocks);
-    lc.blockDim = dim3(TEAM_THREADS);
-    lc.dynamicSmemBytes = sizeof(TeamSmem);
-    lc.stream = c.stream;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = blocks;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    lc.attrs = &at;
-    lc.numAttrs = 1;
-    SC_CUDA(cudaLaunchKernelEx(&lc, k_team, a));
-    c.launches++;
+    const uint32_t blocks = solo ? 1u : team_blocks(c);
+    launch_team(c, k_team, blocks, a);
 
     TeamCtl r;
     {
@@ -1307,6 +1410,43 @@ void team_run(Ctx& c, const DevGraph& g, uint32_t* memb, uint64_t C, const sc_le
     if (r.memb2) d2d(c, memb, a.memb2, r.n);
     const TeamBuf& b = a.buf[r.buf];
     out.graph.reset(graph_from_contraction(c, r.n, r.E, b.ptr, b.nbr, b.w, b.node_w));
+}
+
+uint32_t tail_limit(const Ctx& c, const DevGraph& g, const sc_leiden_config& cfg) {
+    if (cfg.has_max_community_weight || g.max_degree > BLOCK_DEGREE || g.E > 0xFFFFFFFFull) return 0;
+    return team_blocks(c) * TAIL_NODES_PER_BLOCK;
+}
+
+TailResult tail_run(Ctx& c, const void* params, uint32_t n, const uint32_t* first, uint32_t* const lists[2],
+                    uint32_t* const counts[2], uint32_t* stamp, uint32_t sweep, uint32_t epoch, uint64_t moves_before,
+                    uint64_t budget) {
+    DBuf<TailCtl> ctl(c, 1);
+    TailArgs a{};
+    a.p = *static_cast<const Params*>(params);
+    a.first = first;
+    a.list[0] = lists[0];
+    a.list[1] = lists[1];
+    a.count[0] = counts[0];
+    a.count[1] = counts[1];
+    a.stamp = stamp;
+    a.n = n;
+    a.sweep = sweep;
+    a.epoch = epoch;
+    a.limit = std::min<uint32_t>(TEAM_MAX_NODES, 2 * team_blocks(c) * TAIL_NODES_PER_BLOCK);
+    a.moves_before = moves_before;
+    a.budget = budget;
+    a.ctl = ctl.get();
+    if (a.p.inst) launch_team(c, k_move_tail<true>, team_blocks(c), a);
+    else launch_team(c, k_move_tail<false>, team_blocks(c), a);
+    const TailCtl r = to_host(c, ctl.get());
+    TailResult t;
+    t.done = r.done != 0;
+    t.swapped = r.which != 0;
+    t.sweep = r.sweep;
+    t.epoch = r.epoch;
+    t.swept = r.swept;
+    t.moves_before = r.moves_before;
+    return t;
 }
 
 }  // namespace sc

@@ -44,4 +44,21 @@ bool team_takes(Ctx& c, const DevGraph& g, const sc_leiden_config& cfg);
 void team_run(Ctx& c, const DevGraph& g, uint32_t* memb, uint64_t C, const sc_leiden_config& cfg, uint64_t pass_seed,
               uint64_t level, double improvement, TeamSpace& space, uint32_t* node_map, TeamResult& out);
 
+// The last sweeps of a larger level's local moving: once a sweep has at most
+// tail_limit active nodes (0: the team cannot take this level), the team runs on
+// until the level is done or a sweep outgrows it.
+uint32_t tail_limit(const Ctx& c, const DevGraph& g, const sc_leiden_config& cfg);
+struct TailResult {
+    bool done = false;
+    bool swapped = false;  // not done: the next sweep's list is lists[1], its count counts[1]
+    uint32_t sweep = 0;    // not done: the sweep to go on with
+    uint32_t epoch = 0, swept = 0;
+    uint64_t moves_before = 0;
+};
+// params: the level's Params (sc_move.cuh), its counters and gains running on.
+// first: the list of sweep `sweep` (lists[0], or null for all n nodes).
+TailResult tail_run(Ctx& c, const void* params, uint32_t n, const uint32_t* first, uint32_t* const lists[2],
+                    uint32_t* const counts[2], uint32_t* stamp, uint32_t sweep, uint32_t epoch, uint64_t moves_before,
+                    uint64_t budget);
+
 }  // namespace sc

@@ -87,3 +87,28 @@ def test_a_long_run_ends_in_the_team():
     g = sc_gpu.knn_gaussian(X, 12, sigma=sc_gpu.SIGMA_KTH, sym=sc_gpu.SYM_UNION, build_graph=True).graph
     for f in ("rb", "cpm", "louvain"):
         _check(g, seed=5, **CONFIGS[f])
+
+
+@pytest.mark.parametrize("cfg", ["rb", "cpm", "louvain"])
+@pytest.mark.parametrize("n,hub", [(9000, 0), (40_000, 1500), (40_000, 4096), (40_000, 4097), (40_000, 9000)])
+def test_last_sweeps_of_larger_levels(n, hub, cfg):
+    """The last sweeps run on the team: rows of a warp, a quarter of a block, a
+    block (a hub of 1,500 to 4,096 entries), and a hub past what it takes. The
+    same graph in a batch of two goes through the instances' form of the kernel."""
+    src, dst, w, _ = synth.planted_partition(n, 60, 8, 2, seed=n + hub)
+    if hub:
+        src = np.concatenate([src, np.zeros(hub, np.uint64)])
+        dst = np.concatenate([dst, 1 + np.arange(hub, dtype=np.uint64)])
+        w = np.concatenate([w, np.full(hub, 0.5)])
+    g = sc_gpu.CSRNetwork.from_edge_arrays(n, src, dst, w)
+    c = sc_gpu.LeidenConfig(seed=hub, **CONFIGS[cfg])
+    saved = sc_gpu.get_tuning()
+    want = sc_gpu.leiden(g, c)
+    two = sc_gpu.leiden_batch([g, g], [c, c], union=True)
+    for r in two:
+        assert np.array_equal(r.labels(), want.labels())
+    sc_gpu.set_tuning({**saved, "small_batch": 0, "lanes32_max_degree": 16})
+    try:
+        assert np.array_equal(sc_gpu.leiden(g, c).labels(), want.labels())
+    finally:
+        sc_gpu.set_tuning(saved)
