@@ -1406,67 +1406,50 @@ __global__ void k_km_accum(const float* __restrict__ X, uint64_t n, uint32_t d, 
         if (s_cnt[i]) atomicAdd(cnt + i, s_cnt[i]);
 }
 
-// Farthest-point seeding: d2min[i] = min(d2min[i], |x_i - c|^2) for the newest
-// centre c; the next centre is the sample point farthest from every centre
-// chosen so far (ties to the lower index), so separated groups of points each
-// get a centre before any group gets a second.
-__global__ void k_seed_update(const float* __restrict__ Xs, uint64_t n, uint32_t d, const float* __restrict__ c,
-                              float* d2min) {
+// Farthest-point seeding, step t >= 1: centre t - 1 is the sample point that key
+// t - 1 names (step 1: the first point); d2min[i] = min(d2min[i], |x_i - c|^2);
+// key t receives the point farthest from every centre chosen so far (ties to the
+// lower index), so separated groups of points each get a centre before any group
+// gets a second. A key is the distance's bits (non-negative floats order like
+// them) over the complement of the index, so one atomicMax per block finds it:
+// a second launch of one block for the search took 16 of a step's 23 us, 2.8 ms
+// for 121 centres; a step takes 7.3 us now. One more step (update == 0) only
+// writes the last centre.
+__global__ void __launch_bounds__(256) k_seed_step(const float* __restrict__ Xs, uint64_t n, uint32_t d, uint32_t t,
+                                                   int update, float* d2min, unsigned long long* keys,
+                                                   float* __restrict__ cent) {
+    __shared__ float s_c[64];
+    __shared__ unsigned long long s_key[8];
+    const uint32_t pick = t == 1 ? 0u : ~(uint32_t)keys[t - 1];
+    for (uint32_t j = threadIdx.x; j < d; j += blockDim.x) {
+        const float v = Xs[(uint64_t)pick * d + j];
+        s_c[j] = v;
+        if (blockIdx.x == 0) cent[(uint64_t)(t - 1) * d + j] = v;
+    }
+    if (!update) return;
+    __syncthreads();
+    unsigned long long key = 0;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         float acc = 0.0f;
         for (uint32_t j = 0; j < d; ++j) {
-            const float df = __fsub_rn(Xs[i * d + j], c[j]);
+            const float df = __fsub_rn(Xs[i * d + j], s_c[j]);
             acc = __fmaf_rn(df, df, acc);
         }
-        d2min[i] = fminf(d2min[i], acc);
-    }
-}
-
-// One block: the index of the largest d2min (lowest index on ties); copies
-// that point into centre slot `t`.
-__global__ void k_seed_pick(const float* __restrict__ Xs, uint64_t n, uint32_t d, const float* __restrict__ d2min,
-                            float* cent, uint32_t t) {
-    __shared__ float sv[32];
-    __shared__ uint32_t si[32];
-    float bv = -1.0f;
-    uint32_t bi = 0;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const float v = d2min[i];
-        if (v > bv) {
-            bv = v;
-            bi = i;
-        }
+        const float m = fminf(d2min[i], acc);
+        d2min[i] = m;
+        const unsigned long long k = ((unsigned long long)__float_as_uint(m) << 32) | (uint32_t)~(uint32_t)i;
+        key = k > key ? k : key;
     }
     for (int o = 16; o; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xFFFFFFFFu, bv, o);
-        const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
-        if (ov > bv || (ov == bv && oi < bi)) {
-            bv = ov;
-            bi = oi;
-        }
+        const unsigned long long k = __shfl_xor_sync(0xFFFFFFFFu, key, o);
+        key = k > key ? k : key;
     }
-    if ((threadIdx.x & 31) == 0) {
-        sv[threadIdx.x >> 5] = bv;
-        si[threadIdx.x >> 5] = bi;
-    }
+    if ((threadIdx.x & 31) == 0) s_key[threadIdx.x >> 5] = key;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        const uint32_t nw = blockDim.x >> 5;
-        bv = threadIdx.x < nw ? sv[threadIdx.x] : -1.0f;
-        bi = threadIdx.x < nw ? si[threadIdx.x] : 0xFFFFFFFFu;
-        for (int o = 16; o; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xFFFFFFFFu, bv, o);
-            const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, bi, o);
-            if (ov > bv || (ov == bv && oi < bi)) {
-                bv = ov;
-                bi = oi;
-            }
-        }
-        if (threadIdx.x == 0) si[0] = bi;
+    if (threadIdx.x == 0) {
+        for (uint32_t w = 1; w < (blockDim.x >> 5); ++w) key = s_key[w] > key ? s_key[w] : key;
+        atomicMax(keys + t, key);
     }
-    __syncthreads();
-    const uint32_t pick = si[0];
-    for (uint32_t j = threadIdx.x; j < d; j += blockDim.x) cent[(uint64_t)t * d + j] = Xs[(uint64_t)pick * d + j];
 }
 
 // New centroids; an empty cluster keeps its centroid.
@@ -1505,32 +1488,93 @@ __device__ __forceinline__ float unord32(unsigned k) {
 // so its queries need similar clusters.
 constexpr uint32_t FINE = 256;
 
+// |x - m|^2 of a point in registers (zeros past d) and a row of ceil4(d) floats
+// that starts on 16 bytes (zeros past d: those terms add +0), summed in
+// ascending order. Four values a load: read one at a time, the loads (the same
+// address for every thread of a warp) set the pace of the kernels below.
+__device__ __forceinline__ float sq_dist_padded(const float (&x)[64], const float* __restrict__ m, uint32_t d) {
+    const float4* m4 = reinterpret_cast<const float4*>(m);
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        if ((uint32_t)(4 * j) < d) {
+            const float4 v = m4[j];
+            float df = __fsub_rn(x[4 * j], v.x);
+            acc = __fmaf_rn(df, df, acc);
+            df = __fsub_rn(x[4 * j + 1], v.y);
+            acc = __fmaf_rn(df, df, acc);
+            df = __fsub_rn(x[4 * j + 2], v.z);
+            acc = __fmaf_rn(df, df, acc);
+            df = __fsub_rn(x[4 * j + 3], v.w);
+            acc = __fmaf_rn(df, df, acc);
+        }
+    return acc;
+}
+
+// rows[i] of src (rows of d floats) as row i of dst (rows of dp, zeros past d).
+__global__ void k_gather_rows_padded(const float* __restrict__ src, const uint32_t* __restrict__ rows, uint64_t n,
+                                     uint32_t d, uint32_t dp, float* dst) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n * dp; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t j = (uint32_t)(i % dp);
+        dst[i] = j < d ? src[(uint64_t)rows[i / dp] * d + j] : 0.0f;
+    }
+}
+
 __global__ void k_fine_assign(const float* __restrict__ Xs, uint64_t n, uint32_t d, const uint32_t* __restrict__ cl,
-                              const uint64_t* __restrict__ cstart, const uint32_t* __restrict__ fbase,
+                              const float* __restrict__ fcent, uint32_t dp, const uint32_t* __restrict__ fbase,
                               uint32_t* fine) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t b = cl[i];
-        const uint64_t s0 = cstart[b], s1 = cstart[b + 1];
-        float x[64];  // the point in registers (d <= 62)
+        const uint32_t f0 = fbase[b], f1 = fbase[b + 1];
+        float x[64];  // the point in registers (d <= 62), zeros past d
 #pragma unroll
         for (int j = 0; j < 64; ++j) x[j] = (uint32_t)j < d ? Xs[i * d + j] : 0.0f;
         float best = INFINITY;
-        uint32_t bf = 0, f = 0;
-        for (uint64_t p = s0; p < s1; p += FINE, ++f) {
-            const float* m = Xs + p * d;
-            float acc = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 64; ++j)
-                if ((uint32_t)j < d) {
-                    const float df = __fsub_rn(x[j], m[j]);
-                    acc = __fmaf_rn(df, df, acc);
-                }
+        uint32_t bf = f0;
+        for (uint32_t f = f0; f < f1; ++f) {
+            const float acc = sq_dist_padded(x, fcent + (uint64_t)f * dp, d);
             if (acc < best) {
                 best = acc;
                 bf = f;
             }
         }
-        fine[i] = fbase[b] + bf;
+        fine[i] = bf;
+    }
+}
+
+// start[q] = the first of the sorted points whose cluster is q or more, q = 0 .. K.
+__global__ void k_cluster_starts(const uint32_t* __restrict__ cl, uint64_t n, uint32_t K, uint64_t* start) {
+    for (uint32_t q = threadIdx.x; q <= K; q += blockDim.x) {
+        uint64_t lo = 0, hi = n;
+        while (lo < hi) {
+            const uint64_t mid = (lo + hi) >> 1;
+            if (cl[mid] < q) lo = mid + 1;
+            else hi = mid;
+        }
+        start[q] = lo;
+    }
+}
+
+// Unit vectors between the centres, a thread per (a, b): Ua[a][b] = Ub[b][a] =
+// (c_b - c_a) / |c_b - c_a| in rows of dp floats (zeros past d, and for a zero
+// direction, which bounds nothing).
+__global__ void k_directions(const float* __restrict__ cent, uint32_t K, uint32_t d, uint32_t dp, float* Ua,
+                             float* Ub) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < K * K; i += gridDim.x * blockDim.x) {
+        const uint32_t a = i / K, b = i % K;
+        double nrm = 0.0;
+        for (uint32_t j = 0; j < d; ++j) {
+            const double t = (double)cent[(uint64_t)b * d + j] - (double)cent[(uint64_t)a * d + j];
+            nrm += t * t;
+        }
+        nrm = sqrt(nrm);
+        for (uint32_t j = 0; j < dp; ++j) {
+            float u = 0.0f;
+            if (j < d && nrm != 0.0)
+                u = (float)(((double)cent[(uint64_t)b * d + j] - (double)cent[(uint64_t)a * d + j]) / nrm);
+            Ua[((uint64_t)a * K + b) * dp + j] = u;
+            Ub[((uint64_t)b * K + a) * dp + j] = u;
+        }
     }
 }
 
@@ -1549,14 +1593,15 @@ struct Chunk {
 __global__ void k_cluster_extent(const float* __restrict__ Xs, uint32_t d, const Chunk* __restrict__ chunks,
                                  const float* __restrict__ cent, const float* __restrict__ Ub, uint32_t K,
                                  unsigned* rad, unsigned* lo, unsigned* hi) {
-    extern __shared__ float sm[];
-    float* su = sm;                                   // K * d
-    unsigned* slo = (unsigned*)(su + (size_t)K * d);  // K
+    extern __shared__ __align__(16) float sm[];
+    const uint32_t dp = (d + 3) & ~3u;
+    float* su = sm;                                    // K * dp
+    unsigned* slo = (unsigned*)(su + (size_t)K * dp);  // K
     unsigned* shi = slo + K;                          // K
     __shared__ unsigned srad;
     const Chunk ch = chunks[blockIdx.x];
     const uint32_t b = ch.cluster;
-    for (uint32_t i = threadIdx.x; i < K * d; i += blockDim.x) su[i] = Ub[(uint64_t)b * K * d + i];
+    for (uint32_t i = threadIdx.x; i < K * dp; i += blockDim.x) su[i] = Ub[(uint64_t)b * K * dp + i];
     for (uint32_t i = threadIdx.x; i < K; i += blockDim.x) {
         slo[i] = 0xFFFFFFFFu;
         shi[i] = 0u;
@@ -1581,11 +1626,17 @@ __global__ void k_cluster_extent(const float* __restrict__ Xs, uint32_t d, const
         for (int o = 16; o; o >>= 1) kr = max(kr, __shfl_xor_sync(FULL, kr, o));
         if ((threadIdx.x & 31) == 0) atomicMax(&srad, kr);
         for (uint32_t a = 0; a < K; ++a) {
-            const float* u = su + (size_t)a * d;
-            float p = 0.0f;
+            const float4* u4 = reinterpret_cast<const float4*>(su + (size_t)a * dp);
+            float p = 0.0f;  // terms past d are +0: the same sum
 #pragma unroll
-            for (int j = 0; j < 64; ++j)
-                if ((uint32_t)j < d) p = __fmaf_rn(x[j], u[j], p);
+            for (int j = 0; j < 16; ++j)
+                if ((uint32_t)(4 * j) < d) {
+                    const float4 u = u4[j];
+                    p = __fmaf_rn(x[4 * j], u.x, p);
+                    p = __fmaf_rn(x[4 * j + 1], u.y, p);
+                    p = __fmaf_rn(x[4 * j + 2], u.z, p);
+                    p = __fmaf_rn(x[4 * j + 3], u.w, p);
+                }
             unsigned kl = ord32(p), kh = kl;
             for (int o = 16; o; o >>= 1) {
                 kl = min(kl, __shfl_xor_sync(FULL, kl, o));
@@ -1616,17 +1667,20 @@ __global__ void k_cluster_needs(const float* __restrict__ Xs, uint32_t d, const 
                                 const float* __restrict__ Ua, const unsigned* __restrict__ lo,
                                 const unsigned* __restrict__ hi, uint32_t K, float eps, uint32_t words,
                                 unsigned long long* mask) {
-    extern __shared__ float sm[];
-    float* su = sm;                       // K * d: directions from a to every b
-    float* sc = su + (size_t)K * d;       // K * d: centres
-    float* sr = sc + (size_t)K * d;       // K: radii
-    float* sl = sr + K;                   // K: lo[a][b]
-    float* sh = sl + K;                   // K: hi[a][b]
+    extern __shared__ __align__(16) float sm[];
+    // rows of dp floats, read as float4: one load feeds eight operations (one
+    // float at a time the loads set the pace: 3.9 ms at 1M x 50, 1.65 now)
+    const uint32_t dp = (d + 3) & ~3u;
+    float* su = sm;                        // K * dp: directions from a to every b
+    float* sc = su + (size_t)K * dp;       // K * dp: centres
+    float* sr = sc + (size_t)K * dp;       // K: radii
+    float* sl = sr + K;                    // K: lo[a][b]
+    float* sh = sl + K;                    // K: hi[a][b]
     const Chunk ch = chunks[blockIdx.x];
     const uint32_t a = ch.cluster;
-    for (uint32_t i = threadIdx.x; i < K * d; i += blockDim.x) {
-        su[i] = Ua[(uint64_t)a * K * d + i];
-        sc[i] = cent[i];
+    for (uint32_t i = threadIdx.x; i < K * dp; i += blockDim.x) {
+        su[i] = Ua[(uint64_t)a * K * dp + i];
+        sc[i] = i % dp < d ? cent[(uint64_t)(i / dp) * d + i % dp] : 0.0f;
     }
     for (uint32_t b = threadIdx.x; b < K; b += blockDim.x) {
         sr[b] = unord32(rad[b]);
@@ -1648,15 +1702,25 @@ __global__ void k_cluster_needs(const float* __restrict__ Xs, uint32_t d, const 
         for (uint32_t b = 0; b < K; ++b) {
             bool need = false;
             if (b != a) {
-                const float* m = sc + (size_t)b * d;
-                const float* u = su + (size_t)b * d;
-                float dc = 0.0f, p = 0.0f;
+                const float4* m4 = reinterpret_cast<const float4*>(sc + (size_t)b * dp);
+                const float4* u4 = reinterpret_cast<const float4*>(su + (size_t)b * dp);
+                float dc = 0.0f, p = 0.0f;  // terms past d are +0: the same sums
 #pragma unroll
-                for (int j = 0; j < 64; ++j)
-                    if ((uint32_t)j < d) {
-                        const float df = x[j] - m[j];
+                for (int j = 0; j < 16; ++j)
+                    if ((uint32_t)(4 * j) < d) {
+                        const float4 m = m4[j], u = u4[j];
+                        float df = x[4 * j] - m.x;
                         dc = __fmaf_rn(df, df, dc);
-                        p = __fmaf_rn(x[j], u[j], p);
+                        p = __fmaf_rn(x[4 * j], u.x, p);
+                        df = x[4 * j + 1] - m.y;
+                        dc = __fmaf_rn(df, df, dc);
+                        p = __fmaf_rn(x[4 * j + 1], u.y, p);
+                        df = x[4 * j + 2] - m.z;
+                        dc = __fmaf_rn(df, df, dc);
+                        p = __fmaf_rn(x[4 * j + 2], u.z, p);
+                        df = x[4 * j + 3] - m.w;
+                        dc = __fmaf_rn(df, df, dc);
+                        p = __fmaf_rn(x[4 * j + 3], u.w, p);
                     }
                 const float ball = sqrtf(dc) * (1.0f - 1e-5f) - sr[b] - eps;
                 const float slab = fmaxf(sl[b] - p, p - sh[b]) - 2.0f * eps;
@@ -1722,12 +1786,12 @@ __global__ void k_cell_count(const uint32_t* __restrict__ cell, uint64_t n, unsi
 }
 
 __global__ void k_cell_radius(const float* __restrict__ Xs, uint64_t n, uint32_t d, const uint32_t* __restrict__ cell,
-                              const float* __restrict__ fcent, unsigned* crad) {
+                              const float* __restrict__ fcent, uint32_t dp, unsigned* crad) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t f = cell[i];
         float r2 = 0.0f;
         for (uint32_t j = 0; j < d; ++j) {
-            const float df = Xs[i * d + j] - fcent[(uint64_t)f * d + j];
+            const float df = Xs[i * d + j] - fcent[(uint64_t)f * dp + j];
             r2 = __fmaf_rn(df, df, r2);
         }
         atomicMax(crad + f, ord32(sqrtf(r2)));
@@ -1743,6 +1807,10 @@ __global__ void k_cell_radius(const float* __restrict__ Xs, uint64_t n, uint32_t
 // excludes, for all queries at once, every cell with
 // |g - c_f| - r_g - r_f > max kth; only the remaining cells are tested per
 // query. Both tests carry the same rounding margins, the group test twice.
+// Bound by the instructions of the tests: 8.3 ms at 1M x 50 with every warp
+// testing every kept cell, a block per cluster in the first test and one float
+// a load; 4.4 with a warp per cluster there, warps that start at different
+// cells and skip the settled ones, and float4 rows.
 __global__ void k_group_cells(const float* __restrict__ Xs, uint64_t n, uint32_t d, const uint32_t* __restrict__ ord,
                               const float* __restrict__ kb, const unsigned long long* __restrict__ gmask,
                               const uint32_t* __restrict__ gown,
@@ -1754,6 +1822,7 @@ __global__ void k_group_cells(const float* __restrict__ Xs, uint64_t n, uint32_t
     const uint64_t r = g * (QT * TILE) + threadIdx.x;
     const bool ok = r < n;
     const uint64_t sq = ok ? ord[r] : ord[n - 1];
+    const uint32_t dp = (d + 3) & ~3u;
     float x[64];
 #pragma unroll
     for (int j = 0; j < 64; ++j) x[j] = (uint32_t)j < d ? Xs[sq * d + j] : 0.0f;
@@ -1792,15 +1861,23 @@ __global__ void k_group_cells(const float* __restrict__ Xs, uint64_t n, uint32_t
     __syncthreads();
     const float rg = unord32(s_r) * (1.0f + 1e-5f), kmax = unord32(s_k);
     const uint32_t a0 = gown[2 * g], a1 = gown[2 * g + 1];
-    // the group-ball test, a thread per cell
-    for (uint32_t b = 0; b < K; ++b) {
+    // the group-ball test: a warp per candidate cluster, a lane per cell (a
+    // cluster holds some tens of cells)
+    for (uint32_t b = wid; b < K; b += nw) {
         const bool cand = (b >= a0 && b <= a1) || ((gmask[g * words + b / 64] >> (b % 64)) & 1ull);
-        if (!cand) continue;  // uniform over the block
-        for (uint32_t f = fbase[b] + threadIdx.x; f < fbase[b + 1]; f += blockDim.x) {
-            const float* m = fcent + (uint64_t)f * d;
+        if (!cand) continue;  // uniform over the warp
+        for (uint32_t f = fbase[b] + lane; f < fbase[b + 1]; f += 32) {
+            const float4* m4 = reinterpret_cast<const float4*>(fcent + (uint64_t)f * dp);
             float dc = 0.0f;
-            for (uint32_t j = 0; j < d; ++j) {
-                const float df = s_c[j] - m[j];
+            for (uint32_t j = 0; j < dp; j += 4) {
+                const float4 v = m4[j / 4];
+                float df = s_c[j] - v.x;
+                dc = __fmaf_rn(df, df, dc);
+                df = s_c[j + 1] - v.y;
+                dc = __fmaf_rn(df, df, dc);
+                df = s_c[j + 2] - v.z;
+                dc = __fmaf_rn(df, df, dc);
+                df = s_c[j + 3] - v.w;
                 dc = __fmaf_rn(df, df, dc);
             }
             if (!(sqrtf(dc) * (1.0f - 1e-5f) - rg - unord32(crad[f]) - 2.0f * eps > kmax))
@@ -1810,29 +1887,40 @@ __global__ void k_group_cells(const float* __restrict__ Xs, uint64_t n, uint32_t
     __syncthreads();
     // the per-query test on the cells the group ball kept, for the queries
     // whose own cluster or needs hold the cell's cluster (the group scans the
-    // union of its queries' needs; each query tests only its own)
+    // union of its queries' needs; each query tests only its own). One query
+    // that needs a cell settles it for the group, so the warps start at
+    // different words and pass over the cells that another has already set.
     const uint32_t myown = qcl[sq];
     const unsigned long long* mym = qmask + sq * words;
-    uint32_t b = 0;  // the cluster of cell f (cells ascend, so does b)
-    for (uint32_t wd = 0; wd < cwords; ++wd) {
-        unsigned bits = s_maybe[wd];  // uniform over the block
-        while (bits) {
-            const uint32_t f = wd * 32 + (uint32_t)(__ffs(bits) - 1);
-            bits &= bits - 1;
-            while (fbase[b + 1] <= f) ++b;
-            const bool mine = ok && (b == myown || ((mym[b / 64] >> (b % 64)) & 1ull));
-            if (!__any_sync(0xFFFFFFFFu, mine)) continue;
-            const float* m = fcent + (uint64_t)f * d;
-            float dc = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 64; ++j)
-                if ((uint32_t)j < d) {
-                    const float df = x[j] - m[j];
-                    dc = __fmaf_rn(df, df, dc);
-                }
-            const bool need = mine && sqrtf(dc) * (1.0f - 1e-5f) - unord32(crad[f]) - eps <= kth;
-            // one shared OR per warp that needs the cell (most cells are needed by all or none)
-            if (__ballot_sync(0xFFFFFFFFu, need) && lane == 0) atomicOr(s_bits + f / 32, 1u << (f % 32));
+    const volatile unsigned* v_bits = s_bits;
+    const uint32_t rot = wid * cwords / nw;
+    for (uint32_t base = 0; base < cwords; base += 32) {
+        const uint32_t at = (rot + base + lane) % cwords;
+        const unsigned kept = base + lane < cwords ? s_maybe[at] : 0u;
+        unsigned left = __ballot_sync(0xFFFFFFFFu, kept != 0u);
+        while (left) {
+            const int l = __ffs(left) - 1;
+            left &= left - 1;
+            unsigned bits = __shfl_sync(0xFFFFFFFFu, kept, l);
+            const uint32_t wd = (rot + base + l) % cwords;
+            uint32_t b = 0;  // the cluster of the word's first cell (cells ascend, so does b)
+            for (uint32_t hi = K, f = wd * 32 + (uint32_t)(__ffs(bits) - 1); hi - b > 1;) {
+                const uint32_t mid = (b + hi) >> 1;
+                if (fbase[mid] <= f) b = mid;
+                else hi = mid;
+            }
+            while (bits) {
+                const uint32_t bit = (uint32_t)(__ffs(bits) - 1), f = wd * 32 + bit;
+                bits &= bits - 1;
+                while (fbase[b + 1] <= f) ++b;
+                const bool mine = ok && !((v_bits[wd] >> bit) & 1u) &&
+                                  (b == myown || ((mym[b / 64] >> (b % 64)) & 1ull));
+                if (!__any_sync(0xFFFFFFFFu, mine)) continue;
+                const float dc = sq_dist_padded(x, fcent + (uint64_t)f * dp, d);
+                const bool need = mine && sqrtf(dc) * (1.0f - 1e-5f) - unord32(crad[f]) - eps <= kth;
+                // one shared OR per warp that needs the cell
+                if (__ballot_sync(0xFFFFFFFFu, need) && lane == 0) atomicOr(s_bits + wd, 1u << bit);
+            }
         }
     }
     __syncthreads();
@@ -1881,7 +1969,7 @@ __global__ void k_order_tiles(const float* __restrict__ Xs, uint64_t n, uint32_t
         uint32_t t = 0xFFFFFFFFu;
         if (k < cnt) {
             t = t0 + k;
-            const float* m = fcent + (uint64_t)tile_cell[t] * d;
+            const float* m = fcent + (uint64_t)tile_cell[t] * ((d + 3) & ~3u);
             key = 0.0f;
             for (uint32_t j = 0; j < d; ++j) {
                 const float df = s_c[j] - m[j];
@@ -2106,15 +2194,14 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     {
         // farthest-point seeds: the first sample point, then the farthest from all chosen so far
         DBuf<float> d2min(c, ns);
+        DBuf<unsigned long long> keys(c, K + 1);
         SC_CUDA(cudaMemsetAsync(d2min.get(), 0x7F, ns * sizeof(float), c.stream));  // a huge finite value
-        d2d(c, cent.get(), Xsub.get(), d);
-        for (uint32_t t = 1; t < K; ++t) {
-            k_seed_update<<<grid_for(ns, 256), 256, 0, c.stream>>>(Xsub.get(), ns, d, cent.get() + (uint64_t)(t - 1) * d,
-                                                                   d2min.get());
-            k_seed_pick<<<1, 1024, 0, c.stream>>>(Xsub.get(), ns, d, d2min.get(), cent.get(), t);
-        }
+        zero(c, keys.get(), K + 1);
+        for (uint32_t t = 1; t <= K; ++t)
+            k_seed_step<<<t < K ? grid_for(ns, 256) : 1, 256, 0, c.stream>>>(Xsub.get(), ns, d, t, t < K, d2min.get(),
+                                                                             keys.get(), cent.get());
         SC_LAUNCH_CHECK();
-        c.launches += 2 * (K - 1);
+        c.launches += K;
     }
     DBuf<uint32_t> assign(c, n);
     DBuf<unsigned long long> sums(c, (uint64_t)K * d);
@@ -2152,36 +2239,37 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     k_gather_rows<<<grid_for(n * d, 256), 256, 0, c.stream>>>(dX, perm0.get(), n, d, Xs.get());
     SC_LAUNCH_CHECK();
     c.launches++;
-    std::vector<uint32_t> h_cl(n);
-    std::vector<float> h_cent((uint64_t)K * d);
-    d2h(c, h_cl.data(), cl_s.get(), n);
-    d2h(c, h_cent.data(), cent.get(), (uint64_t)K * d);
-    sync(c);
-    std::vector<uint64_t> start(K + 1, 0);
-    for (uint64_t i = 0; i < n; ++i) start[h_cl[i] + 1]++;
-    for (uint32_t q = 0; q < K; ++q) start[q + 1] += start[q];
+    DBuf<uint64_t> d_start(c, K + 1);
+    k_cluster_starts<<<1, 512, 0, c.stream>>>(cl_s.get(), n, K, d_start.get());
+    SC_LAUNCH_CHECK();
+    c.launches++;
+    std::vector<uint64_t> start(K + 1);
+    {
+        Mailbox mb(c);
+        const uint64_t* hs = mb.get(d_start.get(), K + 1);
+        mb.wait();
+        std::copy(hs, hs + K + 1, start.begin());
+    }
     // 3. fine cells inside every cluster, then the final order: (cluster, cell)
     std::vector<uint32_t> fbase(K + 1, 0);
     for (uint32_t q = 0; q < K; ++q) fbase[q + 1] = fbase[q] + (uint32_t)((start[q + 1] - start[q] + FINE - 1) / FINE);
-    DBuf<uint64_t> d_start(c, K + 1);
     DBuf<uint32_t> d_fbase(c, K + 1), fine(c, n), fine_s(c, n), perm(c, n);
-    h2d(c, d_start.get(), start.data(), K + 1);
     h2d(c, d_fbase.get(), fbase.data(), K + 1);
-    k_fine_assign<<<grid_for(n, 256), 256, 0, c.stream>>>(Xs.get(), n, d, cl_s.get(), d_start.get(), d_fbase.get(),
-                                                           fine.get());
-    SC_LAUNCH_CHECK();
-    c.launches++;
-    // each cell's centre: the sample point that defined it (read before Xs is re-sorted)
+    // each cell's centre: the sample point that defines it (read before Xs is re-sorted)
     const uint32_t F = fbase[K];
     std::vector<uint32_t> cell_rows(F);
     for (uint32_t q = 0; q < K; ++q)
         for (uint32_t j = 0; j < fbase[q + 1] - fbase[q]; ++j) cell_rows[fbase[q] + j] = (uint32_t)(start[q] + (uint64_t)j * FINE);
     DBuf<uint32_t> d_cell_rows(c, std::max<uint32_t>(F, 1));
-    DBuf<float> fcent(c, (uint64_t)std::max<uint32_t>(F, 1) * d);
+    const uint32_t dp = (d + 3) & ~3u;  // rows of the centre and direction tables, read as float4
+    DBuf<float> fcent(c, (uint64_t)std::max<uint32_t>(F, 1) * dp);
     h2d(c, d_cell_rows.get(), cell_rows.data(), F);
-    k_gather_rows<<<grid_for((uint64_t)F * d, 256), 256, 0, c.stream>>>(Xs.get(), d_cell_rows.get(), F, d, fcent.get());
+    k_gather_rows_padded<<<grid_for((uint64_t)F * dp, 256), 256, 0, c.stream>>>(Xs.get(), d_cell_rows.get(), F, d, dp,
+                                                                             fcent.get());
+    k_fine_assign<<<grid_for(n, 256), 256, 0, c.stream>>>(Xs.get(), n, d, cl_s.get(), fcent.get(), dp, d_fbase.get(),
+                                                           fine.get());
     SC_LAUNCH_CHECK();
-    c.launches++;
+    c.launches += 2;
     sort_pairs(c, fine.get(), fine_s.get(), perm0.get(), perm.get(), n, bits_for(std::max<uint32_t>(F, 2) - 1));
     fine.release();
     perm0.release();
@@ -2193,7 +2281,7 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     zero(c, ccnt.get(), F);
     zero(c, crad.get(), F);
     k_cell_count<<<grid_for(n, 256), 256, 0, c.stream>>>(fine_s.get(), n, ccnt.get());
-    k_cell_radius<<<grid_for(n, 256), 256, 0, c.stream>>>(Xs.get(), n, d, fine_s.get(), fcent.get(), crad.get());
+    k_cell_radius<<<grid_for(n, 256), 256, 0, c.stream>>>(Xs.get(), n, d, fine_s.get(), fcent.get(), dp, crad.get());
     SC_LAUNCH_CHECK();
     c.launches += 2;
     std::vector<unsigned> h_ccnt(F);
@@ -2204,25 +2292,10 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     for (uint32_t f = 0; f < F; ++f) cstart[f + 1] = cstart[f] + h_ccnt[f];
     tm.mark();  // 2: sorted by cluster and cell
     // 4. cluster extents: radius, and [lo, hi] along every direction between centres
-    std::vector<float> Ua((uint64_t)K * K * d, 0.0f), Ub((uint64_t)K * K * d, 0.0f);
-    for (uint32_t qa = 0; qa < K; ++qa)
-        for (uint32_t qb = 0; qb < K; ++qb) {
-            double nrm = 0.0;
-            for (uint32_t j = 0; j < d; ++j) {
-                const double t = (double)h_cent[qb * d + j] - (double)h_cent[qa * d + j];
-                nrm += t * t;
-            }
-            nrm = std::sqrt(nrm);
-            if (qa == qb || nrm == 0.0) continue;  // a zero direction bounds nothing
-            for (uint32_t j = 0; j < d; ++j) {
-                const float u = (float)(((double)h_cent[qb * d + j] - (double)h_cent[qa * d + j]) / nrm);
-                Ua[((uint64_t)qa * K + qb) * d + j] = u;
-                Ub[((uint64_t)qb * K + qa) * d + j] = u;
-            }
-        }
-    DBuf<float> d_Ua(c, (uint64_t)K * K * d), d_Ub(c, (uint64_t)K * K * d);
-    h2d(c, d_Ua.get(), Ua.data(), (uint64_t)K * K * d);
-    h2d(c, d_Ub.get(), Ub.data(), (uint64_t)K * K * d);
+    DBuf<float> d_Ua(c, (uint64_t)K * K * dp), d_Ub(c, (uint64_t)K * K * dp);
+    k_directions<<<grid_for((uint64_t)K * K, 128), 128, 0, c.stream>>>(cent.get(), K, d, dp, d_Ua.get(), d_Ub.get());
+    SC_LAUNCH_CHECK();
+    c.launches++;
     const uint64_t ngroups = (n + QT * TILE - 1) / (QT * TILE);
     const uint64_t ntiles = (n + TILE - 1) / TILE;
     // chunks: inside one cluster for the extents; inside one cluster and one query group for the bounds
@@ -2244,7 +2317,7 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     zero(c, rad.get(), K);
     zero(c, hi.get(), (uint64_t)K * K);
     SC_CUDA(cudaMemsetAsync(lo.get(), 0xFF, (uint64_t)K * K * 4, c.stream));
-    const size_t sm_ext = (size_t)K * d * 4 + (size_t)K * 8;
+    const size_t sm_ext = (size_t)K * dp * 4 + (size_t)K * 8;
     SC_CUDA(cudaFuncSetAttribute(k_cluster_extent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_ext));
     k_cluster_extent<<<(unsigned)ch_ext.size(), 256, sm_ext, c.stream>>>(Xs.get(), d, d_ch_ext.get(), cent.get(),
                                                                          d_Ub.get(), K, rad.get(), lo.get(), hi.get());
@@ -2254,10 +2327,13 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     TcOperands op;
     prep_operands(c, Xs.get(), n, d, 0, n, precision, scale_words.get(), op);
     tm.mark();  // 3: extents and operands
+    // the points of the clusters that query group g lies in
     auto own = [&](uint64_t g, std::vector<std::pair<uint64_t, uint64_t>>& pts) {
-        const uint32_t a0 = h_cl[g * QT * TILE], a1 = h_cl[std::min<uint64_t>(n, (g + 1) * QT * TILE) - 1];
+        auto cluster_of = [&](uint64_t i) {
+            return (uint64_t)(std::upper_bound(start.begin(), start.end(), i) - start.begin()) - 1;
+        };
+        const uint64_t a0 = cluster_of(g * QT * TILE), a1 = cluster_of(std::min<uint64_t>(n, (g + 1) * QT * TILE) - 1);
         pts.emplace_back(start[a0], start[a1 + 1]);
-        return std::make_pair(a0, a1);
     };
     DBuf<uint32_t> cidx(c, n * RTOTAL);
     // the candidates' exact re-rank, queries in the order `ord` (nullable: the sorted order)
@@ -2336,7 +2412,7 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     const float R = std::sqrt(std::max(maxnorm, 0.0f)) + 1.0f;
     const float eps = 8.0f * (float)d * std::ldexp(1.0f, -24) * 2.0f * R;
     tm.mark();  // 5: bounds begin (after pass 1)
-    const size_t sm_need = (size_t)K * d * 8 + (size_t)K * 12;
+    const size_t sm_need = (size_t)K * dp * 8 + (size_t)K * 12;
     SC_CUDA(cudaFuncSetAttribute(k_cluster_needs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_need));
     k_cluster_needs<<<(unsigned)ch_need.size(), QT * TILE, sm_need, c.stream>>>(
         Xs.get(), d, d_ch_need.get(), kb.get(), cent.get(), rad.get(), d_Ua.get(), lo.get(), hi.get(), K, eps, words,
