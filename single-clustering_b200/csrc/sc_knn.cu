@@ -107,6 +107,17 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// One lane of a converged warp, the same one each time.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(p));
+    return p != 0;
+}
+
 // Shared-memory matrix descriptor, K-major, swizzled rows of KA * 2 bytes:
 // start >> 4 at [0,14), stride between 8-row groups >> 4 at [32,46),
 // version 1 at [46,48), layout at [61,64) (4 = 64B swizzle, 2 = 128B swizzle).
@@ -185,54 +196,127 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&v)[64]) {
     for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// A (query, half)'s kept candidates: RCAND slots of shared memory, filled in
-// order; a full row replaces its worst. The search for the worst is kept out of
-// line: inlined into the unrolled filter it overflows the instruction cache.
-struct Kept {
-    float thr;     // scores at or above it are not candidates
-    uint32_t off;  // the slot the next candidate goes to
-};
-constexpr uint32_t SLOT_STRIDE = QT * HALVES * TILE;  // (tile, half, row) owners: one column per owner
+// 8 accumulator columns of this lane's row.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
 
-// The worst of a full row (highest score, lowest slot on ties).
-__device__ __noinline__ Kept row_worst(const float* cs, uint32_t owner) {
-    float worst = -INFINITY;
-    uint32_t at = owner;
-#pragma unroll 8
-    for (int s = 0; s < RCAND; ++s) {
-        const float x = cs[s * SLOT_STRIDE + owner];
-        if (x > worst) {
-            worst = x;
-            at = s * SLOT_STRIDE + owner;
+// A (query, half)'s candidates: CAND_SLOTS slots of shared memory, filled in
+// order; when a row of the warp has no room for the next, all rows are cut back
+// to their RCAND best together. Every lane of the warp calls it. A row of `cnt` keeps
+// min(cnt, RCAND), in the first slots. Returns the score
+// from which on nothing is a candidate any more: the worst kept of a full row,
+// else cap. Near tiles bring a row's candidates in a burst, 95 a query at
+// 1M x 50; a search for the worst of a full row at each of them (a call for one
+// or two rows at a time, while all warps of the block wait) held up every warp by
+// 290 cycles a tile, this by 60.
+constexpr uint32_t SLOT_STRIDE = QT * HALVES * TILE;  // (tile, half, row) owners: one column per owner
+constexpr int CAND_SLOTS = RCAND + 4;
+__device__ __noinline__ float cand_cut(float* cs, uint32_t* ci, uint32_t owner, uint32_t cnt, float cap) {
+    constexpr int TOP = CAND_SLOTS - RCAND + 1;
+    float top[TOP];  // the row's largest, descending
+#pragma unroll
+    for (int i = 0; i < TOP; ++i) top[i] = -INFINITY;
+#pragma unroll 4
+    for (uint32_t s = 0; s < (uint32_t)CAND_SLOTS; ++s) {
+        float v = s < cnt ? cs[s * SLOT_STRIDE + owner] : -INFINITY;
+#pragma unroll
+        for (int i = 0; i < TOP; ++i) {
+            const float hi = fmaxf(top[i], v);
+            v = fminf(top[i], v);
+            top[i] = hi;
         }
     }
-    return Kept{worst, at};
+    if (cnt < (uint32_t)RCAND) return cap;
+    const uint32_t drop = cnt - RCAND;  // of the largest: the worst kept is top[drop]
+    float worst = top[0];
+    uint32_t ties = 0;  // dropped ones that equal the worst kept
+#pragma unroll
+    for (int i = 1; i < TOP; ++i)
+        if ((uint32_t)i <= drop) {
+            ties = top[i] == worst ? ties + 1 : 0;
+            worst = top[i];
+        }
+    if (drop) {
+        uint32_t w = owner;
+#pragma unroll 4
+        for (uint32_t s = 0; s < cnt; ++s) {
+            const float v = cs[s * SLOT_STRIDE + owner];
+            const uint32_t id = ci[s * SLOT_STRIDE + owner];
+            bool keep = v <= worst;
+            if (v == worst && ties) {  // as many of the equal ones as do not fit
+                keep = false;
+                --ties;
+            }
+            if (keep) {
+                cs[w] = v;
+                ci[w] = id;
+                w += SLOT_STRIDE;
+            }
+        }
+    }
+    return fminf(worst, cap);
 }
 
 // A bounding scan keeps scores alone: BOUND_SLOTS per (query, half), cut back to
 // the BOUND_KEEP smallest (ascending, in the first slots) when a row of the warp
 // is nearly full. Returns the largest kept of a row that holds BOUND_KEEP or
 // more, +inf for one that holds fewer. Every lane of the warp calls it.
+//
+// Its time counts for every warp of the block: with one tile of slack, all wait
+// for the one that cuts. Each value moved up through the list in turn took 15,800
+// cycles a cut (15 cuts a warp in 1750 tiles of 1M x 50 points), 16 values at a
+// time through a sorting network 10,400; the scan went from 7.3 to 5.8 ms.
 constexpr int BOUND_KEEP = 16;
 constexpr int BOUND_SLOTS = 2 * RCAND;  // the candidates' scores and ids in one
+
+__device__ __forceinline__ void order2(float& a, float& b) {
+    const float lo = fminf(a, b);
+    b = fmaxf(a, b);
+    a = lo;
+}
+
 __device__ __noinline__ float bound_cut(float* cs, uint32_t owner, uint32_t cnt) {
-    float best[BOUND_KEEP];
+    static_assert(BOUND_KEEP == 16 && BOUND_SLOTS % 16 == 0, "blocks of 16 slots");
+    float best[16];
 #pragma unroll
-    for (int i = 0; i < BOUND_KEEP; ++i) best[i] = INFINITY;
+    for (int i = 0; i < 16; ++i) best[i] = INFINITY;
 #pragma unroll 1
-    for (uint32_t s = 0; s < (uint32_t)BOUND_SLOTS; ++s) {
-        float v = s < cnt ? cs[s * SLOT_STRIDE + owner] : INFINITY;
-        if (!__any_sync(0xFFFFFFFFu, v < best[BOUND_KEEP - 1])) continue;
+    for (uint32_t s = 0; s < (uint32_t)BOUND_SLOTS; s += 16) {
+        if (!__any_sync(0xFFFFFFFFu, s < cnt)) break;
+        float v[16];
 #pragma unroll
-        for (int i = 0; i < BOUND_KEEP; ++i) {  // v takes its place, the rest move up by one
-            const float lo = fminf(best[i], v);
-            v = fmaxf(best[i], v);
-            best[i] = lo;
-        }
+        for (uint32_t i = 0; i < 16; ++i) v[i] = s + i < cnt ? cs[(s + i) * SLOT_STRIDE + owner] : INFINITY;
+        // Batcher's odd-even merge sort, ascending
+#pragma unroll
+        for (int p = 1; p < 16; p <<= 1)
+#pragma unroll
+            for (int k = p; k >= 1; k >>= 1)
+#pragma unroll
+                for (int j = k % p; j + k < 16; j += 2 * k)
+#pragma unroll
+                    for (int i = 0; i < k; ++i)
+                        if (i + j + k < 16 && (i + j) / (2 * p) == (i + j + k) / (2 * p)) order2(v[i + j], v[i + j + k]);
+        // the 16 smallest of both lists, a bitonic sequence, then in order
+#pragma unroll
+        for (int i = 0; i < 16; ++i) best[i] = fminf(best[i], v[15 - i]);
+#pragma unroll
+        for (int k = 8; k >= 1; k >>= 1)
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if ((i & k) == 0) order2(best[i], best[i + k]);
     }
 #pragma unroll
-    for (int i = 0; i < BOUND_KEEP; ++i) cs[i * SLOT_STRIDE + owner] = best[i];
-    return best[BOUND_KEEP - 1];
+    for (int i = 0; i < 16; ++i) cs[i * SLOT_STRIDE + owner] = best[i];
+    return best[15];
 }
 
 // ------------------------------------------------------------ prep
@@ -432,9 +516,9 @@ struct KnnSmem {
     static constexpr uint32_t A_OFF = 0;
     static constexpr uint32_t B_OFF = A_OFF + QT * TILE_BYTES;
     static constexpr uint32_t C_OFF = B_OFF + STAGES * TILE_BYTES;               // candidate scores
-    static constexpr uint32_t I_OFF = C_OFF + RCAND * SLOTS * 4;                 // candidate ids (or more scores)
-    static constexpr uint32_t BAR_OFF = I_OFF + RCAND * SLOTS * 4;
-    static constexpr uint32_t NBAR = 2 * STAGES + 4 + 2;
+    static constexpr uint32_t I_OFF = C_OFF + CAND_SLOTS * SLOTS * 4;            // candidate ids (or more scores)
+    static constexpr uint32_t BAR_OFF = I_OFF + CAND_SLOTS * SLOTS * 4;
+    static constexpr uint32_t NBAR = 2 * STAGES + 2 * 2 * QT + 2;
     static constexpr uint32_t MISC_OFF = BAR_OFF + NBAR * 8;
     static constexpr uint32_t BYTES = MISC_OFF + 64 + 1024;  // + alignment slack
     static_assert(BYTES <= 227 * 1024, "shared memory of the kNN kernel exceeds 227 KB");
@@ -443,26 +527,42 @@ struct KnnSmem {
 
 // The point tiles a query group scans, in order: every tile, or (a pruned
 // search) the group's ranges of (first tile, tile count), which never overlap.
+// The next range is in registers before the current one ends: the loads of
+// a range list of single tiles stood in every tile's way.
 struct TileWalk {
     const uint2* r;
     uint32_t nr, ri, off, all;
+    uint2 cur, nxt;
+    __device__ uint2 at(uint32_t i) const { return r && i < nr ? r[i] : make_uint2(0u, 0u); }
     __device__ TileWalk(const uint32_t* rptr, const uint2* rngs, uint32_t g, uint32_t ntiles)
-        : r(rptr ? rngs + rptr[g] : nullptr), nr(rptr ? rptr[g + 1] - rptr[g] : 0), ri(0), off(0), all(ntiles) {}
+        : r(rptr ? rngs + rptr[g] : nullptr), nr(rptr ? rptr[g + 1] - rptr[g] : 0), ri(0), off(0), all(ntiles) {
+        cur = at(0);
+        nxt = at(1);
+    }
     __device__ uint32_t count() const {
         if (!r) return all;
         uint32_t c = 0;
         for (uint32_t i = 0; i < nr; ++i) c += r[i].y;
         return c;
     }
-    __device__ uint32_t next() {
+    __device__ uint32_t next() {  // called count() times at most
         if (!r) return off++;
-        while (off >= r[ri].y) {
+        while (off >= cur.y) {
+            cur = nxt;
             ++ri;
+            nxt = at(ri + 1);
             off = 0;
         }
-        return r[ri].x + off++;
+        return cur.x + off++;
     }
 };
+
+// min of three in one instruction; a NaN gives way to a number, like fminf.
+__device__ __forceinline__ float fmin3(float a, float b, float c) {
+    float m;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+    return m;
+}
 
 // F8: the operands are e4m3 bytes with the row size of BF16 KA columns.
 // rptr / rngs (nullable): the tile ranges of each query group (pruned search).
@@ -479,15 +579,15 @@ struct TileWalk {
 // (two of a query's nearest seldom share 8 columns); no ids, no list to keep in
 // order. Otherwise cand_idx[q] receives the candidates' ids.
 //
-// The epilogue sets the pace (K = 32 or 64 leaves the tensor pipe a quarter to
-// a half busy at best). Per tile a warp reads its 64 columns at once, frees the
-// accumulator, and takes minima of 8 columns; only an 8-column group in which
-// some row's minimum passes that row's threshold is looked at again, all rows
-// of the warp together, a candidate costing two predicated stores. A row is
-// searched for its worst only when it is full; one that starts from a bounding
-// scan's bound (some 20 candidates) hardly ever is. Taking the rows one by one,
-// with a search of the row's slots for every candidate, the two scans of
-// 1M x 50 points took 31.1 and 56.4 ms; they take 8.5 and 16.4 ms.
+// The epilogue sets the pace (K = 64 leaves the tensor pipe 31 to 42% busy), and
+// of it the warp that is slowest, since all others wait for it within a tile. Per
+// tile a warp reads its 64 columns at once and takes minima of 8 columns (three
+// values an instruction); only an 8-column group in which some row's minimum
+// passes that row's threshold is looked at again, all rows of the warp together, a
+// candidate costing two predicated stores. Rows are cut back when one is full
+// (cand_cut, bound_cut). Taking the rows one by one, with a search of the row's
+// slots for every candidate, the two scans of 1M x 50 points took 31.1 and 56.4
+// ms, a search only for a full row 8.5 and 16.4; 5.8 and 11.7 ms now.
 template <int KA, bool F8, bool BOUND = false>
 __global__ void __launch_bounds__(KNN_THREADS, 1)
     k_knn_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, uint32_t n,
@@ -504,14 +604,16 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
     uint64_t* bars = (uint64_t*)(smem + L::BAR_OFF);
     uint64_t* full = bars;                 // [L::STAGES] B tile landed
     uint64_t* empty = bars + L::STAGES;       // [L::STAGES] B tile consumed by the MMAs
-    uint64_t* accfull = bars + 2 * L::STAGES;       // [2] accumulator ready
-    uint64_t* accempty = bars + 2 * L::STAGES + 2;  // [2] accumulator drained
-    uint64_t* afull = bars + 2 * L::STAGES + 4;     // query tiles landed
-    uint64_t* aempty = bars + 2 * L::STAGES + 5;    // query tiles no longer read
+    // an accumulator per (buffer, query tile), handed over on its own: the warps
+    // of one query tile work while the other's products are under way
+    uint64_t* accfull = bars + 2 * L::STAGES;  // [2][QT] accumulator ready
+    uint64_t* accempty = accfull + 2 * QT;     // [2][QT] accumulator drained
+    uint64_t* afull = accempty + 2 * QT;       // query tiles landed
+    uint64_t* aempty = afull + 1;              // query tiles no longer read
     uint32_t* misc = (uint32_t*)(smem + L::MISC_OFF);
     volatile uint32_t* abort_flag = misc + 1;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t ntiles = (n + TILE - 1) / TILE;          // point tiles (B)
     const uint32_t ngroups = (nq + QT * TILE - 1) / (QT * TILE);  // query tile groups (A)
     // the i-th group of this CTA, ngroups when there is none
@@ -525,9 +627,9 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
             mbar_init(full + s, 1);
             mbar_init(empty + s, 1);
         }
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < 2 * QT; ++b) {
             mbar_init(accfull + b, 1);
-            mbar_init(accempty + b, NUM_EPI_WARPS);
+            mbar_init(accempty + b, NUM_EPI_WARPS / QT);
         }
         mbar_init(afull, 1);
         mbar_init(aempty, 1);
@@ -548,7 +650,8 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
     if (warp == 0) {
         // ---------------- TMA producer
         if (lane == 0) {
-            uint64_t it = 0;  // global B tile counter (all groups)
+            uint64_t it = 0;                    // B tiles issued, all groups
+            uint32_t stage = 0, s_parity = 0;  // the stage in turn
             uint32_t gi = 0;
             bool a_in_flight = false;
             for (uint32_t g; (g = group_at(gi)) < ngroups && !*abort_flag; ++gi) {
@@ -568,15 +671,18 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
                 const uint32_t cnt = walk.count();
                 for (uint32_t t = 0; t < cnt; ++t, ++it) {
                     const uint32_t tile = walk.next();
-                    const uint32_t s = (uint32_t)(it % L::STAGES);
-                    const uint64_t use = it / L::STAGES;
-                    if (use > 0 && !mbar_wait(empty + s, (uint32_t)((use - 1) & 1), lim)) {
+                    // a stage's first use passes at once: its barrier is in phase 0
+                    if (!mbar_wait(empty + stage, s_parity ^ 1u, lim)) {
                         *abort_flag = 1;
                         break;
                     }
                     if (*abort_flag) break;
-                    mbar_expect_tx(full + s, L::TILE_BYTES);
-                    tma_load_2d(sB + s * L::TILE_BYTES, &tmB, full + s, 0, (int)(tile * TILE));
+                    mbar_expect_tx(full + stage, L::TILE_BYTES);
+                    tma_load_2d(sB + stage * L::TILE_BYTES, &tmB, full + stage, 0, (int)(tile * TILE));
+                    if (++stage == (uint32_t)L::STAGES) {
+                        stage = 0;
+                        s_parity ^= 1u;
+                    }
                 }
             }
             // drain: the copies issued last (one per stage, and the query tiles)
@@ -588,60 +694,67 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc =
-                F8 ? idesc_e4m3_128x128() : idesc_16bit_128x128(f16_exp(scale) != INT32_MIN);
-            uint64_t it = 0;
-            uint32_t gi = 0;
-            for (uint32_t g; (g = group_at(gi)) < ngroups && !*abort_flag; ++gi) {
-                if (!mbar_wait(afull, gi & 1, lim)) {
-                    *abort_flag = 1;
-                    break;
-                }
-                fence_after();
-                const uint32_t cnt = TileWalk(rptr, rngs, g, ntiles).count();
-                for (uint32_t t = 0; t < cnt; ++t, ++it) {
-                    const uint32_t s = (uint32_t)(it % L::STAGES);
-                    const uint32_t b = (uint32_t)(it & 1);
-                    const uint64_t use_b = it >> 1;
-                    if (!mbar_wait(full + s, (uint32_t)((it / L::STAGES) & 1), lim)) {
-                        *abort_flag = 1;
-                        break;
-                    }
-                    if (use_b > 0 && !mbar_wait(accempty + b, (uint32_t)((use_b - 1) & 1), lim)) {
-                        *abort_flag = 1;
-                        break;
-                    }
-                    fence_after();
-                    const uint32_t bbase = smem_u32(sB + s * L::TILE_BYTES);
+        // ---------------- MMA issuer. One warp issues every product, so its
+        // instructions are on each tile's path: the whole warp walks the tiles
+        // (addresses and descriptors are then uniform), one lane issues, and
+        // stages and parities are counted, not divided. With a descriptor built
+        // for every product and 64-bit remainders the issue alone took 1040
+        // cycles of a tile's 2200 (300 to 500 now), the products 512.
+        const uint32_t idesc = F8 ? idesc_e4m3_128x128() : idesc_16bit_128x128(f16_exp(scale) != INT32_MIN);
+        const uint64_t adesc = smem_desc<KA>(smem_u32(sA)), bdesc = smem_desc<KA>(smem_u32(sB));
+        constexpr uint32_t TILE_STEP = L::TILE_BYTES >> 4;  // of a descriptor's start address
+        const bool issuer = elect_one();
+        uint64_t* last = nullptr;  // the newest accumulator commit and its parity
+        uint32_t last_parity = 0;
+        uint32_t s = 0, s_parity = 0, b = 0, b_parity = 0;  // the B stage and accumulator buffer in turn
+        uint32_t gi = 0;
+        bool ok = true;
+        for (uint32_t g; ok && (g = group_at(gi)) < ngroups && !__any_sync(0xFFFFFFFFu, *abort_flag != 0); ++gi) {
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(afull, gi & 1, lim));
+            if (!ok) break;
+            fence_after();
+            const uint32_t cnt = __shfl_sync(0xFFFFFFFFu, TileWalk(rptr, rngs, g, ntiles).count(), 0);
+            for (uint32_t t = 0; t < cnt; ++t) {
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait(full + s, s_parity, lim));
+                const uint64_t bd = bdesc + s * TILE_STEP;
 #pragma unroll
-                    for (int q = 0; q < QT; ++q) {
-                        const uint32_t abase = smem_u32(sA + q * L::TILE_BYTES);
-                        const uint32_t d = tmem + b * (QT * TILE) + q * TILE;
+                for (int q = 0; q < QT; ++q) {
+                    const uint32_t acc = b * QT + q;
+                    // a buffer's first use passes at once: its barrier is in phase 0
+                    if (ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(accempty + acc, b_parity ^ 1u, lim));
+                    if (!ok) break;
+                    fence_after();
+                    const uint64_t ad = adesc + q * TILE_STEP;
+                    if (issuer) {
 #pragma unroll
                         for (int kk = 0; kk < KA / 16; ++kk) {  // 32 bytes of K per MMA
                             if constexpr (F8)
-                                mma_e4m3(d, smem_desc<KA>(abase + kk * 32), smem_desc<KA>(bbase + kk * 32), idesc,
-                                         kk > 0 ? 1u : 0u);
+                                mma_e4m3(tmem + acc * TILE, ad + kk * 2, bd + kk * 2, idesc, kk > 0 ? 1u : 0u);
                             else
-                                mma_16bit(d, smem_desc<KA>(abase + kk * 32), smem_desc<KA>(bbase + kk * 32), idesc,
-                                         kk > 0 ? 1u : 0u);
+                                mma_16bit(tmem + acc * TILE, ad + kk * 2, bd + kk * 2, idesc, kk > 0 ? 1u : 0u);
                         }
+                        mma_commit(accfull + acc);
                     }
-                    mma_commit(empty + s);
-                    mma_commit(accfull + b);
+                    last = accfull + acc;
+                    last_parity = b_parity;
                 }
-                mma_commit(aempty);
+                if (!ok) break;
+                if (issuer) mma_commit(empty + s);
+                if (++s == (uint32_t)L::STAGES) {
+                    s = 0;
+                    s_parity ^= 1u;
+                }
+                b ^= 1u;
+                b_parity ^= b ^ 1u;  // both buffers used
             }
-            // drain: MMAs complete in issue order, so once the last tile's
-            // accumulator commit has arrived none is left writing TMEM or
-            // arriving on this CTA's barriers (waits with the default limit)
-            if (*abort_flag && it > 0) {
-                const uint64_t x = it - 1;
-                mbar_wait(accfull + (uint32_t)(x & 1), (uint32_t)((x >> 1) & 1));
-            }
+            if (ok && issuer) mma_commit(aempty);
         }
+        if (!ok) *abort_flag = 1;
+        // drain: MMAs complete in issue order, so once the last tile's
+        // accumulator commit has arrived none is left writing TMEM or
+        // arriving on this CTA's barriers (waits with the default limit)
+        if (__any_sync(0xFFFFFFFFu, *abort_flag != 0) && last) mbar_wait(last, last_parity);
+        __syncwarp();
     } else {
         // ---------------- epilogue: 16 warps; warp % 4 selects the TMEM lane quarter
         // (hardware rule), (warp - 2) / 4 the (query tile, column half) it reads
@@ -653,7 +766,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
         const int row = lq * 32 + lane;         // row within the query tile
         const uint32_t owner = combo * TILE + row;  // candidate-buffer column
         constexpr uint32_t S = SLOT_STRIDE;
-        uint64_t it = 0;
+        uint32_t b = 0, b_parity = 0;  // the accumulator buffer in turn
         uint32_t gi = 0;
         for (uint32_t g; (g = group_at(gi)) < ngroups && !*abort_flag; ++gi) {
             const uint64_t qrow = (uint64_t)g * QT * TILE + q * TILE + row;
@@ -663,19 +776,25 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
             uint32_t off = owner;  // where the next one goes
             TileWalk walk(rptr, rngs, g, ntiles);
             const uint32_t tcnt = walk.count();
-            for (uint32_t t = 0; t < tcnt; ++t, ++it) {
+            for (uint32_t t = 0; t < tcnt; ++t) {
                 const uint32_t tile = walk.next();
-                const uint32_t b = (uint32_t)(it & 1);
-                if (!__all_sync(0xFFFFFFFFu, mbar_wait(accfull + b, (uint32_t)((it >> 1) & 1), lim))) {
+                const uint32_t acc = b * QT + q;
+                if (!__all_sync(0xFFFFFFFFu, mbar_wait(accfull + acc, b_parity, lim))) {
                     *abort_flag = 1;
                     break;
                 }
                 fence_after();
+                const uint32_t taddr = tmem + ((uint32_t)(lq * 32) << 16) + acc * TILE + h * (TILE / HALVES);
                 float r[64];
-                tmem_ld64(tmem + ((uint32_t)(lq * 32) << 16) + b * (QT * TILE) + q * TILE + h * (TILE / HALVES), r);
-                fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(accempty + b);  // the scores are in registers
+                tmem_ld64(taddr, r);
+                auto release = [&] {  // the accumulator is no longer read
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(accempty + acc);
+                };
+                if constexpr (BOUND) release();
+                b ^= 1u;
+                b_parity ^= b ^ 1u;
                 const uint32_t base_idx = tile * TILE + h * (TILE / HALVES);
                 if (base_idx + 64 > n) {  // the last tile's rows past the points hold zeros, not scores
 #pragma unroll
@@ -686,12 +805,13 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
 #pragma unroll
                 for (int j8 = 0; j8 < 8; ++j8) {
                     const float* x = r + j8 * 8;
-                    m[j8] = fminf(fminf(fminf(x[0], x[1]), fminf(x[2], x[3])),
-                                  fminf(fminf(x[4], x[5]), fminf(x[6], x[7])));
+                    m[j8] = fminf(fmin3(x[0], x[1], x[2]), fmin3(fmin3(x[3], x[4], x[5]), x[6], x[7]));
                 }
-                const float mall = fminf(fminf(fminf(m[0], m[1]), fminf(m[2], m[3])),
-                                         fminf(fminf(m[4], m[5]), fminf(m[6], m[7])));
-                if (!__any_sync(0xFFFFFFFFu, mall < thr)) continue;
+                const float mall = fminf(fmin3(m[0], m[1], m[2]), fmin3(fmin3(m[3], m[4], m[5]), m[6], m[7]));
+                if (!__any_sync(0xFFFFFFFFu, mall < thr)) {
+                    if constexpr (!BOUND) release();
+                    continue;
+                }
                 if constexpr (BOUND) {
                     if (__any_sync(0xFFFFFFFFu, cnt > BOUND_SLOTS - 8)) {  // a tile adds up to 8
                         thr = fminf(thr, bound_cut(cs, owner, cnt));
@@ -707,24 +827,47 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
                         }
                     }
                 } else {
+                    // the 8-column groups with a candidate, read again one at a time:
+                    // the same few instructions for all of them (unrolled over the 64
+                    // columns they were fetched anew for each hit), and the columns'
+                    // registers are free for them
+                    unsigned groups = 0;
 #pragma unroll
-                    for (int j8 = 0; j8 < 8; ++j8) {
-                        if (!__any_sync(0xFFFFFFFFu, m[j8] < thr)) continue;
+                    for (int j8 = 0; j8 < 8; ++j8)
+                        groups |= (__any_sync(0xFFFFFFFFu, m[j8] < thr) ? 1u : 0u) << j8;
+#pragma unroll 1
+                    while (groups) {
+                        const uint32_t j8 = (uint32_t)__ffs(groups) - 1;
+                        groups &= groups - 1;
+                        float x[8];
+                        tmem_ld8(taddr + j8 * 8, x);
+                        const uint32_t id = base_idx + j8 * 8;
+                        if (id + 8 > n) {
 #pragma unroll
-                        for (int j = j8 * 8; j < j8 * 8 + 8; ++j) {
-                            if (r[j] < thr) {
-                                cs[off] = r[j];
-                                ci[off] = base_idx + j;
-                                ++cnt;
-                                off += S;
-                                if (cnt >= (uint32_t)RCAND) {
-                                    const Kept kp = row_worst(cs, owner);
-                                    thr = fminf(kp.thr, capv);
-                                    off = kp.off;
-                                }
+                            for (int j = 0; j < 8; ++j)
+                                if (id + j >= n) x[j] = INFINITY;
+                        }
+#pragma unroll
+                        for (int j4 = 0; j4 < 8; j4 += 4) {
+                            uint32_t more = cnt;
+#pragma unroll
+                            for (int j = j4; j < j4 + 4; ++j) more += x[j] < thr ? 1u : 0u;
+                            if (__any_sync(0xFFFFFFFFu, more > (uint32_t)CAND_SLOTS)) {
+                                thr = fminf(thr, cand_cut(cs, ci, owner, cnt, capv));
+                                cnt = cnt < RCAND ? cnt : RCAND;
+                                off = cnt * S + owner;
                             }
+#pragma unroll
+                            for (int j = j4; j < j4 + 4; ++j)
+                                if (x[j] < thr) {
+                                    cs[off] = x[j];
+                                    ci[off] = id + j;
+                                    ++cnt;
+                                    off += S;
+                                }
                         }
                     }
+                    release();
                 }
             }
             if (__any_sync(0xFFFFFFFFu, *abort_flag != 0)) break;
@@ -733,10 +876,11 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
                 if (qrow < nq)
                     for (int s2 = 0; s2 < BOUND_KEEP; ++s2)
                         bound[(qrow * HALVES + h) * BOUND_KEEP + s2] = cs[s2 * S + owner];
-            } else if (qrow < nq) {
-                const uint32_t have = cnt < RCAND ? cnt : RCAND;
-                for (uint32_t s2 = 0; s2 < (uint32_t)RCAND; ++s2)
-                    cand_idx[qrow * RTOTAL + h * RCAND + s2] = s2 < have ? ci[s2 * S + owner] : 0xFFFFFFFFu;
+            } else {
+                cand_cut(cs, ci, owner, cnt, capv);
+                if (qrow < nq)
+                    for (uint32_t s2 = 0; s2 < (uint32_t)RCAND; ++s2)
+                        cand_idx[qrow * RTOTAL + h * RCAND + s2] = s2 < cnt ? ci[s2 * S + owner] : 0xFFFFFFFFu;
             }
         }
     }
