@@ -103,3 +103,20 @@ def test_fp32_halves_against_fp64(n, d, k):
     assert np.array_equal(idx[:, 0], np.arange(n))
     assert np.all(np.isinf(d2[:, m:])) and np.all(idx[:, m:] == 0xFFFFFFFF)
     assert np.all(np.abs(d2[:, :m] - want[:, :m]) <= 2.0 ** -18 * want[:, :m] + 1e-30)
+
+
+@pytest.mark.parametrize("n,d,k", [(640, 6, 15), (2000, 12, 15), (4099, 20, 24)])
+def test_rows_that_fill_up_are_cut_back(n, d, k):
+    """Groups of 64 consecutive points, later ones nearer to the group's centre:
+    all near points of a query stand in the same half of a tile and the nearest
+    come last, so a row fills up and is cut back again and again."""
+    rng = np.random.Generator(np.random.PCG64(n + k))
+    group, place = np.arange(n) // 64, np.arange(n) % 64
+    u = rng.normal(size=(n, d))
+    u /= np.linalg.norm(u, axis=1, keepdims=True)
+    centres = rng.normal(size=(group[-1] + 1, d)) * 8.0
+    X = (centres[group] + u * (4.0 - 3.0 * place / 64)[:, None]).astype(np.float32)
+    a = sc_gpu.knn_gaussian(X, k, precision=sc_gpu.KNN_FP32)
+    b = sc_gpu.knn_gaussian(X, k, precision=sc_gpu.KNN_BF16)
+    assert np.array_equal(a.index, b.index)
+    assert np.array_equal(a.distances.view(np.uint32), b.distances.view(np.uint32))
