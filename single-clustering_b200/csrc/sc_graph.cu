@@ -1238,8 +1238,7 @@ __device__ __forceinline__ void agg_insert_fix_combined(uint32_t* keys, unsigned
                                                         uint64_t mask, bool valid, uint32_t h,
                                                         unsigned long long x, uint32_t* status) {
     const unsigned lane = threadIdx.x & 31u;
-    const unsigned long long key = valid ? (unsigned long long)h : (0xFFFFFFFF00000000ull | lane);
-    const unsigned mm = __match_any_sync(0xFFFFFFFFu, key);
+    const unsigned mm = peers_of(h, valid);
     const unsigned long long acc = peer_sum(mm, valid ? x : 0ull);
     if (!valid || (int)lane != __ffs(mm) - 1) return;
     uint64_t slot = agg_hash(h) & mask;
@@ -1296,8 +1295,7 @@ __global__ void __launch_bounds__(32 * AGG_WARPS)
             for (int k = 0; k < 4; ++k) {
                 if (!__any_sync(FULL, ok[k])) break;
                 // lanes with the same key add through the lowest one (exact regime: any grouping)
-                const unsigned long long key = ok[k] ? (unsigned long long)h[k] : (0xFFFFFFFF00000000ull | (unsigned)lane);
-                const unsigned mm = __match_any_sync(FULL, key);
+                const unsigned mm = peers_of(h[k], ok[k]);
                 const double acc = peer_sum(mm, (double)x[k]);
                 if (ok[k] && lane == __ffs(mm) - 1) agg_insert(keys, vals, (uint32_t)size - 1, h[k], acc, status);
             }
@@ -1506,8 +1504,7 @@ __global__ void __launch_bounds__(AGG_DENSE_THREADS)
                         ok[k] = false;
                     }
                     if (!__any_sync(FULL, ok[k])) continue;
-                    const unsigned long long key = ok[k] ? (unsigned long long)h[k] : (0xFFFFFFFF00000000ull | lane);
-                    const unsigned mm = __match_any_sync(FULL, key);
+                    const unsigned mm = peers_of(h[k], ok[k]);
                     const unsigned long long sum = peer_sum(mm, ok[k] ? fix : 0ull);
                     if (ok[k] && (int)lane == __ffs(mm) - 1) atomicAdd(acc + h[k], sum);
                 }

@@ -13,7 +13,7 @@
 // In the exact regime the fixed-point values are the f64 values themselves.
 //
 // Degree buckets: a group of G = 8 / 16 / 32 lanes per node for degree <= G
-// (neighbour communities merged with __match_any_sync, no shared memory);
+// (neighbour communities merged in registers, no shared memory);
 // one 256-thread block per node above that, with an open-addressing hash in
 // shared memory (global memory past its capacity).
 #include <random>
@@ -58,7 +58,9 @@ __device__ __forceinline__ void flush_counters(unsigned long long* counters, uns
 // another, a division each (two lanes without a candidate take the own and the
 // fresh one); start a block per handful of nodes, so that the prefetch below never
 // ran and every warp ended with three atomics on the same counters. The first
-// batch of a 1M x 30 graph: 210 -> 167 us (G = 16) and 174 -> 105 us (G = 32).
+// batch of a 1M x 30 graph: 210 -> 167 us (G = 16) and 174 -> 105 us (G = 32);
+// 142 and 82 us since the match is one of 32 bits (peers_of) and the argmax is of
+// integer reductions (group_best): waits on shuffles were a third of the stalls.
 template <int G, bool REFINE, bool MULTI>
 __global__ void __launch_bounds__(TB, 4) k_decide_small(Params p, const uint32_t* __restrict__ list,
                                                         const uint64_t* __restrict__ lbeg,
@@ -128,8 +130,7 @@ __global__ void __launch_bounds__(TB, 4) k_decide_small(Params p, const uint32_t
         }
         const double k = from_fix(kf, p.scale), a = from_fix(af, p.nscale);
         if (!REFINE) try_fresh = try_fresh && (!p.has_limit || a <= p.limit);
-        const uint64_t key = valid ? (((uint64_t)gw << 32) | cu) : (0xFFFFFFFF00000000ull | (uint64_t)lane);
-        const unsigned mm = __match_any_sync(FULL, key);
+        const unsigned mm = valid ? peers_of(cu, valid) & gmask : peers_of(cu, valid);
         const bool leader = valid && (__ffs(mm) - 1 == lane);
         const long long acc = peer_sum(mm, valid ? to_fix((double)wt, p.inv_scale) : 0ll);
         // weight to the own community
@@ -192,18 +193,7 @@ __global__ void __launch_bounds__(TB, 4) k_decide_small(Params p, const uint32_t
             snodes += 1;
             sdeg += (unsigned long long)deg;
         }
-        // argmax over the group: higher key, then lower id
-#pragma unroll
-        for (int o = G / 2; o; o >>= 1) {
-            double og = __shfl_xor_sync(FULL, g, o);
-            uint32_t oc = __shfl_xor_sync(FULL, c, o);
-            uint32_t om = __shfl_xor_sync(FULL, cu_member, o);
-            if (better(og, oc, g, c)) {
-                g = og;
-                c = oc;
-                cu_member = om;
-            }
-        }
+        group_best<G>(g, c, cu_member);
         if (!REFINE) {
             if (sub == 0 && eligible) {
                 uint32_t best = own;
@@ -336,8 +326,7 @@ __global__ void __launch_bounds__(32 * WARPS_PER_BLOCK) k_decide_warp(Params p, 
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 if (base0 + 32 * t >= e) break;  // warp-uniform
-                const uint64_t key = ok[t] ? (uint64_t)cu[t] : (0xFFFFFFFF00000000ull | lane);
-                const unsigned peers = __match_any_sync(FULL, key);
+                const unsigned peers = peers_of(cu[t], ok[t]);
                 const long long x = peer_sum(peers, ok[t] ? to_fix((double)w[t], p.inv_scale) : 0ll);
                 if (ok[t] && __ffs(peers) - 1 == lane)
                     hinsert_listed(keys, vals, mask, cu[t], x, p.status, s_list[wib], &s_cnt[wib], WARP_DEGREE);
@@ -373,14 +362,7 @@ __global__ void __launch_bounds__(32 * WARPS_PER_BLOCK) k_decide_warp(Params p, 
                 c = cu;
             }
         }
-        for (int o = 16; o; o >>= 1) {
-            const double og = __shfl_xor_sync(FULL, g, o);
-            const uint32_t oc = __shfl_xor_sync(FULL, c, o);
-            if (better(og, oc, g, c)) {
-                g = og;
-                c = oc;
-            }
-        }
+        warp_best(g, c);
         scand += lc;
         uint32_t target = NONE32;
         long long dg = 0;
@@ -509,8 +491,7 @@ __global__ void __launch_bounds__(TB) k_decide_block(Params p, const uint32_t* _
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
                     if (base0 + t * stride >= e) break;  // warp-uniform
-                    const uint64_t key = ok[t] ? (uint64_t)cu[t] : (0xFFFFFFFF00000000ull | lane);
-                    const unsigned peers = __match_any_sync(0xFFFFFFFFu, key);
+                    const unsigned peers = peers_of(cu[t], ok[t]);
                     const long long x = peer_sum(peers, ok[t] ? to_fix((double)w[t], p.inv_scale) : 0ll);
                     if (ok[t] && __ffs(peers) - 1 == (int)lane) hinsert(keys, vals, mask, cu[t], x, p.status);
                 }
@@ -643,8 +624,11 @@ __global__ void k_apply(Params p, const uint32_t* __restrict__ list, uint32_t co
 // What it appends gathers in a queue of its own in shared memory and goes out
 // with one atomic per some hundred entries: one returning atomic on the one
 // counter for every 16 entries of a row was what bound it (318 us for the first
-// batch of a 1M x 30 graph, 156 now).
-constexpr int ACT_QUEUE = 320;  // entries of a warp's queue: a step adds up to 32
+// batch of a 1M x 30 graph, 139 then). Now it is the round trips: entry, then
+// membership and stamp together, then the atomic; with two row pairs in flight
+// 121 us.
+constexpr int ACT_QUEUE = 320;  // entries of a warp's queue: a row pair adds up to 32
+constexpr int ACT_ROWS = 2;     // row pairs in flight
 __global__ void __launch_bounds__(TB) k_activate(Params p, const uint32_t* __restrict__ list, uint32_t count,
                                                  uint32_t window, uint32_t* stamp, uint32_t mark, uint32_t* next_list,
                                                  uint32_t* next_count) {
@@ -678,29 +662,47 @@ __global__ void __launch_bounds__(TB) k_activate(Params p, const uint32_t* __res
             }
         }
         unsigned todo = __ballot_sync(FULL, moved);
-        while (todo) {  // the lowest two of the moved nodes, half a warp each
-            const unsigned rest = todo & (todo - 1);
-            const int L0 = __ffs(todo) - 1, L1 = rest ? __ffs(rest) - 1 : L0;
-            todo = rest & (rest - 1);
-            const int L = half ? L1 : L0;
-            const uint32_t v = __shfl_sync(FULL, mv, L), t = __shfl_sync(FULL, mt, L);
-            uint32_t d = __shfl_sync(FULL, md, L);
-            const uint64_t b = __shfl_sync(FULL, mb, L);
-            if (half && !rest) d = 0;
-            const uint32_t most = max(d, __shfl_xor_sync(FULL, d, 16));
+        while (todo) {  // the lowest ACT_ROWS pairs of the moved nodes, half a warp a node
+            uint32_t v[ACT_ROWS], t[ACT_ROWS], d[ACT_ROWS], most = 0;
+            uint64_t b[ACT_ROWS];
+#pragma unroll
+            for (int r = 0; r < ACT_ROWS; ++r) {
+                const unsigned rest = todo & (todo - 1);
+                const int L0 = todo ? __ffs(todo) - 1 : 0, L1 = rest ? __ffs(rest) - 1 : L0;
+                const bool none = half ? !rest : !todo;
+                todo = rest & (rest - 1);
+                const int L = half ? L1 : L0;
+                v[r] = __shfl_sync(FULL, mv, L), t[r] = __shfl_sync(FULL, mt, L);
+                d[r] = __shfl_sync(FULL, md, L);
+                b[r] = __shfl_sync(FULL, mb, L);
+                if (none) d[r] = 0;
+                most = max(most, d[r]);
+            }
+            most = max(most, __shfl_xor_sync(FULL, most, 16));
             for (uint32_t j0 = 0; j0 < most; j0 += 16) {
-                uint32_t u = 0;
-                bool add = false;
-                if (j0 + sub < d) {
-                    u = p.nbr[b + j0 + sub];
+                uint32_t u[ACT_ROWS], mu[ACT_ROWS], su[ACT_ROWS];
+#pragma unroll
+                for (int r = 0; r < ACT_ROWS; ++r) u[r] = j0 + sub < d[r] ? p.nbr[b[r] + j0 + sub] : v[r];
+#pragma unroll
+                for (int r = 0; r < ACT_ROWS; ++r)
+                    if (u[r] != v[r]) {
+                        mu[r] = p.memb[u[r]];
+                        su[r] = stamp[u[r]];
+                    }
+                unsigned bal[ACT_ROWS];
+#pragma unroll
+                for (int r = 0; r < ACT_ROWS; ++r) {
                     // a plain read first: a node already queued for the next sweep
                     // (the common case once many of its neighbours moved) costs no atomic
-                    add = u != v && p.memb[u] != t && stamp[u] < mark && atomicMax(stamp + u, mark) < mark;
+                    const bool add =
+                        u[r] != v[r] && mu[r] != t[r] && su[r] < mark && atomicMax(stamp + u[r], mark) < mark;
+                    bal[r] = __ballot_sync(FULL, add);
                 }
-                const unsigned bal = __ballot_sync(FULL, add);
-                if (bal) {
-                    if (add) queue[queued + __popc(bal & ((1u << lane) - 1u))] = u;
-                    queued += __popc(bal);
+#pragma unroll
+                for (int r = 0; r < ACT_ROWS; ++r) {
+                    if (!bal[r]) continue;
+                    if (bal[r] >> lane & 1u) queue[queued + __popc(bal[r] & ((1u << lane) - 1u))] = u[r];
+                    queued += __popc(bal[r]);
                     __syncwarp();
                     if (queued > ACT_QUEUE - 32) flush();
                 }

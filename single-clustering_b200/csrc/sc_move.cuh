@@ -117,6 +117,65 @@ __device__ __forceinline__ bool better(double g, uint32_t c, double bg, uint32_t
     return g > bg || (g == bg && c < bc);
 }
 
+// The best (g, c) of a warp, or of each half, by `better`: the largest key, then
+// the lowest id. Integer reductions of the key's two words in the doubles' order
+// (zeros made positive: they are equal): four rounds of shuffles and double
+// comparisons are a chain of 16 dependent shuffles. A NaN is no candidate.
+__device__ __forceinline__ uint64_t order_key(double g) {
+    const uint64_t b = (uint64_t)__double_as_longlong(g == g ? __dadd_rn(g, 0.0) : -INFINITY);
+    return b ^ ((b >> 63) ? ~0ull : 1ull << 63);
+}
+__device__ __forceinline__ double key_order(uint64_t k) {
+    return __longlong_as_double((long long)(k ^ ((k >> 63) ? 1ull << 63 : ~0ull)));
+}
+
+__device__ __forceinline__ void warp_best(double& g, uint32_t& c) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const uint64_t k = order_key(g);
+    const uint32_t hi = __reduce_max_sync(FULL, (uint32_t)(k >> 32));
+    bool top = (uint32_t)(k >> 32) == hi;
+    const uint32_t lo = __reduce_max_sync(FULL, top ? (uint32_t)k : 0u);
+    top = top && (uint32_t)k == lo;
+    c = __reduce_min_sync(FULL, top ? c : 0xFFFFFFFFu);
+    g = key_order((uint64_t)hi << 32 | lo);
+}
+
+// The same for the groups of G lanes of a warp, with what the best one's lane
+// holds in m.
+template <int G>
+__device__ __forceinline__ void group_best(double& g, uint32_t& c, uint32_t& m) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    if constexpr (G >= 16) {
+        const bool up = G == 16 && (threadIdx.x & 16u);
+        auto max_of = [&](uint32_t x) {
+            if (G == 32) return __reduce_max_sync(FULL, x);
+            const uint32_t a = __reduce_max_sync(FULL, up ? 0u : x), b = __reduce_max_sync(FULL, up ? x : 0u);
+            return up ? b : a;
+        };
+        const uint64_t k = order_key(g);
+        const uint32_t hi = max_of((uint32_t)(k >> 32));
+        bool top = (uint32_t)(k >> 32) == hi;
+        const uint32_t lo = max_of(top ? (uint32_t)k : 0u);
+        top = top && (uint32_t)k == lo;
+        const uint32_t best = ~max_of(top ? ~c : 0u);
+        const unsigned at = __ballot_sync(FULL, top && c == best) & (G == 32 ? FULL : up ? 0xFFFF0000u : 0xFFFFu);
+        m = __shfl_sync(FULL, m, __ffs(at) - 1);
+        c = best;
+        g = key_order((uint64_t)hi << 32 | lo);
+    } else {
+#pragma unroll
+        for (int o = G / 2; o; o >>= 1) {
+            const double og = __shfl_xor_sync(FULL, g, o);
+            const uint32_t oc = __shfl_xor_sync(FULL, c, o), om = __shfl_xor_sync(FULL, m, o);
+            if (better(og, oc, g, c)) {
+                g = og;
+                c = oc;
+                m = om;
+            }
+        }
+    }
+}
+
 __device__ __forceinline__ uint64_t prio(uint64_t seed, uint32_t ep, uint32_t v) {
     return hash3(seed ^ 0xA5A5A5A5DEADBEEFull, ep, v);
 }

@@ -152,8 +152,7 @@ __global__ void k_internal_atomic(const uint32_t* __restrict__ erow, const uint3
                 in = memb[u] == c;
             }
         }
-        const unsigned peers =
-            __match_any_sync(0xFFFFFFFFu, in ? (unsigned long long)c : (0xFFFFFFFF00000000ull | lane));
+        const unsigned peers = peers_of(c, in);
         const double x = peer_sum(peers, in ? (double)w[e] : 0.0);
         if (in && __ffs(peers) - 1 == (int)lane) atomicAdd(local ? s_in + c : internal + c, x);
     }

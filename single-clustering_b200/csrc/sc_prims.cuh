@@ -132,8 +132,16 @@ void zero(Ctx& c, T* d, size_t n) {
 inline void sync(Ctx& c) { SC_CUDA(cudaStreamSynchronize(c.stream)); }
 
 
+// The lanes of the warp that are ok and hold this lane's key; a lane that is not
+// ok is alone. A match of 32 bits: keys of 64 (with the lane above the key where
+// it is not ok) take two. Every lane of the warp must call it.
+__device__ __forceinline__ unsigned peers_of(uint32_t key, bool ok) {
+    const unsigned same = __match_any_sync(0xFFFFFFFFu, key), in = __ballot_sync(0xFFFFFFFFu, ok);
+    return ok ? same & in : 1u << (threadIdx.x & 31u);
+}
+
 // Sum of x over this lane's peers (the lanes holding the same key; `peers` from
-// __match_any_sync), complete in the lowest peer. A tree fold over each peer
+// peers_of), complete in the lowest peer. A tree fold over each peer
 // group's ranks: in round r a peer whose rank has bit r clear adds the value of
 // the next peer above it that is still open, then the peers with bit r set
 // close; five rounds at most. Use it where the grouping cannot change the sum:

@@ -266,17 +266,6 @@ __device__ __forceinline__ uint32_t choose(const Params& p, const NodeCfg& q, co
     return best;
 }
 
-__device__ __forceinline__ void warp_best(double& g, uint32_t& c) {
-    for (int o = 16; o; o >>= 1) {
-        const double og = __shfl_xor_sync(0xFFFFFFFFu, g, o);
-        const uint32_t oc = __shfl_xor_sync(0xFFFFFFFFu, c, o);
-        if (better(og, oc, g, c)) {
-            g = og;
-            c = oc;
-        }
-    }
-}
-
 // One warp decides node v (row at b, deg <= WARP_DEGREE). Returns the number of
 // candidate communities (the same in every lane).
 template <bool REFINE, bool MULTI>
@@ -301,7 +290,7 @@ __device__ uint32_t decide_warp(const Params& p, uint32_t v, uint64_t b, uint32_
             ok0 = u0 != v && (!REFINE || p.constraint[u0] == cv);
             if (ok0) cu0 = p.memb[u0];
         }
-        const unsigned peers = __match_any_sync(FULL, ok0 ? (uint64_t)cu0 : (0xFFFFFFFF00000000ull | lane));
+        const unsigned peers = peers_of(cu0, ok0);
         const long long acc = peer_sum(peers, ok0 ? x : 0ll);
         const bool lead = ok0 && __ffs(peers) - 1 == (int)lane;
         const unsigned ob = __ballot_sync(FULL, lead && cu0 == own);
@@ -358,7 +347,7 @@ __device__ uint32_t decide_warp(const Params& p, uint32_t v, uint64_t b, uint32_
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 if (base0 + 32 * k >= deg) break;  // warp-uniform
-                const unsigned peers = __match_any_sync(FULL, ok[k] ? (uint64_t)cu[k] : (0xFFFFFFFF00000000ull | lane));
+                const unsigned peers = peers_of(cu[k], ok[k]);
                 const long long x = peer_sum(peers, ok[k] ? to_fix((double)w[k], p.inv_scale) : 0ll);
                 if (ok[k] && __ffs(peers) - 1 == (int)lane)
                     hinsert_listed(t.keys, t.vals, mask, cu[k], x, p.status, t.list, s_cnt, WARP_DEGREE);
@@ -485,7 +474,7 @@ __device__ uint32_t decide_group(const Params& p, uint32_t v, uint32_t slots, Te
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             if (j0 + k * grp.threads >= e) break;  // warp-uniform
-            const unsigned peers = __match_any_sync(FULL, ok[k] ? (uint64_t)cu[k] : (0xFFFFFFFF00000000ull | lane));
+            const unsigned peers = peers_of(cu[k], ok[k]);
             const long long x = peer_sum(peers, ok[k] ? to_fix((double)w[k], p.inv_scale) : 0ll);
             if (!ok[k] || __ffs(peers) - 1 != (int)lane) continue;
             if (DENSE) atomicAdd((unsigned long long*)(sums + cu[k]), (unsigned long long)x);
@@ -758,7 +747,7 @@ __device__ void contract_warp(const Params& p, const TeamArgs& a, const TeamSmem
                 h = a.grp[p.nbr[j]];
                 x = to_fix((double)p.w[j], p.inv_scale);
             }
-            const unsigned peers = __match_any_sync(FULL, ok ? (uint64_t)h : (0xFFFFFFFF00000000ull | lane));
+            const unsigned peers = peers_of(h, ok);
             const long long acc = peer_sum(peers, x);
             if (ok && __ffs(peers) - 1 == (int)lane) hinsert(t.keys, t.vals, size - 1, h, acc, a.status);
         }
@@ -816,7 +805,7 @@ __device__ void contract_block(const Params& p, const TeamArgs& a, TeamSmem& s, 
             for (int k = 0; k < 4; ++k) {
                 if (j0 + 32 * k >= e) break;  // warp-uniform
                 const bool ok = h[k] != NONE32;
-                const unsigned peers = __match_any_sync(FULL, ok ? (uint64_t)h[k] : (0xFFFFFFFF00000000ull | lane));
+                const unsigned peers = peers_of(h[k], ok);
                 const long long x = peer_sum(peers, ok ? to_fix((double)w[k], p.inv_scale) : 0ll);
                 if (ok && __ffs(peers) - 1 == (int)lane)
                     atomicAdd((unsigned long long*)(s.dense + h[k]), (unsigned long long)x);
