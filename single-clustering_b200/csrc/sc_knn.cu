@@ -1632,25 +1632,33 @@ __device__ __forceinline__ float unord32(unsigned k) {
 // so its queries need similar clusters.
 constexpr uint32_t FINE = 256;
 
-// |x - m|^2 of a point in registers (zeros past d) and a row of ceil4(d) floats
+// |x - m|^2 of a point in registers (zeros past d) and a row of row_pad(d) floats
 // that starts on 16 bytes (zeros past d: those terms add +0), summed in
-// ascending order. Four values a load: read one at a time, the loads (the same
-// address for every thread of a warp) set the pace of the kernels below.
+// ascending order. 8 values are on their way at once: read one or four at a
+// time, the loads (the same address for every thread of a warp) set the pace of
+// the kernels below (fine cells of 1M x 50: 2.3 ms with one, 2.0 with four, 1.4
+// now).
+__host__ __device__ __forceinline__ uint32_t row_pad(uint32_t d) { return (d + 7) & ~7u; }
 __device__ __forceinline__ float sq_dist_padded(const float (&x)[64], const float* __restrict__ m, uint32_t d) {
     const float4* m4 = reinterpret_cast<const float4*>(m);
     float acc = 0.0f;
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if ((uint32_t)(4 * j) < d) {
-            const float4 v = m4[j];
-            float df = __fsub_rn(x[4 * j], v.x);
-            acc = __fmaf_rn(df, df, acc);
-            df = __fsub_rn(x[4 * j + 1], v.y);
-            acc = __fmaf_rn(df, df, acc);
-            df = __fsub_rn(x[4 * j + 2], v.z);
-            acc = __fmaf_rn(df, df, acc);
-            df = __fsub_rn(x[4 * j + 3], v.w);
-            acc = __fmaf_rn(df, df, acc);
+    for (int j = 0; j < 64; j += 8)
+        if ((uint32_t)j < d) {
+            float4 v[2];
+#pragma unroll
+            for (int t = 0; t < 2; ++t) v[t] = m4[j / 4 + t];
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                float df = __fsub_rn(x[j + 4 * t], v[t].x);
+                acc = __fmaf_rn(df, df, acc);
+                df = __fsub_rn(x[j + 4 * t + 1], v[t].y);
+                acc = __fmaf_rn(df, df, acc);
+                df = __fsub_rn(x[j + 4 * t + 2], v[t].z);
+                acc = __fmaf_rn(df, df, acc);
+                df = __fsub_rn(x[j + 4 * t + 3], v[t].w);
+                acc = __fmaf_rn(df, df, acc);
+            }
         }
     return acc;
 }
@@ -1954,7 +1962,9 @@ __global__ void k_cell_radius(const float* __restrict__ Xs, uint64_t n, uint32_t
 // Bound by the instructions of the tests: 8.3 ms at 1M x 50 with every warp
 // testing every kept cell, a block per cluster in the first test and one float
 // a load; 4.4 with a warp per cluster there, warps that start at different
-// cells and skip the settled ones, and float4 rows.
+// cells and skip the settled ones, and float4 rows; 4.1 with two of them a step.
+// Stopping at a partial sum that excludes the cell for the whole warp made it
+// slower (5.8): the cells the group ball keeps are mostly near.
 __global__ void k_group_cells(const float* __restrict__ Xs, uint64_t n, uint32_t d, const uint32_t* __restrict__ ord,
                               const float* __restrict__ kb, const unsigned long long* __restrict__ gmask,
                               const uint32_t* __restrict__ gown,
@@ -1966,7 +1976,7 @@ __global__ void k_group_cells(const float* __restrict__ Xs, uint64_t n, uint32_t
     const uint64_t r = g * (QT * TILE) + threadIdx.x;
     const bool ok = r < n;
     const uint64_t sq = ok ? ord[r] : ord[n - 1];
-    const uint32_t dp = (d + 3) & ~3u;
+    const uint32_t dp = row_pad(d);
     float x[64];
 #pragma unroll
     for (int j = 0; j < 64; ++j) x[j] = (uint32_t)j < d ? Xs[sq * d + j] : 0.0f;
@@ -2113,7 +2123,7 @@ __global__ void k_order_tiles(const float* __restrict__ Xs, uint64_t n, uint32_t
         uint32_t t = 0xFFFFFFFFu;
         if (k < cnt) {
             t = t0 + k;
-            const float* m = fcent + (uint64_t)tile_cell[t] * ((d + 3) & ~3u);
+            const float* m = fcent + (uint64_t)tile_cell[t] * row_pad(d);
             key = 0.0f;
             for (uint32_t j = 0; j < d; ++j) {
                 const float df = s_c[j] - m[j];
@@ -2405,12 +2415,13 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     for (uint32_t q = 0; q < K; ++q)
         for (uint32_t j = 0; j < fbase[q + 1] - fbase[q]; ++j) cell_rows[fbase[q] + j] = (uint32_t)(start[q] + (uint64_t)j * FINE);
     DBuf<uint32_t> d_cell_rows(c, std::max<uint32_t>(F, 1));
-    const uint32_t dp = (d + 3) & ~3u;  // rows of the centre and direction tables, read as float4
-    DBuf<float> fcent(c, (uint64_t)std::max<uint32_t>(F, 1) * dp);
+    const uint32_t dp = (d + 3) & ~3u;  // rows of the direction tables, read as float4
+    const uint32_t fp = row_pad(d);     // rows of the cells' centres
+    DBuf<float> fcent(c, (uint64_t)std::max<uint32_t>(F, 1) * fp);
     h2d(c, d_cell_rows.get(), cell_rows.data(), F);
-    k_gather_rows_padded<<<grid_for((uint64_t)F * dp, 256), 256, 0, c.stream>>>(Xs.get(), d_cell_rows.get(), F, d, dp,
+    k_gather_rows_padded<<<grid_for((uint64_t)F * fp, 256), 256, 0, c.stream>>>(Xs.get(), d_cell_rows.get(), F, d, fp,
                                                                              fcent.get());
-    k_fine_assign<<<grid_for(n, 256), 256, 0, c.stream>>>(Xs.get(), n, d, cl_s.get(), fcent.get(), dp, d_fbase.get(),
+    k_fine_assign<<<grid_for(n, 256), 256, 0, c.stream>>>(Xs.get(), n, d, cl_s.get(), fcent.get(), fp, d_fbase.get(),
                                                            fine.get());
     SC_LAUNCH_CHECK();
     c.launches += 2;
@@ -2425,7 +2436,7 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
     zero(c, ccnt.get(), F);
     zero(c, crad.get(), F);
     k_cell_count<<<grid_for(n, 256), 256, 0, c.stream>>>(fine_s.get(), n, ccnt.get());
-    k_cell_radius<<<grid_for(n, 256), 256, 0, c.stream>>>(Xs.get(), n, d, fine_s.get(), fcent.get(), dp, crad.get());
+    k_cell_radius<<<grid_for(n, 256), 256, 0, c.stream>>>(Xs.get(), n, d, fine_s.get(), fcent.get(), fp, crad.get());
     SC_LAUNCH_CHECK();
     c.launches += 2;
     std::vector<unsigned> h_ccnt(F);

@@ -108,9 +108,9 @@ __device__ __forceinline__ double gain_of(const Params& p, const NodeCfg& q, dou
                                    q.four_m));
     }
     return __dsub_rn(__dadd_rn(wto, sl),
-                     __ddiv_rn(__dmul_rn(__dmul_rn(q.gamma, a),
+                     __dmul_rn(__dmul_rn(__dmul_rn(q.gamma, a),
                                          __dsub_rn(__dadd_rn(__dmul_rn(2.0, nc), a), 1.0)),
-                               2.0));
+                               0.5));  // x / 2, exactly
 }
 
 __device__ __forceinline__ bool better(double g, uint32_t c, double bg, uint32_t bc) {
