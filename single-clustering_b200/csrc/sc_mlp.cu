@@ -73,18 +73,84 @@ constexpr int MLP_BLOCKS = 148 * 4;
 
 // For every stored entry e = (i, j): Σ w_ix over the neighbours x != i of i
 // with label(x) = label(j), over k_i — the entry of i's neighbour-label
-// histogram at j's community, as a share of i's strength. A warp takes a run
-// of the row's 32-entry chunks (the e-chunks) and walks all its chunks (the
-// x-chunks): in each x-chunk the lanes of one label find each other with
-// __match_any_sync, the lowest of them sums the group's weights in lane order,
-// and the warp broadcasts (label, sum) once per distinct label; a lane adds
-// the sums of its entry's label. Per entry the order is fixed (chunks
-// ascending, lanes ascending inside a chunk), so the result is the same on
-// every run.
+// histogram at j's community, as a share of i's strength. The lanes that hold
+// one label in a 32-entry chunk of the row fold their weights in a fixed tree
+// (peer_sum); a label's sums are added in the order of the chunks. So the order
+// is fixed per entry and the result the same on every run.
+
+// One chunk (most rows): the sum is read back from the label's lowest lane.
+__device__ __forceinline__ void label_share_chunk(const uint32_t* __restrict__ nbr, const float* __restrict__ w,
+                                                  const uint32_t* __restrict__ label, uint32_t i, uint64_t a,
+                                                  uint64_t b, double ki, float* __restrict__ share) {
+    const uint64_t e = a + (threadIdx.x & 31u);
+    const bool in = e < b;
+    const uint32_t v = in ? nbr[e] : 0u;
+    const uint32_t l = in ? label[v] : 0u;
+    const double x = in && v != i ? (double)w[e] : 0.0;
+    const unsigned peers = peers_of(l, in);
+    const double sum = __shfl_sync(0xFFFFFFFFu, peer_sum(peers, x), __ffs(peers) - 1);
+    if (in) share[e] = (float)(sum / ki);
+}
+
+// A longer row with few labels: the labels' sums in a table of the warp's own.
+// False (nothing written) when there are more than LS_LABELS labels.
+constexpr uint32_t LS_SLOTS = 512, LS_LABELS = LS_SLOTS / 2, LS_EMPTY = 0xFFFFFFFFu;
+__device__ bool label_share_table(const uint32_t* __restrict__ nbr, const float* __restrict__ w,
+                                  const uint32_t* __restrict__ label, uint32_t i, uint64_t a, uint64_t b, double ki,
+                                  uint32_t* keys, double* sums, float* __restrict__ share) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u;
+    auto slot_of = [](uint32_t l) { return (l * 2654435761u) >> 23; };  // the hash's top 9 bits
+    static_assert(LS_SLOTS == 1u << 9, "slot_of takes 9 bits");
+    for (uint32_t s = lane; s < LS_SLOTS; s += 32) keys[s] = LS_EMPTY;
+    __syncwarp();
+    uint32_t held = 0;
+    for (uint64_t x0 = a; x0 < b; x0 += 32) {
+        const uint64_t x = x0 + lane;
+        const uint32_t v = x < b ? nbr[x] : i;
+        const bool valid = v != i;
+        const uint32_t l = valid ? label[v] : 0u;
+        const unsigned peers = peers_of(l, valid);
+        const double sum = peer_sum(peers, valid ? (double)w[x] : 0.0);
+        bool fresh = false;
+        if (valid && __ffs(peers) - 1 == (int)lane) {  // one lane per label: no two on one sum
+            for (uint32_t h = slot_of(l);; h = (h + 1) & (LS_SLOTS - 1)) {
+                uint32_t k = keys[h];
+                if (k == LS_EMPTY) {
+                    k = atomicCAS(keys + h, LS_EMPTY, l);
+                    fresh = k == LS_EMPTY;
+                }
+                if (fresh || k == l) {
+                    sums[h] = fresh ? sum : sums[h] + sum;
+                    break;
+                }
+            }
+        }
+        held += __popc(__ballot_sync(FULL, fresh));
+        __syncwarp();
+        if (held > LS_LABELS) return false;  // a chunk adds 32 at most: the table never fills
+    }
+    for (uint64_t e = a + lane; e < b; e += 32) {
+        const uint32_t l = label[nbr[e]];
+        double sum = 0.0;
+        for (uint32_t h = slot_of(l);; h = (h + 1) & (LS_SLOTS - 1)) {
+            const uint32_t k = keys[h];
+            if (k == l) sum = sums[h];
+            if (k == l || k == LS_EMPTY) break;
+        }
+        share[e] = (float)(sum / ki);
+    }
+    __syncwarp();  // the table is cleared for the next row
+    return true;
+}
+
+// Any row: the warp takes a run of its chunks (the e-chunks) and walks all its
+// chunks (the x-chunks), whose (label, sum) pairs it broadcasts.
 __device__ void label_share_chunks(const uint32_t* __restrict__ nbr,
                                    const float* __restrict__ w, const uint32_t* __restrict__ label, uint32_t i,
                                    uint64_t a, uint64_t b, uint64_t ce_begin, uint64_t ce_step, double ki,
                                    float* __restrict__ share) {
+    const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
     for (uint64_t e0 = a + ce_begin * 32; e0 < b; e0 += ce_step * 32) {
         const uint64_t e = e0 + lane;
@@ -101,19 +167,14 @@ __device__ void label_share_chunks(const uint32_t* __restrict__ nbr,
                 lx = label[v];
                 wx = w[x];
             }
-            const unsigned long long key = valid ? (unsigned long long)lx : ((1ull << 32) | (unsigned)lane);
-            const unsigned peers = __match_any_sync(0xFFFFFFFFu, key);
-            double sum = 0.0;
-            for (int t = 0; t < 32; ++t) {
-                const float wt = __shfl_sync(0xFFFFFFFFu, wx, t);
-                if ((peers >> t) & 1u) sum += (double)wt;
-            }
-            unsigned leaders = __ballot_sync(0xFFFFFFFFu, valid && (__ffs(peers) - 1) == lane);
+            const unsigned peers = peers_of(lx, valid);
+            const double sum = peer_sum(peers, valid ? (double)wx : 0.0);
+            unsigned leaders = __ballot_sync(FULL, valid && (__ffs(peers) - 1) == lane);
             while (leaders) {
                 const int l = __ffs(leaders) - 1;
                 leaders &= leaders - 1;
-                const uint32_t Ll = __shfl_sync(0xFFFFFFFFu, lx, l);
-                const double Sl = __shfl_sync(0xFFFFFFFFu, sum, l);
+                const uint32_t Ll = __shfl_sync(FULL, lx, l);
+                const double Sl = __shfl_sync(FULL, sum, l);
                 if (Ll == L) acc += Sl;
             }
         }
@@ -122,16 +183,25 @@ __device__ void label_share_chunks(const uint32_t* __restrict__ nbr,
 }
 
 // Rows of at most 32 chunks: a warp per row. Longer rows are left to
-// k_label_share_big.
-__global__ void k_label_share(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ nbr,
-                              const float* __restrict__ w, const uint32_t* __restrict__ label,
-                              const double* __restrict__ strength, uint64_t n, float* __restrict__ share) {
+// k_label_share_big. A launch on the 100k x 50 kNN graph waited for the warps of
+// its longest rows, whose every e-chunk walked every x-chunk and summed by 32
+// broadcasts: 456 us; 100 with the table and peer_sum.
+__global__ void __launch_bounds__(TB) k_label_share(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ nbr,
+                                                    const float* __restrict__ w, const uint32_t* __restrict__ label,
+                                                    const double* __restrict__ strength, uint64_t n,
+                                                    float* __restrict__ share) {
+    __shared__ uint32_t s_keys[TB / 32][LS_SLOTS];
+    __shared__ double s_sums[TB / 32][LS_SLOTS];
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint32_t wib = threadIdx.x >> 5;
     for (uint64_t i = warp; i < n; i += nwarps) {
         const uint64_t a = ptr[i], b = ptr[i + 1];
+        const double ki = fmax(strength[i], 1e-300);
         if (b - a > 32 * 32) continue;
-        label_share_chunks(nbr, w, label, (uint32_t)i, a, b, 0, 1, fmax(strength[i], 1e-300), share);
+        if (b - a <= 32) label_share_chunk(nbr, w, label, (uint32_t)i, a, b, ki, share);
+        else if (!label_share_table(nbr, w, label, (uint32_t)i, a, b, ki, s_keys[wib], s_sums[wib], share))
+            label_share_chunks(nbr, w, label, (uint32_t)i, a, b, 0, 1, ki, share);
     }
 }
 
@@ -759,15 +829,20 @@ void launch_mlp_tc(Ctx& c, const float* feat, const uint8_t* label, uint64_t M, 
     c.launches++;
 }
 
+// The blocks' gradients summed in block order, a thread a parameter. Bound by
+// the loads' round trips: 16 are on their way at once, and a warp is a block of
+// its own (81 us with one at a time in 8 blocks of 256 threads; 38 now).
 __global__ void k_grad_reduce(const float* __restrict__ partial, const double* __restrict__ partial_loss, int nblocks,
                               uint64_t M, float* grad, double* loss) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < MLP_NPARAM; i += gridDim.x * blockDim.x) {
         double acc = 0.0;
+#pragma unroll 16
         for (int b = 0; b < nblocks; ++b) acc += partial[(uint64_t)b * MLP_NPARAM + i];
         grad[i] = M ? (float)(acc / (double)M) : 0.0f;  // mean over edges
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
         double acc = 0.0;
+#pragma unroll 16
         for (int b = 0; b < nblocks; ++b) acc += partial_loss[b];
         *loss = M ? acc / (double)M : 0.0;
     }
@@ -1033,7 +1108,7 @@ double grad_at(Ctx& c, const Mlp& m, const EdgeSet& es, const uint8_t* labels, f
     DBuf<float> partial(c, (uint64_t)MLP_BLOCKS * MLP_NPARAM);
     DBuf<double> partial_loss(c, MLP_BLOCKS), loss(c, 1);
     launch_mlp_tc<true>(c, es.feat.get(), labels, es.M, wb.get(), nullptr, partial.get(), partial_loss.get());
-    k_grad_reduce<<<8, 256, 0, c.stream>>>(partial.get(), partial_loss.get(), MLP_BLOCKS, es.M, d_grad, loss.get());
+    k_grad_reduce<<<(MLP_NPARAM + 31) / 32 + 1, 32, 0, c.stream>>>(partial.get(), partial_loss.get(), MLP_BLOCKS, es.M, d_grad, loss.get());
     SC_LAUNCH_CHECK();
     c.launches += 3;
     return to_host(c, loss.get());
