@@ -97,6 +97,7 @@ sc_status init_ctx(sc::Ctx& c, int device, bool side_streams = true) {
         if (cudaEventCreateWithFlags(&c.ev_aux_start, cudaEventDisableTiming) != cudaSuccess) return SC_E_CUDA;
         if (cudaEventCreateWithFlags(&c.ev_aux_done, cudaEventDisableTiming) != cudaSuccess) return SC_E_CUDA;
     }
+    if (cudaEventCreateWithFlags(&c.ev_read, cudaEventDisableTiming) != cudaSuccess) return SC_E_CUDA;
     if (cudaHostAlloc((void**)&c.mailbox, sc::MAILBOX_BYTES, cudaHostAllocDefault) != cudaSuccess) {
         c.mailbox = nullptr;
         return SC_E_CUDA;
@@ -130,6 +131,8 @@ void release_ctx(sc::Ctx& c) {
     }
     if (c.ev_fork) cudaEventDestroy(c.ev_fork);
     c.ev_fork = nullptr;
+    if (c.ev_read) cudaEventDestroy(c.ev_read);
+    c.ev_read = nullptr;
     if (c.aux) {
         cudaStreamSynchronize(c.aux);
         cudaStreamDestroy(c.aux);

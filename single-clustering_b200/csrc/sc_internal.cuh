@@ -96,6 +96,7 @@ struct Ctx {
     // (bucket counts, counters, sizes): copies into it are truly asynchronous, so
     // several can be queued and completed by one stream synchronisation
     uint8_t* mailbox = nullptr;
+    cudaEvent_t ev_read = nullptr;  // a mailbox read that later work on the stream does not wait for
     // pinned staging lanes of large copies to and from pageable memory (created on first use)
     struct Staging* staging = nullptr;
     // large results come back through the staging lanes; not on the contexts of

@@ -739,8 +739,10 @@ __device__ __forceinline__ int bucket_of(uint32_t deg, Route r) {
 template <bool MULTI>
 __global__ void k_bucket_count(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ alist,
                                const uint32_t* __restrict__ acount, uint64_t n, uint64_t seed, uint32_t sweep, int B,
-                               Route route, uint32_t* counts, const uint32_t* inst, const InstCfg* icfg) {
+                               Route route, uint32_t* counts, uint32_t* next_count, const uint32_t* inst,
+                               const InstCfg* icfg) {
     __shared__ uint32_t sc[64];
+    if (next_count && blockIdx.x == 0 && threadIdx.x == 0) *next_count = 0;  // the list this sweep fills
     for (int t = threadIdx.x; t < B * NBUCKET; t += blockDim.x) sc[t] = 0;
     __syncthreads();
     const uint64_t m = alist ? *acount : n;
@@ -766,11 +768,16 @@ template <bool MULTI>
 __global__ void __launch_bounds__(TB)
     k_bucket_scatter(const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ alist,
                      const uint32_t* __restrict__ acount, uint64_t n, uint64_t seed, uint32_t sweep, int B, Route route,
-                     uint32_t* cursor, uint32_t* list, uint64_t* lbeg, uint32_t* ldeg, const uint32_t* inst,
+                     const uint32_t* __restrict__ counts, uint32_t* cursor, uint32_t* list, uint64_t* lbeg, uint32_t* ldeg, const uint32_t* inst,
                      const InstCfg* icfg) {
-    __shared__ uint32_t s_cnt[MAX_SLOTS], s_base[MAX_SLOTS];
+    __shared__ uint32_t s_cnt[MAX_SLOTS], s_base[MAX_SLOTS], s_off[MAX_SLOTS];
     const unsigned lane = threadIdx.x & 31u;
     const int slots = B * NBUCKET;
+    if ((int)threadIdx.x < slots) {  // where each list begins
+        uint32_t off = 0;
+        for (int t = 0; t < (int)threadIdx.x; ++t) off += counts[t];
+        s_off[threadIdx.x] = off;
+    }
     const uint64_t m = alist ? *acount : n;
     for (uint64_t base = blockIdx.x * (uint64_t)(TB * SCATTER_ITEMS); base < m;
          base += (uint64_t)gridDim.x * (TB * SCATTER_ITEMS)) {  // block-uniform
@@ -804,7 +811,8 @@ __global__ void __launch_bounds__(TB)
             rank[t] = __shfl_sync(0xFFFFFFFFu, first, leader) + __popc(mm & ((1u << lane) - 1u));
         }
         __syncthreads();
-        for (int t = threadIdx.x; t < slots; t += TB) s_base[t] = s_cnt[t] ? atomicAdd(cursor + t, s_cnt[t]) : 0u;
+        for (int t = threadIdx.x; t < slots; t += TB)
+            s_base[t] = s_cnt[t] ? s_off[t] + atomicAdd(cursor + t, s_cnt[t]) : 0u;
         __syncthreads();
 #pragma unroll
         for (int t = 0; t < SCATTER_ITEMS; ++t) {
@@ -870,6 +878,50 @@ Scales scales_for(const DevGraph& g) {
     return s;
 }
 
+// What steers a level's sweeps, in one place: cleared and read back together.
+struct SweepHead {
+    unsigned long long counters[4];
+    long long gain;
+    uint32_t counts[MAX_SLOTS];  // per (batch, bucket): entries of the sweep's lists
+    uint32_t cursor[MAX_SLOTS];  // entries already placed
+};
+
+// The start of a level's local moving or refinement, in one launch: the per-node
+// state cleared, the communities (ids < S) empty, or (identity: refinement) one
+// per node with that node in it. Cleared one array at a time, with the singletons
+// counted by atomics, it was 8 to 13 launches (and 0.35 ms for 4M singletons).
+struct LevelStart {
+    uint64_t n, S;
+    uint32_t *epoch, *moved, *stamp, *hint;  // n each; the last three nullable
+    long long *Kf, *Wf;                      // S each; Wf nullable
+    uint32_t* csize;
+    unsigned long long* claim;  // S, nullable
+    SweepHead* head;
+    uint32_t* identity;  // n, nullable
+    const double *strength, *node_w;
+    double inv_scale, inv_nscale;
+};
+__global__ void k_level_start(LevelStart a) {
+    if (blockIdx.x == 0)
+        for (uint32_t i = threadIdx.x; i < sizeof(SweepHead) / 4; i += blockDim.x)
+            reinterpret_cast<uint32_t*>(a.head)[i] = 0;
+    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < a.S;
+         v += (uint64_t)gridDim.x * blockDim.x) {
+        const bool node = v < a.n, single = node && a.identity;
+        if (node) {
+            a.epoch[v] = 0;
+            if (a.moved) a.moved[v] = 0;
+            if (a.stamp) a.stamp[v] = 0;
+            if (a.hint) a.hint[v] = 0;
+        }
+        if (single) a.identity[v] = (uint32_t)v;
+        a.Kf[v] = single ? to_fix(a.strength[v], a.inv_scale) : 0ll;
+        if (a.Wf) a.Wf[v] = single ? to_fix(a.node_w[v], a.inv_nscale) : 0ll;
+        a.csize[v] = single ? 1u : 0u;
+        if (a.claim) a.claim[v] = 0;
+    }
+}
+
 struct Workspace {
     DBuf<uint32_t> tgt, hint, from, epoch, list, moved;
     DBuf<uint64_t> lbeg;  // row start of each list entry (written by the bucket scatter)
@@ -878,10 +930,7 @@ struct Workspace {
     DBuf<uint32_t> alist, nlist;    // this sweep's active nodes, the next sweep's
     DBuf<uint32_t> acount, ncount;  // their counts (device)
     DBuf<uint32_t> stamp;           // per node: 1 + the last sweep it was queued for
-    DBuf<uint32_t> counts;
-    DBuf<uint32_t> cursor;  // scatter cursors of the (batch, bucket) lists
-    DBuf<unsigned long long> counters;
-    DBuf<long long> gain_acc;
+    DBuf<SweepHead> head;
     DBuf<uint32_t> gkeys;
     DBuf<long long> gvals;
     uint64_t gcap = 0;
@@ -961,15 +1010,9 @@ void prepare_workspace(Ctx& c, Workspace& ws, const DevGraph& g) {
         ws.acount.alloc(c, 1);
         ws.ncount.alloc(c, 1);
         ws.stamp.alloc(c, m);
-        ws.counts.alloc(c, 64);
-        ws.cursor.alloc(c, 64);
-        ws.counters.alloc(c, 4);
-        ws.gain_acc.alloc(c, 1);
+        ws.head.alloc(c, 1);
         ws.cap = m;
     }
-    zero(c, ws.epoch.get(), n);
-    zero(c, ws.moved.get(), n);
-    zero(c, ws.hint.get(), n);
     // global hash / candidate scratch, one slice per block, for the hubs only
     ws.nblk_large = 0;
     ws.gcap = 0;
@@ -1098,30 +1141,32 @@ void batch_decide(Ctx& c, Params& p, Workspace& ws, const uint32_t* offs, int b)
 }
 
 void launch_bucket_count(Ctx& c, const Params& p, const DevGraph& g, const uint32_t* alist, const uint32_t* acount,
-                         uint64_t seed, uint32_t sweep, int B, uint32_t* counts) {
+                         uint64_t seed, uint32_t sweep, int B, uint32_t* counts, uint32_t* next_count) {
     const uint64_t n = g.n;
     if (p.inst)
         k_bucket_count<true><<<grid_for(n, TB), TB, 0, c.stream>>>(g.ptr, alist, acount, n, seed, sweep, B,
-                                                                   route_of(c), counts, p.inst, p.icfg);
+                                                                   route_of(c), counts, next_count, p.inst, p.icfg);
     else
         k_bucket_count<false><<<grid_for(n, TB), TB, 0, c.stream>>>(g.ptr, alist, acount, n, seed, sweep, B,
-                                                                    route_of(c), counts, nullptr, nullptr);
+                                                                    route_of(c), counts, next_count, nullptr, nullptr);
     SC_LAUNCH_CHECK();
     c.launches++;
 }
 
+// The grid is for all nodes: the host does not know yet how many are active.
 void launch_bucket_scatter(Ctx& c, const Params& p, const DevGraph& g, const uint32_t* alist,
-                           const uint32_t* acount, uint64_t work, uint64_t seed, uint32_t sweep, int B,
-                           Workspace& ws) {
+                           const uint32_t* acount, uint64_t seed, uint32_t sweep, int B, Workspace& ws) {
     const uint64_t n = g.n;
+    const unsigned grid = grid_for(n, TB * SCATTER_ITEMS);
+    SweepHead* h = ws.head.get();
     if (p.inst)
-        k_bucket_scatter<true><<<grid_for(work, TB * SCATTER_ITEMS), TB, 0, c.stream>>>(g.ptr, alist, acount, n, seed, sweep, B,
-                                                                        route_of(c), ws.cursor.get(), ws.list.get(),
-                                                                        ws.lbeg.get(), ws.ldeg.get(), p.inst, p.icfg);
+        k_bucket_scatter<true><<<grid, TB, 0, c.stream>>>(g.ptr, alist, acount, n, seed, sweep, B, route_of(c),
+                                                          h->counts, h->cursor, ws.list.get(), ws.lbeg.get(),
+                                                          ws.ldeg.get(), p.inst, p.icfg);
     else
-        k_bucket_scatter<false><<<grid_for(work, TB * SCATTER_ITEMS), TB, 0, c.stream>>>(g.ptr, alist, acount, n, seed, sweep, B,
-                                                                         route_of(c), ws.cursor.get(), ws.list.get(),
-                                                                         ws.lbeg.get(), ws.ldeg.get(), nullptr, nullptr);
+        k_bucket_scatter<false><<<grid, TB, 0, c.stream>>>(g.ptr, alist, acount, n, seed, sweep, B, route_of(c),
+                                                           h->counts, h->cursor, ws.list.get(), ws.lbeg.get(),
+                                                           ws.ldeg.get(), nullptr, nullptr);
     SC_LAUNCH_CHECK();
     c.launches++;
 }
@@ -1151,14 +1196,14 @@ MoveResult local_move(Ctx& c, const DevGraph& g, Workspace& ws, uint32_t* memb, 
     DBuf<long long> Kf(c, S), Wf(c, need_nc ? S : 0);  // Wf only where CPM or the cap reads it
     DBuf<uint32_t> csize(c, S);
     DBuf<unsigned long long> claim(c, cfg.has_max_community_weight ? S : 0);
-    zero(c, claim.get(), claim.n);
-    zero(c, Kf.get(), S);
-    zero(c, Wf.get(), Wf.n);
-    zero(c, csize.get(), S);
+    const LevelStart start{n, S, ws.epoch.get(), ws.moved.get(), ws.stamp.get(), ws.hint.get(), Kf.get(),
+                           need_nc ? Wf.get() : nullptr, csize.get(), claim.n ? claim.get() : nullptr, ws.head.get(),
+                           nullptr, g.strength, g.node_w, sc.inv, sc.ninv};
+    k_level_start<<<grid_for(S, TB), TB, 0, c.stream>>>(start);
     k_init_comm<<<grid_for(n, TB), TB, 0, c.stream>>>(memb, n, g.strength, g.node_w, sc.inv, sc.ninv,
                                                       Kf.get(), Wf.get(), csize.get());
     SC_LAUNCH_CHECK();
-    c.launches++;
+    c.launches += 2;
     Params p{};
     p.ptr = g.ptr;
     p.nbr = g.nbr;
@@ -1191,8 +1236,8 @@ MoveResult local_move(Ctx& c, const DevGraph& g, Workspace& ws, uint32_t* memb, 
     p.theta = 0.0;
     p.seed = seed;
     p.status = c.d_status;
-    p.counters = ws.counters.get();
-    p.gain_acc = ws.gain_acc.get();
+    p.counters = ws.head.get()->counters;
+    p.gain_acc = &ws.head.get()->gain;
     p.claim = claim.get();
     p.moved = ws.moved.get();
     if (ml) {
@@ -1200,11 +1245,6 @@ MoveResult local_move(Ctx& c, const DevGraph& g, Workspace& ws, uint32_t* memb, 
         p.icfg = ml->icfg;
         p.gain_inst = ml->gain_inst;
     }
-    zero(c, ws.counters.get(), 4);
-    zero(c, ws.gain_acc.get(), 1);
-    zero(c, ws.epoch.get(), n);
-    zero(c, ws.moved.get(), n);
-    zero(c, ws.stamp.get(), n);
     bool all_active = true;  // sweep 0 visits every node
     const int B = LM_BATCHES;
     uint32_t epoch = 0;
@@ -1216,18 +1256,23 @@ MoveResult local_move(Ctx& c, const DevGraph& g, Workspace& ws, uint32_t* memb, 
     bool read_fresh = false;  // last_ctr / last_gacc hold the counters' current values
     const uint32_t tail = tail_limit(c, g, cfg);
     for (uint32_t sweep = 0; sweep < (uint32_t)MAX_SWEEPS; ++sweep) {
-        zero(c, ws.counts.get(), B * NBUCKET);
-        zero(c, ws.ncount.get(), 1);
+        if (sweep > 0) zero(c, ws.head.get()->counts, 2 * MAX_SLOTS);  // and the cursors behind them
         const uint32_t* alist = all_active ? nullptr : ws.alist.get();
-        launch_bucket_count(c, p, g, alist, ws.acount.get(), seed, sweep, B, ws.counts.get());
+        launch_bucket_count(c, p, g, alist, ws.acount.get(), seed, sweep, B, ws.head.get()->counts, ws.ncount.get());
         uint32_t counts[64];
         unsigned long long ctr[4];
         {
+            // the lists are written while the host reads their sizes and decides
+            // what the sweep does with them
             Mailbox mb(c);
-            const uint32_t* hc = mb.get(ws.counts.get(), B * NBUCKET);
-            const unsigned long long* hk = mb.get(ws.counters.get(), 4);
-            const long long* hg = mb.get(ws.gain_acc.get(), 1);
-            mb.wait();
+            const SweepHead* h = reinterpret_cast<const SweepHead*>(
+                mb.get(reinterpret_cast<const uint8_t*>(ws.head.get()), offsetof(SweepHead, cursor)));
+            mb.mark();
+            launch_bucket_scatter(c, p, g, alist, ws.acount.get(), seed, sweep, B, ws);
+            mb.wait_marked();
+            const uint32_t* hc = h->counts;
+            const unsigned long long* hk = h->counters;
+            const long long* hg = &h->gain;
             std::memcpy(counts, hc, sizeof(uint32_t) * B * NBUCKET);
             std::memcpy(ctr, hk, sizeof ctr);
             std::memcpy(last_ctr, hk, sizeof ctr);
@@ -1264,9 +1309,6 @@ MoveResult local_move(Ctx& c, const DevGraph& g, Workspace& ws, uint32_t* memb, 
             sweep = t.sweep - 1;
             continue;
         }
-        h2d(c, ws.cursor.get(), offs, B * NBUCKET);
-        launch_bucket_scatter(c, p, g, alist, ws.acount.get(), all_active ? n : offs[B * NBUCKET], seed, sweep, B,
-                              ws);
         // A batch's re-queue reads memberships and writes only the next sweep's
         // list, so with an auxiliary stream it runs while the next batch decides;
         // it must end before the next batch commits (which changes memberships).
@@ -1313,8 +1355,8 @@ MoveResult local_move(Ctx& c, const DevGraph& g, Workspace& ws, uint32_t* memb, 
     }
     if (!read_fresh) {  // the team, or the sweep limit after launching a sweep, ended the loop
         Mailbox mb(c);
-        const unsigned long long* hk = mb.get(ws.counters.get(), 4);
-        const long long* hg = mb.get(ws.gain_acc.get(), 1);
+        const unsigned long long* hk = mb.get(ws.head.get()->counters, 4);
+        const long long* hg = mb.get(&ws.head.get()->gain, 1);
         mb.wait();
         std::memcpy(last_ctr, hk, sizeof last_ctr);
         last_gacc = *hg;
@@ -1352,15 +1394,12 @@ void refine(Ctx& c, const DevGraph& g, Workspace& ws, const uint32_t* constraint
     DBuf<long long> Kf(c, n), Wf(c, need_nc ? n : 0);  // Wf only where CPM or the cap reads it
     DBuf<uint32_t> csize(c, n);
     DBuf<unsigned long long> claim(c, cfg.has_max_community_weight ? n : 0);
-    zero(c, claim.get(), claim.n);
-    zero(c, Kf.get(), n);
-    zero(c, Wf.get(), Wf.n);
-    zero(c, csize.get(), n);
-    k_identity<<<grid_for(n, TB), TB, 0, c.stream>>>(refined, n);
-    k_init_comm<<<grid_for(n, TB), TB, 0, c.stream>>>(refined, n, g.strength, g.node_w, sc.inv, sc.ninv,
-                                                      Kf.get(), Wf.get(), csize.get());
+    const LevelStart start{n, n, ws.epoch.get(), nullptr, nullptr, nullptr, Kf.get(), need_nc ? Wf.get() : nullptr,
+                           csize.get(), claim.n ? claim.get() : nullptr, ws.head.get(), refined, g.strength, g.node_w,
+                           sc.inv, sc.ninv};
+    k_level_start<<<grid_for(n, TB), TB, 0, c.stream>>>(start);
     SC_LAUNCH_CHECK();
-    c.launches += 2;
+    c.launches++;
     Params p{};
     p.ptr = g.ptr;
     p.nbr = g.nbr;
@@ -1394,8 +1433,8 @@ void refine(Ctx& c, const DevGraph& g, Workspace& ws, const uint32_t* constraint
     p.theta = cfg.refine_randomness * mean_edge;  // refine.rs:44-50
     p.seed = seed;
     p.status = c.d_status;
-    p.counters = ws.counters.get();
-    p.gain_acc = ws.gain_acc.get();
+    p.counters = ws.head.get()->counters;
+    p.gain_acc = &ws.head.get()->gain;
     p.claim = claim.get();
     p.moved = ws.moved.get();
     if (ml) {
@@ -1403,23 +1442,20 @@ void refine(Ctx& c, const DevGraph& g, Workspace& ws, const uint32_t* constraint
         p.icfg = ml->icfg;
         p.gain_inst = ml->gain_inst;
     }
-    zero(c, ws.counters.get(), 4);
-    zero(c, ws.epoch.get(), n);
     const int B = RF_BATCHES;
-    zero(c, ws.counts.get(), B * NBUCKET);
-    launch_bucket_count(c, p, g, nullptr, nullptr, seed, 0xFFFFFFFFu, B, ws.counts.get());
+    launch_bucket_count(c, p, g, nullptr, nullptr, seed, 0xFFFFFFFFu, B, ws.head.get()->counts, nullptr);
     uint32_t counts[64];
     {
         Mailbox mb(c);
-        const uint32_t* hc = mb.get(ws.counts.get(), B * NBUCKET);
-        mb.wait();
+        const uint32_t* hc = mb.get(ws.head.get()->counts, B * NBUCKET);
+        mb.mark();
+        launch_bucket_scatter(c, p, g, nullptr, nullptr, seed, 0xFFFFFFFFu, B, ws);
+        mb.wait_marked();
         std::memcpy(counts, hc, sizeof(uint32_t) * B * NBUCKET);
     }
     uint32_t offs[65];
     offs[0] = 0;
     for (int t = 0; t < B * NBUCKET; ++t) offs[t + 1] = offs[t] + counts[t];
-    h2d(c, ws.cursor.get(), offs, B * NBUCKET);
-    launch_bucket_scatter(c, p, g, nullptr, nullptr, n, seed, 0xFFFFFFFFu, B, ws);
     for (int b = 0; b < B; ++b) {
         p.cur = (uint32_t)(b + 1);
         uint32_t lo = offs[b * NBUCKET], hi = offs[(b + 1) * NBUCKET];
@@ -1429,7 +1465,7 @@ void refine(Ctx& c, const DevGraph& g, Workspace& ws, const uint32_t* constraint
         launch_claim_apply<true>(c, p, ws.list.get() + lo, hi - lo, false);
     }
     // counters go to the run's totals on the device (read once, at the end of the run)
-    k_add_refine_counters<<<1, 32, 0, c.stream>>>(ws.counters.get(), c.d_refine_ctr);
+    k_add_refine_counters<<<1, 32, 0, c.stream>>>(ws.head.get()->counters, c.d_refine_ctr);
     SC_LAUNCH_CHECK();
     c.launches++;
 }

@@ -103,6 +103,10 @@ struct Mailbox {
         return h;
     }
     void wait() { SC_CUDA(cudaStreamSynchronize(c.stream)); }
+    // mark() after the reads, then more work on the stream, then wait_marked():
+    // the host has the words while that work runs
+    void mark() { SC_CUDA(cudaEventRecord(c.ev_read, c.stream)); }
+    void wait_marked() { SC_CUDA(cudaEventSynchronize(c.ev_read)); }
 };
 
 template <class T>
