@@ -240,21 +240,33 @@ __global__ void __launch_bounds__(TB) k_row_stats(const uint64_t* __restrict__ p
             e = ptr[v + 1];
         }
         double sl = 0.0, acc = 0.0;
-        for (uint64_t i = b + sub; i < e; i += 16) {
-            const float x = w[i];
-            const uint32_t u = nbr[i];
-            st.low_w = min(st.low_w, lowbit_exp_f32(x));
-            const double s = (double)x;
-            if (u == (uint32_t)v) {
-                st.loops = 1;
-                sl = s;
-                acc = __dadd_rn(acc, __dmul_rn(2.0, s));
-            } else {
-                acc = __dadd_rn(acc, s);
+        for (uint64_t i0 = b + sub; i0 < e; i0 += 64) {  // four entries' loads in flight
+            float x4[4];
+            uint32_t u4[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const bool in = i0 + 16 * k < e;
+                x4[k] = in ? w[i0 + 16 * k] : 0.0f;
+                u4[k] = in ? nbr[i0 + 16 * k] : 0u;
             }
-            if (u >= (uint32_t)v) {
-                ++st.ecount;
-                st.upper = __dadd_rn(st.upper, s);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (i0 + 16 * k >= e) break;
+                const float x = x4[k];
+                const uint32_t u = u4[k];
+                st.low_w = min(st.low_w, lowbit_exp_f32(x));
+                const double s = (double)x;
+                if (u == (uint32_t)v) {
+                    st.loops = 1;
+                    sl = s;
+                    acc = __dadd_rn(acc, __dmul_rn(2.0, s));
+                } else {
+                    acc = __dadd_rn(acc, s);
+                }
+                if (u >= (uint32_t)v) {
+                    ++st.ecount;
+                    st.upper = __dadd_rn(st.upper, s);
+                }
             }
         }
         for (int o = 8; o; o >>= 1) {
@@ -789,16 +801,78 @@ __global__ void k_group_keys(const uint32_t* __restrict__ erow, const uint32_t* 
     }
 }
 
+// The same entries, compacted as they are found, a block's with one atomic: their
+// order depends on timing, so only where a segment's sum does not depend on its
+// order. Keys and flags of every entry written out, and two selections of them,
+// took 0.71 ms for 57M entries; this takes 0.33.
+constexpr int KEY_ITEMS = 8;
+__global__ void __launch_bounds__(TB) k_group_keys_compact(const uint32_t* __restrict__ erow,
+                                                           const uint32_t* __restrict__ nbr,
+                                                           const float* __restrict__ w,
+                                                           const uint32_t* __restrict__ grp, uint64_t E, uint64_t G,
+                                                           uint64_t* ukeys, float* uw, unsigned long long* count) {
+    __shared__ uint32_t s_warp[TB / 32];
+    __shared__ unsigned long long s_base;
+    const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    for (uint64_t base = blockIdx.x * (uint64_t)(TB * KEY_ITEMS); base < E;
+         base += (uint64_t)gridDim.x * (TB * KEY_ITEMS)) {  // block-uniform
+        uint32_t g[KEY_ITEMS], h[KEY_ITEMS];
+        unsigned taken[KEY_ITEMS], before = 0;
+#pragma unroll
+        for (int t = 0; t < KEY_ITEMS; ++t) {
+            const uint64_t e = base + t * TB + threadIdx.x;
+            g[t] = e < E ? erow[e] : 0u;
+            h[t] = e < E ? nbr[e] : 0u;
+        }
+#pragma unroll
+        for (int t = 0; t < KEY_ITEMS; ++t) {
+            g[t] = grp[g[t]];
+            h[t] = grp[h[t]];
+        }
+#pragma unroll
+        for (int t = 0; t < KEY_ITEMS; ++t) {
+            taken[t] = __ballot_sync(0xFFFFFFFFu, base + t * TB + threadIdx.x < E && h[t] >= g[t]);
+            before += __popc(taken[t]);
+        }
+        if (lane == 0) s_warp[wid] = before;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t sum = 0;
+            for (int k = 0; k < TB / 32; ++k) {
+                const uint32_t x = s_warp[k];
+                s_warp[k] = sum;
+                sum += x;
+            }
+            s_base = atomicAdd(count, (unsigned long long)sum);
+        }
+        __syncthreads();
+        uint64_t at = s_base + s_warp[wid];
+#pragma unroll
+        for (int t = 0; t < KEY_ITEMS; ++t) {
+            if (taken[t] >> lane & 1u) {
+                const uint64_t o = at + __popc(taken[t] & ((1u << lane) - 1u));
+                ukeys[o] = (uint64_t)g[t] * G + h[t];
+                uw[o] = w[base + t * TB + threadIdx.x];
+            }
+            at += __popc(taken[t]);
+        }
+        __syncthreads();  // s_warp and s_base are reused
+    }
+}
+
+// The zero bytes among x[0, n).
+__global__ void k_count_zeros(const uint8_t* __restrict__ x, uint64_t n, unsigned long long* count) {
+    unsigned d = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        d += x[i] == 0;
+    d = __reduce_add_sync(0xFFFFFFFFu, d);
+    if ((threadIdx.x & 31u) == 0 && d) atomicAdd(count, (unsigned long long)d);
+}
+
 __global__ void k_seg_heads(const uint64_t* __restrict__ keys, uint64_t N, uint8_t* head) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < N;
          i += (uint64_t)gridDim.x * blockDim.x)
         head[i] = (i == 0 || keys[i] != keys[i - 1]);
-}
-
-__global__ void k_iota64(uint64_t* p, uint64_t n) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        p[i] = i;
 }
 
 // The (g, h) segments, 32 per warp: acc in (member asc, neighbour asc) order,
@@ -930,11 +1004,10 @@ uint64_t segment_sums(Ctx& c, const uint64_t* keys_s, const float* w_s, uint64_t
     if (N == 0) return 0;
     DBuf<uint8_t> head(c, N);
     k_seg_heads<<<grid_for(N, TB), TB, 0, c.stream>>>(keys_s, N, head.get());
-    DBuf<uint64_t> iota(c, N), seg(c, N), cnt(c, 1);
-    k_iota64<<<grid_for(N, TB), TB, 0, c.stream>>>(iota.get(), N);
+    DBuf<uint64_t> seg(c, N), cnt(c, 1);
     SC_LAUNCH_CHECK();
-    c.launches += 2;
-    select_flagged(c, iota.get(), head.get(), seg.get(), cnt.get(), N);
+    c.launches++;
+    select_indices(c, head.get(), seg.get(), cnt.get(), N);
     const uint64_t P = to_host(c, cnt.get());
     prow.alloc(c, P);
     pcol.alloc(c, P);
@@ -963,25 +1036,26 @@ uint64_t segment_sums(Ctx& c, const uint64_t* keys_s, const float* w_s, uint64_t
     return P;
 }
 
-// Mirror keys (h, g) of the kept off-diagonal pairs.
-__global__ void k_mirror(const uint32_t* __restrict__ prow, const uint32_t* __restrict__ pcol,
-                         const float* __restrict__ pw, uint64_t P, uint64_t G, uint64_t* mkeys,
-                         float* mw, uint8_t* mflag) {
+// Mirror keys (h, g) of the kept pairs, h in the upper word; a diagonal pair gets
+// h = G, past every row, and is counted.
+__global__ void k_mirror(const uint32_t* __restrict__ prow, const uint32_t* __restrict__ pcol, uint64_t P, uint64_t G,
+                         uint64_t* mkeys, unsigned long long* diagonal) {
+    unsigned d = 0;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < P;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t g = prow[i], h = pcol[i];
-        mkeys[i] = h * G + g;
-        mw[i] = pw[i];
-        mflag[i] = h != g;
+        const uint32_t g = prow[i], h = pcol[i];
+        d += h == g;
+        mkeys[i] = (h == g ? G : (uint64_t)h) << 32 | g;
     }
+    d = __reduce_add_sync(0xFFFFFFFFu, d);
+    if ((threadIdx.x & 31u) == 0 && d) atomicAdd(diagonal, (unsigned long long)d);
 }
 
-__global__ void k_key_rows(const uint64_t* __restrict__ keys, uint64_t N, uint64_t G, uint32_t* rows,
-                           uint32_t* cols) {
+__global__ void k_key_rows(const uint64_t* __restrict__ keys, uint64_t N, uint32_t* rows, uint32_t* cols) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < N;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        rows[i] = (uint32_t)(keys[i] / G);
-        cols[i] = (uint32_t)(keys[i] % G);
+        rows[i] = (uint32_t)(keys[i] >> 32);
+        cols[i] = (uint32_t)keys[i];
     }
 }
 
@@ -1577,7 +1651,7 @@ constexpr uint64_t AGG_SMALL_GRAPH = 1u << 16;  // entries up to which the hash 
 // The share of the entries in rows past the warp kernel, as 1/AGG_SORT_SHARE,
 // above which a graph of more than AGG_SORT_ENTRIES entries takes the sort path.
 constexpr uint64_t AGG_SORT_SHARE = 10;
-constexpr uint64_t AGG_SORT_ENTRIES = 40000000;
+constexpr uint64_t AGG_SORT_ENTRIES = 6000000;
 constexpr uint64_t AGG_SMEM_KEEP = AGG_SMEM_SLOTS / 2;
 
 // A row has at most min(cap, G) distinct neighbour groups; its table needs twice that.
@@ -1799,8 +1873,10 @@ DevGraph* contract_exact(Ctx& c, const DevGraph& g, const uint32_t* d_grp, uint6
         // Where they hold more than a tenth of the entries the sort path is faster:
         // for big rows on any graph but a small one, whose launches it would only
         // add to; for the others once there are AGG_SORT_ENTRIES entries to amortise
-        // its passes (kNN graphs: 4.4M entries 0.85 ms hashed and 1.07 sorted, 45M
-        // 4.2 both, 57M 7.0 and 6.2). With few groups the dense kernel takes any row.
+        // its passes (kNN graphs, second level: 4.4M entries 0.75 ms hashed and 0.81
+        // sorted, 7.8M 1.57 and 1.03, 21M 2.7 and 1.9, 57M 6.2 and 4.3; first level,
+        // whose rows are short: 25M 2.4 and 2.6, 68M 5.9 and 6.3). With few groups
+        // the dense kernel takes any row.
         if (!dense && g.E > AGG_SMALL_GRAPH &&
             (counts[3] * AGG_SORT_SHARE > g.E || (counts[2] * AGG_SORT_SHARE > g.E && g.E > AGG_SORT_ENTRIES)))
             return nullptr;
@@ -2065,18 +2141,28 @@ DevGraph* graph_aggregate(Ctx& c, const DevGraph& g, const uint32_t* d_grp, uint
     DBuf<uint64_t> ukeys, ukeys_s;
     DBuf<float> uw, uw_s;
     if (E) {
-        DBuf<uint64_t> keys(c, E);
-        DBuf<uint8_t> flags(c, E);
-        k_group_keys<<<grid_for(E, TB), TB, 0, c.stream>>>(g.erow, g.nbr, d_grp, E, G, keys.get(),
-                                                           flags.get());
-        SC_LAUNCH_CHECK();
-        c.launches++;
         ukeys.alloc(c, E);
         uw.alloc(c, E);
         DBuf<uint64_t> cnt(c, 1);
-        select_flagged(c, keys.get(), flags.get(), ukeys.get(), cnt.get(), E);
-        select_flagged(c, g.w, flags.get(), uw.get(), cnt.get(), E);
-        N = to_host(c, cnt.get());
+        if (g.exact_w) {
+            DBuf<unsigned long long> found(c, 1);
+            zero(c, found.get(), 1);
+            k_group_keys_compact<<<grid_for(E, TB * KEY_ITEMS), TB, 0, c.stream>>>(
+                g.erow, g.nbr, g.w, d_grp, E, G, ukeys.get(), uw.get(), found.get());
+            SC_LAUNCH_CHECK();
+            c.launches++;
+            N = to_host(c, found.get());
+        } else {
+            DBuf<uint64_t> keys(c, E);
+            DBuf<uint8_t> flags(c, E);
+            k_group_keys<<<grid_for(E, TB), TB, 0, c.stream>>>(g.erow, g.nbr, d_grp, E, G, keys.get(),
+                                                               flags.get());
+            SC_LAUNCH_CHECK();
+            c.launches++;
+            select_flagged(c, keys.get(), flags.get(), ukeys.get(), cnt.get(), E);
+            select_flagged(c, g.w, flags.get(), uw.get(), cnt.get(), E);
+            N = to_host(c, cnt.get());
+        }
         ukeys_s.alloc(c, N);
         uw_s.alloc(c, N);
         sort_pairs(c, ukeys.get(), ukeys_s.get(), uw.get(), uw_s.get(), N,
@@ -2097,42 +2183,51 @@ DevGraph* graph_aggregate(Ctx& c, const DevGraph& g, const uint32_t* d_grp, uint
     DBuf<uint32_t> krow, kcol;
     DBuf<float> kw;
     if (P) {
-        krow.alloc(c, P);
-        kcol.alloc(c, P);
-        kw.alloc(c, P);
-        DBuf<uint64_t> cnt(c, 1);
-        select_flagged(c, prow.get(), keep.get(), krow.get(), cnt.get(), P);
-        select_flagged(c, pcol.get(), keep.get(), kcol.get(), cnt.get(), P);
-        select_flagged(c, pw.get(), keep.get(), kw.get(), cnt.get(), P);
-        K = to_host(c, cnt.get());
+        DBuf<unsigned long long> dropped(c, 1);
+        zero(c, dropped.get(), 1);
+        k_count_zeros<<<grid_for(P, TB), TB, 0, c.stream>>>(keep.get(), P, dropped.get());
+        SC_LAUNCH_CHECK();
+        c.launches++;
+        K = P - to_host(c, dropped.get());
+        if (K == P) {  // the common case: no pair cancels out
+            krow = std::move(prow);
+            kcol = std::move(pcol);
+            kw = std::move(pw);
+        } else {
+            krow.alloc(c, K);
+            kcol.alloc(c, K);
+            kw.alloc(c, K);
+            DBuf<uint64_t> cnt(c, 1);
+            select_flagged(c, prow.get(), keep.get(), krow.get(), cnt.get(), P);
+            select_flagged(c, pcol.get(), keep.get(), kcol.get(), cnt.get(), P);
+            select_flagged(c, pw.get(), keep.get(), kw.get(), cnt.get(), P);
+        }
     }
     prow.release();
     pcol.release();
     pw.release();
     keep.release();
-    // lower triangle: mirrored off-diagonal pairs sorted by (h, g)
+    // lower triangle: mirrored off-diagonal pairs sorted by (h, g). The pairs come
+    // in the order of g, so a stable sort by h alone gives it, with the diagonal
+    // behind the last row: 57M entries at level 1 of a 4M-point run took two
+    // compactions and five passes over both words, 1.3 ms; 0.8 with three passes.
     uint64_t L = 0;
     DBuf<uint32_t> lrow, lcol;
     DBuf<float> lw;
     if (K) {
-        DBuf<uint64_t> mk(c, K), mk_c(c, K), mk_s(c, K);
-        DBuf<float> mw(c, K), mw_c(c, K);
-        DBuf<uint8_t> mf(c, K);
-        k_mirror<<<grid_for(K, TB), TB, 0, c.stream>>>(krow.get(), kcol.get(), kw.get(), K, G,
-                                                       mk.get(), mw.get(), mf.get());
+        DBuf<uint64_t> mk(c, K), mk_s(c, K);
+        DBuf<unsigned long long> diagonal(c, 1);
+        zero(c, diagonal.get(), 1);
+        k_mirror<<<grid_for(K, TB), TB, 0, c.stream>>>(krow.get(), kcol.get(), K, G, mk.get(), diagonal.get());
         SC_LAUNCH_CHECK();
         c.launches++;
-        DBuf<uint64_t> cnt(c, 1);
-        select_flagged(c, mk.get(), mf.get(), mk_c.get(), cnt.get(), K);
-        select_flagged(c, mw.get(), mf.get(), mw_c.get(), cnt.get(), K);
-        L = to_host(c, cnt.get());
-        lw.alloc(c, L);
-        sort_pairs(c, mk_c.get(), mk_s.get(), mw_c.get(), lw.get(), L,
-                   bits_for((uint64_t)G * G - 1));
+        lw.alloc(c, K);
+        sort_pairs(c, mk.get(), mk_s.get(), kw.get(), lw.get(), K, 32 + bits_for(G), 32);
+        L = K - to_host(c, diagonal.get());
         lrow.alloc(c, L);
         lcol.alloc(c, L);
         if (L) {
-            k_key_rows<<<grid_for(L, TB), TB, 0, c.stream>>>(mk_s.get(), L, G, lrow.get(), lcol.get());
+            k_key_rows<<<grid_for(L, TB), TB, 0, c.stream>>>(mk_s.get(), L, lrow.get(), lcol.get());
             SC_LAUNCH_CHECK();
             c.launches++;
         }

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cub/cub.cuh>
+#include <thrust/iterator/counting_iterator.h>
 
 #include "sc_internal.cuh"
 
@@ -14,15 +15,15 @@ inline int bits_for(uint64_t max_value) {
     return b < 1 ? 1 : b;
 }
 
-// Stable LSD radix sort of (key, value) pairs on bits [0, end_bit).
+// Stable LSD radix sort of (key, value) pairs on bits [begin_bit, end_bit).
 template <class K, class V>
-void sort_pairs(Ctx& c, const K* kin, K* kout, const V* vin, V* vout, size_t n, int end_bit) {
+void sort_pairs(Ctx& c, const K* kin, K* kout, const V* vin, V* vout, size_t n, int end_bit, int begin_bit = 0) {
     if (n == 0) return;
     size_t bytes = 0;
-    SC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kin, kout, vin, vout, n, 0, end_bit,
+    SC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kin, kout, vin, vout, n, begin_bit, end_bit,
                                             c.stream));
     DBuf<uint8_t> tmp(c, bytes);
-    SC_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), bytes, kin, kout, vin, vout, n, 0, end_bit,
+    SC_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), bytes, kin, kout, vin, vout, n, begin_bit, end_bit,
                                             c.stream));
     c.launches += 4;
 }
@@ -78,6 +79,17 @@ void device_min(Ctx& c, const T* in, T* out, size_t n) {
 // Stable compaction of `in` where flags != 0; *d_count receives the kept count.
 template <class T, class F>
 void select_flagged(Ctx& c, const T* in, const F* flags, T* out, uint64_t* d_count, size_t n) {
+    size_t bytes = 0;
+    SC_CUDA(cub::DeviceSelect::Flagged(nullptr, bytes, in, flags, out, d_count, n, c.stream));
+    DBuf<uint8_t> tmp(c, bytes);
+    SC_CUDA(cub::DeviceSelect::Flagged(tmp.get(), bytes, in, flags, out, d_count, n, c.stream));
+    c.launches += 2;
+}
+
+// The indices of the set flags, ascending.
+template <class F>
+void select_indices(Ctx& c, const F* flags, uint64_t* out, uint64_t* d_count, size_t n) {
+    const thrust::counting_iterator<uint64_t> in(0);
     size_t bytes = 0;
     SC_CUDA(cub::DeviceSelect::Flagged(nullptr, bytes, in, flags, out, d_count, n, c.stream));
     DBuf<uint8_t> tmp(c, bytes);

@@ -10,10 +10,10 @@ import sc_gpu
 pytestmark = pytest.mark.gpu
 
 
-def _graph(n, m, seed):
+def _graph(n, m, seed, least=1):
     rng = np.random.Generator(np.random.PCG64(seed))
     src, dst = rng.integers(0, n, m).astype(np.uint64), rng.integers(0, n, m).astype(np.uint64)
-    w = (rng.integers(1, 32, m) / 16.0).astype(np.float64)
+    w = (rng.integers(least, 32, m) / 16.0).astype(np.float64)
     return src, dst, w
 
 
@@ -44,6 +44,23 @@ def test_rows_of_every_kind(n, m, groups, skew):
     assert np.array_equal(a["w"].view(np.uint32), ww.view(np.uint32))
     assert og.modularity(lab) == sc_gpu.modularity(gg, lab)
     assert np.array_equal(a["strength"].view(np.uint64), got.strengths().view(np.uint64))
+
+
+@pytest.mark.parametrize("least", [1, 0])
+@pytest.mark.parametrize("n,m,groups", [(16_000, 3_300_000, 13_000), (60_000, 3_300_000, 13_000)])
+def test_many_entries_in_long_rows_are_sorted(n, m, groups, least):
+    """More entries, most of them in long rows, than the tables are the faster for;
+    with and without pairs of weight zero."""
+    src, dst, w = _graph(n, m, n, least)
+    lab = np.random.Generator(np.random.PCG64(m)).integers(0, groups, n)
+    lab[:groups] = np.arange(groups)
+    lab = lab.astype(np.uint64)
+    og = O.Graph.from_edges(n, src=src, dst=dst, w=w)
+    gg = sc_gpu.CSRNetwork.from_edge_arrays(n, src, dst, w)
+    a = og.aggregate(lab).arrays()
+    ptr, nbr, ww = gg.aggregate(lab).to_csr_parts()
+    assert np.array_equal(a["ptr"], ptr) and np.array_equal(a["nbr"], nbr)
+    assert np.array_equal(a["w"].view(np.uint32), ww.view(np.uint32))
 
 
 @pytest.mark.parametrize("communities", [1, 1023, 1024, 1025])
