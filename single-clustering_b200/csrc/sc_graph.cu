@@ -1327,7 +1327,60 @@ __device__ __forceinline__ void agg_insert_fix_combined(uint32_t* keys, unsigned
     atomicOr(status, DEV_OVERFLOW);
 }
 
-__global__ void __launch_bounds__(32 * AGG_WARPS)
+// A warp's 32 E words ascending, word e in register e % E of lane e / E (bitonic:
+// steps shorter than E stay in the lane, the others take a shuffle a word).
+template <int E>
+__device__ __forceinline__ void warp_sort(uint32_t (&v)[E]) {
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+    for (uint32_t k = 2; k <= 32u * E; k <<= 1)
+#pragma unroll
+        for (uint32_t j = k >> 1; j; j >>= 1)
+#pragma unroll
+            for (uint32_t t = 0; t < (uint32_t)E; ++t) {
+                const bool up = ((lane * E + t) & k) == 0;
+                if (j >= (uint32_t)E) {
+                    const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, v[t], j / E);
+                    v[t] = up == ((lane & (j / E)) == 0) ? min(v[t], o) : max(v[t], o);
+                } else if (!(t & j)) {
+                    const uint32_t a = min(v[t], v[t | j]), b = max(v[t], v[t | j]);
+                    v[t] = up ? a : b;
+                    v[t | j] = up ? b : a;
+                }
+            }
+}
+
+// A row's nk <= 32 E kept entries (lk, lw) written out by neighbour: the group
+// above its place of 8 bits in one word, sorted in registers.
+template <int E>
+__device__ __forceinline__ void write_sorted_row(const uint32_t* lk, const float* lw, uint32_t nk, uint32_t* tnbr,
+                                                 float* tw) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t v[E];
+#pragma unroll
+    for (int t = 0; t < E; ++t) {
+        const uint32_t i = t * 32 + lane;
+        v[t] = i < nk ? lk[i] << 8 | i : 0xFFFFFFFFu;
+    }
+    warp_sort(v);
+#pragma unroll
+    for (int t = 0; t < E; ++t) {
+        const uint32_t e = lane * E + t;
+        if (e < nk) {
+            tnbr[e] = v[t] >> 8;
+            tw[e] = lw[v[t] & 255u];
+        }
+    }
+}
+
+// A warp per coarse row of up to AGG_WARP_CAP entries: a table of its groups in
+// shared memory, the kept ones in order of the group. Bound by instructions;
+// placing each entry by comparing it with all the others was a third of them for
+// the 44 entries of an average row (first level of a 4M x 30 graph: 3.4 ms, 3.1
+// with the sort in registers, which takes groups of 24 bits; past those entries
+// are compared). 2.7 with the kept entries in the table's place and 64 registers:
+// 32 warps an SM instead of 24.
+__global__ void __launch_bounds__(32 * AGG_WARPS, 8)
     k_contract_warp(const uint64_t* __restrict__ gstart, const uint32_t* __restrict__ members, uint64_t G,
                     const uint64_t* __restrict__ ptr, const uint32_t* __restrict__ nbr,
                     const float* __restrict__ w, const uint32_t* __restrict__ grp, const uint64_t* __restrict__ cap,
@@ -1335,14 +1388,13 @@ __global__ void __launch_bounds__(32 * AGG_WARPS)
                     float* tw, uint32_t* cnt, uint32_t* status) {
     __shared__ uint32_t s_keys[AGG_WARPS][2 * AGG_WARP_CAP];
     __shared__ double s_vals[AGG_WARPS][2 * AGG_WARP_CAP];
-    __shared__ uint32_t s_lk[AGG_WARPS][AGG_WARP_CAP];
-    __shared__ float s_lw[AGG_WARPS][AGG_WARP_CAP];
     const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     uint32_t* keys = s_keys[wib];
     double* vals = s_vals[wib];
-    uint32_t* lk = s_lk[wib];
-    float* lw = s_lw[wib];
+    // the kept entries take the place of table slots already read
+    uint32_t* lk = keys;
+    float* lw = reinterpret_cast<float*>(vals);
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t g = warp; g < G; g += nwarps) {
@@ -1382,17 +1434,23 @@ __global__ void __launch_bounds__(32 * AGG_WARPS)
             bool keep = false;
             float val = 0.0f;
             if (h != AGG_EMPTY) val = agg_value((uint32_t)g, h, vals[s], loops, &keep);
-            const unsigned bal = __ballot_sync(FULL, keep);
+            const unsigned bal = __ballot_sync(FULL, keep);  // every lane has read its slot
             if (keep) {
                 const uint32_t pos = nk + __popc(bal & ((1u << lane) - 1u));
                 lk[pos] = h;
                 lw[pos] = val;
             }
             nk += __popc(bal);
+            __syncwarp();
         }
-        __syncwarp();
         const uint64_t o = capstart[g];
-        for (uint32_t i = lane; i < nk; i += 32) {
+        static_assert(AGG_WARP_CAP == 256, "places of 8 bits, at most 8 entries a lane");
+        if (G < (1ull << 24) - 1) {  // warp-uniform
+            if (nk <= 32) write_sorted_row<1>(lk, lw, nk, tnbr + o, tw + o);
+            else if (nk <= 64) write_sorted_row<2>(lk, lw, nk, tnbr + o, tw + o);
+            else if (nk <= 128) write_sorted_row<4>(lk, lw, nk, tnbr + o, tw + o);
+            else write_sorted_row<8>(lk, lw, nk, tnbr + o, tw + o);
+        } else for (uint32_t i = lane; i < nk; i += 32) {
             const uint32_t h = lk[i];
             uint32_t r = 0;
             for (uint32_t j = 0; j < nk; ++j) r += lk[j] < h;

@@ -773,11 +773,14 @@ __global__ void __launch_bounds__(TB)
     __shared__ uint32_t s_cnt[MAX_SLOTS], s_base[MAX_SLOTS], s_off[MAX_SLOTS];
     const unsigned lane = threadIdx.x & 31u;
     const int slots = B * NBUCKET;
+    if ((int)threadIdx.x < slots) s_base[threadIdx.x] = counts[threadIdx.x];
+    __syncthreads();
     if ((int)threadIdx.x < slots) {  // where each list begins
         uint32_t off = 0;
-        for (int t = 0; t < (int)threadIdx.x; ++t) off += counts[t];
+        for (int t = 0; t < (int)threadIdx.x; ++t) off += s_base[t];
         s_off[threadIdx.x] = off;
     }
+    __syncthreads();
     const uint64_t m = alist ? *acount : n;
     for (uint64_t base = blockIdx.x * (uint64_t)(TB * SCATTER_ITEMS); base < m;
          base += (uint64_t)gridDim.x * (TB * SCATTER_ITEMS)) {  // block-uniform
