@@ -906,20 +906,28 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
 // Bound by FP32 issue: 2 DP operations a pair (DP: d rounded up to 4, a register
 // array's size). One query a thread left it bound by the broadcast loads
 // instead (a 16-byte load feeds 8 operations, and holds the SM's one load
-// pipe as long as these take): 8.7 ms at 30,011 x 50, 6.3 with two queries and
-// two points at a time (four independent sums). Each half of
-// the points has blocks of its own (blockIdx.y) and keeps its RCAND best in its
-// half of the candidate slots, so small blocks spread evenly (470 of them
-// there). A candidate is two predicated stores into the query's F32_SLOTS
+// pipe as long as these take): 8.7 ms at 30,011 x 50, 6.3 with two queries
+// (and two or four points at a time). The work
+// items (F32_QUERIES queries x a half of the points, the half's RCAND best in its
+// half of the candidate slots) are cut into equal runs of point tiles, one run a
+// resident block, so that a few items fill the chip too: a block per item took
+// 275 us at 1,000 x 30 points, 780 at 5,003 x 30 and 57.3 ms at 100,000 x 50, the
+// runs take 47, 500 and 53.8; at 30,011 x 50 both take 6.3 ms, bound by the load
+// pipe: a 16-byte load feeds 16 operations of a warp and four warps share the
+// pipe. More queries a thread would need more slots than shared memory holds. An
+// item that several blocks share goes through their lists in scratch
+// (k_f32_merge).
+//
+// A candidate is two predicated stores into the query's F32_SLOTS
 // slots; when a row of the warp is nearly full, all rows are cut back to their
 // RCAND best together. The floor is 2.5 ms of FP32 operations; one query a thread,
 // a search of the row for every insertion and DP = 64 for all d > 32 took 9.1 ms.
 constexpr int F32_THREADS = 64;
 constexpr int F32_Q = 2;  // queries a thread
 constexpr int F32_QUERIES = F32_THREADS * F32_Q;
-constexpr int F32_TILE = 64;
-constexpr int F32_SLOTS = 40;
-constexpr int F32_GROUP = 2;  // points taken together: four independent sums a thread
+constexpr int F32_TILE = 32;
+constexpr int F32_SLOTS = 44;
+constexpr int F32_GROUP = 4;  // points taken together: eight independent sums a thread
 
 // Cuts a row of `cnt` candidates to its RCAND best (the last one takes the worst
 // one's slot until RCAND are left); returns the worst kept, or thr with fewer.
@@ -944,91 +952,162 @@ __device__ __noinline__ float f32_cut(float* cs, uint32_t* ci, uint32_t cnt, flo
     return thr;
 }
 
+// The runs: unit u is tile u % per of item u / per, block b takes units
+// [first(b), first(b + 1)).
+struct F32Plan {
+    uint64_t units, per;
+    uint32_t blocks;
+    __host__ __device__ uint64_t first(uint64_t b) const { return b * units / blocks; }
+    __host__ __device__ uint64_t block_of(uint64_t u) const {
+        uint64_t b = u * blocks / units;
+        while (first(b + 1) <= u) ++b;
+        while (first(b) > u) --b;
+        return b;
+    }
+};
+
 template <int DP>
 __global__ void __launch_bounds__(F32_THREADS) k_knn_fp32(const float* __restrict__ X, uint64_t n, uint32_t d,
-                                                          uint64_t q0, uint64_t nq, uint32_t* __restrict__ cand_idx) {
+                                                          uint64_t q0, uint64_t nq, F32Plan plan,
+                                                          uint32_t* __restrict__ cand_idx,
+                                                          unsigned long long* __restrict__ shared_lists) {
     extern __shared__ __align__(16) unsigned char smem[];
     float* tile = (float*)smem;                                // [F32_TILE][DP]
     float* cs = tile + F32_TILE * DP + threadIdx.x;            // [F32_SLOTS][F32_QUERIES], this thread's columns
     uint32_t* ci = (uint32_t*)(cs + F32_SLOTS * F32_QUERIES);  // at 0 and F32_THREADS; the ids beside them
     const uint32_t t = threadIdx.x;
-    const uint64_t lq0 = (uint64_t)blockIdx.x * F32_QUERIES + t;
-    float q[F32_Q][DP], thr[F32_Q];
-    uint32_t cnt[F32_Q];
+    const uint64_t u0 = plan.first(blockIdx.x), u1 = plan.first(blockIdx.x + 1);
+    for (uint64_t unit = u0; unit < u1;) {
+        const uint64_t item = unit / plan.per, half = item % HALVES;
+        const uint64_t stop = (item + 1) * plan.per < u1 ? (item + 1) * plan.per : u1;  // this block's part of it
+        const uint64_t lq0 = item / HALVES * F32_QUERIES + t;
+        float q[F32_Q][DP], thr[F32_Q];
+        uint32_t cnt[F32_Q];
 #pragma unroll
-    for (int u = 0; u < F32_Q; ++u) {
-        const uint64_t lq = lq0 + u * F32_THREADS;
+        for (int u = 0; u < F32_Q; ++u) {
+            const uint64_t lq = lq0 + u * F32_THREADS;
 #pragma unroll
-        for (int j = 0; j < DP; ++j) q[u][j] = (lq < nq && (uint32_t)j < d) ? X[(q0 + lq) * d + j] : 0.0f;
-        thr[u] = lq < nq ? INFINITY : -INFINITY;
-        cnt[u] = 0;
-    }
-    // this half's points, whole tiles
-    const uint64_t tiles = (n + F32_TILE - 1) / F32_TILE, mid = (tiles + 1) / 2 * F32_TILE;
-    const uint64_t p0 = blockIdx.y ? mid : 0, p1 = blockIdx.y ? n : (mid < n ? mid : n);
-    for (uint64_t base = p0; base < p1; base += F32_TILE) {
-        __syncthreads();  // the previous tile is no longer read
-        for (uint32_t e = t; e < (uint32_t)(F32_TILE * DP); e += F32_THREADS) {
-            const uint32_t p = e / DP, j = e % DP;
-            tile[e] = (base + p < p1 && j < d) ? X[(base + p) * d + j] : 0.0f;
+            for (int j = 0; j < DP; ++j) q[u][j] = (lq < nq && (uint32_t)j < d) ? X[(q0 + lq) * d + j] : 0.0f;
+            thr[u] = lq < nq ? INFINITY : -INFINITY;
+            cnt[u] = 0;
         }
-        __syncthreads();
-        const uint32_t points = (p1 - base < (uint64_t)F32_TILE) ? (uint32_t)(p1 - base) : (uint32_t)F32_TILE;
-        for (uint32_t g = 0; g < points; g += F32_GROUP) {
-#pragma unroll
-            for (int u = 0; u < F32_Q; ++u) {
-                if (__any_sync(0xFFFFFFFFu, cnt[u] > F32_SLOTS - F32_GROUP)) {
-                    thr[u] = f32_cut(cs + u * F32_THREADS, ci + u * F32_THREADS, cnt[u], thr[u]);
-                    cnt[u] = cnt[u] < (uint32_t)RCAND ? cnt[u] : (uint32_t)RCAND;
-                }
+        // the points of the item's tiles [unit, stop)
+        const uint64_t h0 = half * plan.per;  // the half's first tile
+        const uint64_t p0 = (h0 + unit % plan.per) * F32_TILE;
+        const uint64_t p1 = min(n, (h0 + (stop - 1) % plan.per + 1) * F32_TILE);
+        for (uint64_t base = p0; base < p1; base += F32_TILE) {
+            __syncthreads();  // the previous tile is no longer read
+            for (uint32_t e = t; e < (uint32_t)(F32_TILE * DP); e += F32_THREADS) {
+                const uint32_t p = e / DP, j = e % DP;
+                tile[e] = (base + p < p1 && j < d) ? X[(base + p) * d + j] : 0.0f;
             }
-            // rows past the last point are zeros in the tile: computed, not taken
-            float acc[F32_GROUP][F32_Q];
-#pragma unroll
-            for (int v = 0; v < F32_GROUP; ++v)
-#pragma unroll
-                for (int u = 0; u < F32_Q; ++u) acc[v][u] = 0.0f;
-            const float4* c4 = (const float4*)(tile + g * DP);
-#pragma unroll
-            for (int j4 = 0; j4 < DP / 4; ++j4) {
-#pragma unroll
-                for (int v = 0; v < F32_GROUP; ++v) {
-                    const float4 c = c4[v * (DP / 4) + j4];
-#pragma unroll
-                    for (int u = 0; u < F32_Q; ++u) {
-                        float df = __fsub_rn(q[u][4 * j4], c.x);
-                        acc[v][u] = __fmaf_rn(df, df, acc[v][u]);
-                        df = __fsub_rn(q[u][4 * j4 + 1], c.y);
-                        acc[v][u] = __fmaf_rn(df, df, acc[v][u]);
-                        df = __fsub_rn(q[u][4 * j4 + 2], c.z);
-                        acc[v][u] = __fmaf_rn(df, df, acc[v][u]);
-                        df = __fsub_rn(q[u][4 * j4 + 3], c.w);
-                        acc[v][u] = __fmaf_rn(df, df, acc[v][u]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int v = 0; v < F32_GROUP; ++v) {
+            __syncthreads();
+            const uint32_t points = (p1 - base < (uint64_t)F32_TILE) ? (uint32_t)(p1 - base) : (uint32_t)F32_TILE;
+            for (uint32_t g = 0; g < points; g += F32_GROUP) {
 #pragma unroll
                 for (int u = 0; u < F32_Q; ++u) {
-                    if (acc[v][u] < thr[u] && g + v < points) {
-                        cs[cnt[u] * F32_QUERIES + u * F32_THREADS] = acc[v][u];
-                        ci[cnt[u] * F32_QUERIES + u * F32_THREADS] = (uint32_t)(base + g + v);
-                        ++cnt[u];
+                    if (__any_sync(0xFFFFFFFFu, cnt[u] > F32_SLOTS - F32_GROUP)) {
+                        thr[u] = f32_cut(cs + u * F32_THREADS, ci + u * F32_THREADS, cnt[u], thr[u]);
+                        cnt[u] = cnt[u] < (uint32_t)RCAND ? cnt[u] : (uint32_t)RCAND;
+                    }
+                }
+                // rows past the last point are zeros in the tile: computed, not taken
+                float acc[F32_GROUP][F32_Q];
+#pragma unroll
+                for (int v = 0; v < F32_GROUP; ++v)
+#pragma unroll
+                    for (int u = 0; u < F32_Q; ++u) acc[v][u] = 0.0f;
+                const float4* c4 = (const float4*)(tile + g * DP);
+#pragma unroll
+                for (int j4 = 0; j4 < DP / 4; ++j4) {
+#pragma unroll
+                    for (int v = 0; v < F32_GROUP; ++v) {
+                        const float4 c = c4[v * (DP / 4) + j4];
+#pragma unroll
+                        for (int u = 0; u < F32_Q; ++u) {
+                            float df = __fsub_rn(q[u][4 * j4], c.x);
+                            acc[v][u] = __fmaf_rn(df, df, acc[v][u]);
+                            df = __fsub_rn(q[u][4 * j4 + 1], c.y);
+                            acc[v][u] = __fmaf_rn(df, df, acc[v][u]);
+                            df = __fsub_rn(q[u][4 * j4 + 2], c.z);
+                            acc[v][u] = __fmaf_rn(df, df, acc[v][u]);
+                            df = __fsub_rn(q[u][4 * j4 + 3], c.w);
+                            acc[v][u] = __fmaf_rn(df, df, acc[v][u]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int v = 0; v < F32_GROUP; ++v) {
+#pragma unroll
+                    for (int u = 0; u < F32_Q; ++u) {
+                        if (acc[v][u] < thr[u] && g + v < points) {
+                            cs[cnt[u] * F32_QUERIES + u * F32_THREADS] = acc[v][u];
+                            ci[cnt[u] * F32_QUERIES + u * F32_THREADS] = (uint32_t)(base + g + v);
+                            ++cnt[u];
+                        }
                     }
                 }
             }
         }
-    }
+        const bool whole = unit == item * plan.per && stop == (item + 1) * plan.per;
+        unsigned long long* part = shared_lists + (2 * (uint64_t)blockIdx.x + (unit == u0 ? 0 : 1)) * F32_QUERIES * RCAND;
 #pragma unroll
-    for (int u = 0; u < F32_Q; ++u) {
-        const uint64_t lq = lq0 + u * F32_THREADS;
-        f32_cut(cs + u * F32_THREADS, ci + u * F32_THREADS, cnt[u], thr[u]);
+        for (int u = 0; u < F32_Q; ++u) {
+            const uint64_t lq = lq0 + u * F32_THREADS;
+            f32_cut(cs + u * F32_THREADS, ci + u * F32_THREADS, cnt[u], thr[u]);
+            if (lq >= nq) continue;
+            const uint32_t kept = cnt[u] < (uint32_t)RCAND ? cnt[u] : (uint32_t)RCAND;
+            if (whole) {
+                uint32_t* out = cand_idx + lq * RTOTAL + half * RCAND;
+                for (uint32_t s2 = 0; s2 < (uint32_t)RCAND; ++s2)
+                    out[s2] = s2 < kept ? ci[s2 * F32_QUERIES + u * F32_THREADS] : 0xFFFFFFFFu;
+            } else {
+                unsigned long long* out = part + (uint64_t)(t + u * F32_THREADS) * RCAND;
+                for (uint32_t s2 = 0; s2 < (uint32_t)RCAND; ++s2) {
+                    const uint32_t at = s2 * F32_QUERIES + u * F32_THREADS;
+                    out[s2] = s2 < kept ? (unsigned long long)__float_as_uint(cs[at]) << 32 | ci[at] : ~0ull;
+                }
+            }
+        }
+        unit = stop;
+    }
+}
+
+// The RCAND best of every item that several blocks shared, a warp per query: the
+// list so far ascending, the next one descending, the smaller of each pair are
+// the best of both. A key is the distance's bits over the id.
+__device__ __forceinline__ unsigned long long warp_sort_keys(unsigned long long v, bool descending) {
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+    for (uint32_t k = 2; k <= 32; k <<= 1)
+#pragma unroll
+        for (uint32_t j = k >> 1; j; j >>= 1) {
+            const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, v, j);
+            const bool up = ((lane & k) == 0) != descending;
+            v = up == ((lane & j) == 0) ? (o < v ? o : v) : (o < v ? v : o);
+        }
+    return v;
+}
+
+__global__ void k_f32_merge(uint64_t nq, uint64_t items, F32Plan plan,
+                            const unsigned long long* __restrict__ shared_lists, uint32_t* __restrict__ cand_idx) {
+    static_assert(RCAND == 32, "a lane per candidate");
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t i = warp; i < items * F32_QUERIES; i += nwarps) {  // warp-uniform
+        const uint64_t item = i / F32_QUERIES, ql = i % F32_QUERIES, lq = item / HALVES * F32_QUERIES + ql;
         if (lq >= nq) continue;
-        const uint32_t kept = cnt[u] < (uint32_t)RCAND ? cnt[u] : (uint32_t)RCAND;
-        uint32_t* out = cand_idx + lq * RTOTAL + blockIdx.y * RCAND;
-        for (uint32_t s2 = 0; s2 < (uint32_t)RCAND; ++s2)
-            out[s2] = s2 < kept ? ci[s2 * F32_QUERIES + u * F32_THREADS] : 0xFFFFFFFFu;
+        const uint64_t b0 = plan.block_of(item * plan.per), b1 = plan.block_of((item + 1) * plan.per - 1);
+        if (b0 == b1) continue;  // written by its block
+        unsigned long long best = ~0ull;
+        for (uint64_t b = b0; b <= b1; ++b) {
+            const uint64_t slot = 2 * b + (plan.first(b) / plan.per == item ? 0 : 1);
+            const unsigned long long v =
+                warp_sort_keys(shared_lists[(slot * F32_QUERIES + ql) * RCAND + lane], b > b0);
+            best = b == b0 ? v : warp_sort_keys(v < best ? v : best, false);
+        }
+        cand_idx[lq * RTOTAL + item % HALVES * RCAND + lane] = best == ~0ull ? 0xFFFFFFFFu : (uint32_t)best;
     }
 }
 
@@ -1036,10 +1115,19 @@ template <int DP>
 void candidates_fp32_dp(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint64_t q0, uint64_t nq, uint32_t* cand_idx) {
     const size_t sm = (size_t)F32_TILE * DP * 4 + (size_t)F32_SLOTS * F32_QUERIES * 8;
     SC_CUDA(cudaFuncSetAttribute(k_knn_fp32<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    const uint64_t blocks = (nq + F32_QUERIES - 1) / F32_QUERIES;
-    k_knn_fp32<DP><<<dim3((unsigned)blocks, HALVES), F32_THREADS, sm, c.stream>>>(dX, n, d, q0, nq, cand_idx);
+    int resident = 0;
+    SC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_knn_fp32<DP>, F32_THREADS, sm));
+    const uint64_t items = (nq + F32_QUERIES - 1) / F32_QUERIES * HALVES;
+    F32Plan plan;
+    plan.per = ((n + F32_TILE - 1) / F32_TILE + HALVES - 1) / HALVES;  // tiles of a half
+    plan.units = items * plan.per;
+    plan.blocks = (uint32_t)std::min<uint64_t>(plan.units, (uint64_t)c.sm_count * std::max(resident, 1));
+    if (!plan.units) return;
+    DBuf<unsigned long long> lists(c, (uint64_t)plan.blocks * 2 * F32_QUERIES * RCAND);
+    k_knn_fp32<DP><<<plan.blocks, F32_THREADS, sm, c.stream>>>(dX, n, d, q0, nq, plan, cand_idx, lists.get());
+    k_f32_merge<<<grid_for(items * F32_QUERIES * 32, 256), 256, 0, c.stream>>>(nq, items, plan, lists.get(), cand_idx);
     SC_LAUNCH_CHECK();
-    c.launches++;
+    c.launches += 2;
 }
 
 // DP = d rounded up to a multiple of 4.

@@ -120,3 +120,17 @@ def test_rows_that_fill_up_are_cut_back(n, d, k):
     b = sc_gpu.knn_gaussian(X, k, precision=sc_gpu.KNN_BF16)
     assert np.array_equal(a.index, b.index)
     assert np.array_equal(a.distances.view(np.uint32), b.distances.view(np.uint32))
+
+
+@pytest.mark.parametrize("n,d,k", [(1000, 30, 10), (9000, 17, 31), (45_000, 4, 8)])
+def test_fp32_items_shared_by_blocks(n, d, k):
+    """The FP32 arm's work items over the blocks: every item in parts, and (the
+    largest) whole items between shared ones, also for a shard of the rows."""
+    X = _points("mixture", n, d, n + d)
+    a = sc_gpu.knn_gaussian(X, k, precision=sc_gpu.KNN_FP32)
+    b = sc_gpu.knn_gaussian(X, k, precision=sc_gpu.KNN_BF16)
+    assert np.array_equal(a.index, b.index)
+    assert np.array_equal(a.distances.view(np.uint32), b.distances.view(np.uint32))
+    lo, hi = n // 3, n // 3 + 300
+    idx, d2 = sc_gpu.knn_search(X, k, lo, hi, precision=sc_gpu.KNN_FP32)
+    assert np.array_equal(idx, a.index[lo:hi])
