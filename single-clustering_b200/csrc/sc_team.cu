@@ -33,7 +33,10 @@ constexpr uint32_t TEAM_CLUSTER = 16;
 // block cost less than the cluster's (64 against 16: 0.74 and 0.78 ms there).
 constexpr uint32_t SOLO_NODES = 64;
 constexpr uint64_t SOLO_ENTRIES = 4096;
-constexpr uint32_t TAIL_NODES_PER_BLOCK = 384;  // active nodes a block, up to which the last sweeps are the team's
+// Active nodes a block, up to which the last sweeps are the team's. With 192 / 384 /
+// 768: CPM at 200k nodes 20.4 / 20.5 / 21.3 ms, 96 uneven graphs 28.2 / 28.4 / 29.4, a
+// sweep of resolutions over 200k nodes 72.4 / 71.9 / 70.9, RB at 4M 106.3 / 106.1 / 106.0.
+constexpr uint32_t TAIL_NODES_PER_BLOCK = 384;
 constexpr uint32_t TEAM_BIG = TEAM_MAX_NODES / 8;  // rows past a warp's table, per block (8 blocks at least, or one of SOLO_NODES)
 constexpr uint32_t GROUPS = 4;  // nodes a block decides side by side (decide_group)
 constexpr uint32_t SLOTS_MAX = 2 * TEAM_MAX_NODES;  // community ids of a level: the partition's and one fresh per node
