@@ -1616,20 +1616,42 @@ __global__ void k_km_assign(const float* __restrict__ X, uint64_t n, uint32_t d,
 }
 
 // Per-cluster coordinate sums in fixed point (x * 2^s rounded; integer adds are
-// associative, so the centroids do not depend on the order) and counts.
-__global__ void k_km_accum(const float* __restrict__ X, uint64_t n, uint32_t d, const uint32_t* __restrict__ assign,
-                           uint32_t K, double scale, unsigned long long* sum, unsigned* cnt) {
+// associative, so the centroids do not depend on the order) and counts. A warp
+// per point, a lane per coordinate, four points' loads in flight: with a point a
+// lane the lanes of one cluster (most of a warp's, with few clusters) added to the
+// same word one after another, 92 us a step for 65,536 x 50 points in 24 clusters;
+// 27 now.
+__global__ void __launch_bounds__(256) k_km_accum(const float* __restrict__ X, uint64_t n, uint32_t d,
+                                                  const uint32_t* __restrict__ assign, uint32_t K, double scale,
+                                                  unsigned long long* sum, unsigned* cnt) {
     extern __shared__ unsigned long long s_sum[];
     unsigned* s_cnt = (unsigned*)(s_sum + K * d);
     for (uint32_t i = threadIdx.x; i < K * d; i += blockDim.x) s_sum[i] = 0;
     for (uint32_t i = threadIdx.x; i < K; i += blockDim.x) s_cnt[i] = 0;
     __syncthreads();
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t c = assign[i];
-        const float* x = X + i * d;
-        for (uint32_t j = 0; j < d; ++j)
-            atomicAdd(s_sum + c * d + j, (unsigned long long)__double2ll_rn((double)x[j] * scale));
-        atomicAdd(s_cnt + c, 1u);
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t i0 = warp; i0 < n; i0 += 4 * nwarps) {  // warp-uniform
+        uint32_t c[4];
+        float x[4][2];  // d <= 62
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const uint64_t i = i0 + t * nwarps;
+            c[t] = i < n ? assign[i] : 0u;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) x[t][h] = i < n && lane + 32 * h < d ? X[i * d + lane + 32 * h] : 0.0f;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            if (i0 + t * nwarps >= n) break;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (lane + 32 * h < d)
+                    atomicAdd(s_sum + c[t] * d + lane + 32 * h,
+                              (unsigned long long)__double2ll_rn((double)x[t][h] * scale));
+            if (lane == 0) atomicAdd(s_cnt + c[t], 1u);
+        }
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < K * d; i += blockDim.x)
@@ -2456,7 +2478,7 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
             Xsub.get(), ns, d, cent.get(), K, assign.get());
         zero(c, sums.get(), (uint64_t)K * d);
         zero(c, cnt.get(), K);
-        k_km_accum<<<grid_for(ns, 256, (unsigned)c.sm_count), 256, sm_accum, c.stream>>>(
+        k_km_accum<<<grid_for(ns * 32, 256, (unsigned)c.sm_count), 256, sm_accum, c.stream>>>(
             Xsub.get(), ns, d, assign.get(), K, scale, sums.get(), cnt.get());
         k_km_update<<<grid_for((uint64_t)K * d, 256), 256, 0, c.stream>>>(sums.get(), cnt.get(), K, d, inv_scale,
                                                                          cent.get());
