@@ -130,7 +130,8 @@ __global__ void __launch_bounds__(TB, 4) k_decide_small(Params p, const uint32_t
         }
         const double k = from_fix(kf, p.scale), a = from_fix(af, p.nscale);
         if (!REFINE) try_fresh = try_fresh && (!p.has_limit || a <= p.limit);
-        const unsigned mm = valid ? peers_of(cu, valid) & gmask : peers_of(cu, valid);
+        // an invalid lane's peers are itself, a lane of its own group
+        const unsigned mm = peers_of(cu, valid) & gmask;
         const bool leader = valid && (__ffs(mm) - 1 == lane);
         const long long acc = peer_sum(mm, valid ? to_fix((double)wt, p.inv_scale) : 0ll);
         // weight to the own community
