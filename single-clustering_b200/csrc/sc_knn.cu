@@ -837,6 +837,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
                         groups |= (__any_sync(0xFFFFFFFFu, m[j8] < thr) ? 1u : 0u) << j8;
 #pragma unroll 1
                     while (groups) {
+                        __syncwarp();  // the lanes part below, at their stores and in cand_cut
                         const uint32_t j8 = (uint32_t)__ffs(groups) - 1;
                         groups &= groups - 1;
                         float x[8];

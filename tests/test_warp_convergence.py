@@ -4,6 +4,10 @@ A function that holds a full-mask warp intrinsic (peers_of: a match and a
 ballot) is one call that all lanes make together: in an arm of a conditional
 expression, or behind && or ||, the lanes stand at different call sites and the
 result depends on whether the compiler merges them.
+
+A load from tensor memory (tmem_ld8, tmem_ld64: tcgen05.ld.sync.aligned) needs
+its warp converged: in the block of code that makes it, a warp-wide operation
+stands in front of it, whatever the lanes did in the round before.
 """
 import os
 import re
@@ -50,3 +54,41 @@ def test_the_check_sees_a_call_in_an_arm():
     assert _per_lane_calls("{ if (a(b) && __match_any_sync(F, c)) x(); }")
     assert not _per_lane_calls("{ m = peers_of(c, x ? 1 : 0); n = ok ? m : 0; }")
     assert not _per_lane_calls("{ const unsigned same = __match_any_sync(F, key); }")
+
+
+def _block_before(src, at):
+    """The text of the innermost block around src[at] up to there, without the blocks closed in it."""
+    depth, i, text = 0, at - 1, []
+    while i >= 0:
+        c = src[i]
+        if c == "}":
+            depth += 1
+        elif c == "{":
+            if depth == 0:
+                return "".join(reversed(text))
+            depth -= 1
+        elif depth == 0:
+            text.append(c)
+        i -= 1
+    return "".join(reversed(text))
+
+
+def _unconverged_loads(src):
+    found = []
+    for m in re.finditer(r"\btmem_ld(?:8|64)\s*\(", src):
+        if re.search(r"\bvoid\s+$", src[:m.start()]):
+            continue  # its definition
+        if not re.search(r"__syncwarp\s*\(|__(?:all|any|ballot)_sync\s*\(", _block_before(src, m.start())):
+            found.append(src.count("\n", 0, m.start()) + 1)
+    return found
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_tensor_memory_loads_follow_a_warp_wide_operation(name):
+    assert _unconverged_loads(_code(name)) == []
+
+
+def test_the_check_sees_a_load_behind_predicated_stores():
+    assert _unconverged_loads("{ __syncwarp(); while (g) { float x[8]; tmem_ld8(a, x); if (x[0] < t) s[0] = x[0]; } }")
+    assert not _unconverged_loads("{ while (g) { __syncwarp(); tmem_ld8(a, x); } }")
+    assert not _unconverged_loads("{ if (!__all_sync(F, w(b))) { break; } tmem_ld64(a, r); }")
