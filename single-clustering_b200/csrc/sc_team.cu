@@ -141,6 +141,7 @@ struct Team {
         if (size == 1) {
             __syncthreads();
         } else {
+            __syncwarp();  // the barrier takes a warp's arrival as one: its lanes come together first
             asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         }
@@ -424,7 +425,10 @@ __device__ uint32_t decide_warp(const Params& p, uint32_t v, uint64_t b, uint32_
 struct Group {
     uint32_t id, threads;  // named barrier 1 + id; threads of the group
     __device__ uint32_t tid() const { return threadIdx.x % threads; }
-    __device__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(1 + id), "r"(threads) : "memory"); }
+    __device__ void sync() const {
+        __syncwarp();  // as in Team::sync
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + id), "r"(threads) : "memory");
+    }
 };
 constexpr uint32_t GROUP_BYTES = SLOTS_MAX / GROUPS * sizeof(long long);
 constexpr uint32_t GROUP_DEGREE = 1024;  // longest row of a quarter's table, and of the block's

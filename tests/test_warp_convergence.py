@@ -7,7 +7,9 @@ result depends on whether the compiler merges them.
 
 A load from tensor memory (tmem_ld8, tmem_ld64: tcgen05.ld.sync.aligned) needs
 its warp converged: in the block of code that makes it, a warp-wide operation
-stands in front of it, whatever the lanes did in the round before.
+stands in front of it, whatever the lanes did in the round before. A barrier
+written as PTX (bar.sync, barrier.cluster.arrive / wait with .aligned) needs the
+same.
 """
 import os
 import re
@@ -92,3 +94,16 @@ def test_the_check_sees_a_load_behind_predicated_stores():
     assert _unconverged_loads("{ __syncwarp(); while (g) { float x[8]; tmem_ld8(a, x); if (x[0] < t) s[0] = x[0]; } }")
     assert not _unconverged_loads("{ while (g) { __syncwarp(); tmem_ld8(a, x); } }")
     assert not _unconverged_loads("{ if (!__all_sync(F, w(b))) { break; } tmem_ld64(a, r); }")
+
+
+def _unconverged_barriers(src):
+    found = []
+    for m in re.finditer(r'asm\s+volatile\s*\(\s*"(bar\.sync|barrier\.cluster\.arrive[^"]*\.aligned)', src):
+        if not re.search(r"__syncwarp\s*\(", _block_before(src, m.start())):
+            found.append(m.group(1))
+    return found
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_aligned_barriers_follow_a_warp_barrier(name):
+    assert _unconverged_barriers(_code(name)) == []
