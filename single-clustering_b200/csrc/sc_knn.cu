@@ -768,7 +768,7 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
         constexpr uint32_t S = SLOT_STRIDE;
         uint32_t b = 0, b_parity = 0;  // the accumulator buffer in turn
         uint32_t gi = 0;
-        for (uint32_t g; (g = group_at(gi)) < ngroups && !*abort_flag; ++gi) {
+        for (uint32_t g; (g = group_at(gi)) < ngroups && !__any_sync(0xFFFFFFFFu, *abort_flag != 0); ++gi) {
             const uint64_t qrow = (uint64_t)g * QT * TILE + q * TILE + row;
             const float capv = (!BOUND && qcap && qrow < nq) ? qcap[qrow] : INFINITY;
             float thr = qrow < nq ? capv : -INFINITY;  // rows past the last query take nothing

@@ -10,6 +10,10 @@ its warp converged: in the block of code that makes it, a warp-wide operation
 stands in front of it, whatever the lanes did in the round before. A barrier
 written as PTX (bar.sync, barrier.cluster.arrive / wait with .aligned) needs the
 same.
+
+The flag that ends the kNN scan early is read by a whole warp (__any_sync) where
+its lanes go on to warp-wide operations: lanes that read it one by one could part
+there, and some would wait for the others.
 """
 import os
 import re
@@ -107,3 +111,13 @@ def _unconverged_barriers(src):
 @pytest.mark.parametrize("name", FILES)
 def test_aligned_barriers_follow_a_warp_barrier(name):
     assert _unconverged_barriers(_code(name)) == []
+
+
+def test_the_scan_stops_by_the_warp():
+    src = _code("sc_knn.cu")
+    kernel = src[src.index("k_knn_tc(const __grid_constant__"):]
+    kernel = kernel[kernel.index("if (warp == 1)"):]  # behind the producer, which is one lane
+    kernel = kernel[:kernel.index("__syncthreads()")]
+    reads = [m.start() for m in re.finditer(r"\*abort_flag(?!\s*=[^=])", kernel)]
+    assert reads
+    assert all(kernel[:at].endswith("__any_sync(0xFFFFFFFFu, ") for at in reads)
