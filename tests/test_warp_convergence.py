@@ -116,7 +116,7 @@ def test_aligned_barriers_follow_a_warp_barrier(name):
 def test_the_scan_stops_by_the_warp():
     src = _code("sc_knn.cu")
     kernel = src[src.index("k_knn_tc(const __grid_constant__"):]
-    kernel = kernel[kernel.index("if (warp == 1)"):]  # behind the producer, which is one lane
+    kernel = kernel[kernel.index("else if (warp == 1)"):]  # behind the producer, which is one lane
     kernel = kernel[:kernel.index("__syncthreads()")]
     reads = [m.start() for m in re.finditer(r"\*abort_flag(?!\s*=[^=])", kernel)]
     assert reads
