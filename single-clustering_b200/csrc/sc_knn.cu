@@ -211,8 +211,8 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 
 // A (query, half)'s candidates: CAND_SLOTS slots of shared memory, filled in
 // order; when a row of the warp has no room for the next, all rows are cut back
-// to their RCAND best together. Every lane of the warp calls it. A row of `cnt` keeps
-// min(cnt, RCAND), in the first slots. Returns the score
+// to their RCAND best together, equal ones by their order. Every lane of the warp
+// calls it. A row of `cnt` keeps min(cnt, RCAND), in the first slots. Returns the score
 // from which on nothing is a candidate any more: the worst kept of a full row,
 // else cap. Near tiles bring a row's candidates in a burst, 95 a query at
 // 1M x 50; a search for the worst of a full row at each of them (a call for one
@@ -246,15 +246,23 @@ __device__ __noinline__ float cand_cut(float* cs, uint32_t* ci, uint32_t owner, 
             worst = top[i];
         }
     if (drop) {
+        // of the entries that equal the worst kept the first ones stay: slots fill
+        // in the order of the points, and ties go to the lower index
+        uint32_t room = 0xFFFFFFFFu;
+        if (ties) {
+            room = 0;
+            for (uint32_t s = 0; s < cnt; ++s) room += cs[s * SLOT_STRIDE + owner] == worst ? 1u : 0u;
+            room -= ties;
+        }
         uint32_t w = owner;
 #pragma unroll 4
         for (uint32_t s = 0; s < cnt; ++s) {
             const float v = cs[s * SLOT_STRIDE + owner];
             const uint32_t id = ci[s * SLOT_STRIDE + owner];
             bool keep = v <= worst;
-            if (v == worst && ties) {  // as many of the equal ones as do not fit
-                keep = false;
-                --ties;
+            if (v == worst) {
+                keep = room > 0;
+                room -= keep ? 1u : 0u;
             }
             if (keep) {
                 cs[w] = v;
@@ -930,15 +938,17 @@ constexpr int F32_TILE = 32;
 constexpr int F32_SLOTS = 44;
 constexpr int F32_GROUP = 4;  // points taken together: eight independent sums a thread
 
-// Cuts a row of `cnt` candidates to its RCAND best (the last one takes the worst
-// one's slot until RCAND are left); returns the worst kept, or thr with fewer.
+// Cuts a row of `cnt` candidates to its RCAND best by (distance, id): the last one
+// takes the worst one's slot until RCAND are left. Returns the worst distance kept,
+// or thr with fewer.
 __device__ __noinline__ float f32_cut(float* cs, uint32_t* ci, uint32_t cnt, float thr) {
     while (cnt >= (uint32_t)RCAND) {
         float worst = -INFINITY;
-        uint32_t at = 0;
+        uint32_t at = 0, last = 0;  // the first and the last slot that hold the worst
 #pragma unroll 8
         for (uint32_t s = 0; s < cnt; ++s) {
             const float x = cs[s * F32_QUERIES];
+            if (x >= worst) last = s;
             if (x > worst) {
                 worst = x;
                 at = s;
@@ -946,6 +956,9 @@ __device__ __noinline__ float f32_cut(float* cs, uint32_t* ci, uint32_t cnt, flo
         }
         thr = worst;
         if (cnt == (uint32_t)RCAND) break;
+        if (at != last)  // equal ones: the highest id goes
+            for (uint32_t s = at + 1; s <= last; ++s)
+                if (cs[s * F32_QUERIES] == worst && ci[s * F32_QUERIES] > ci[at * F32_QUERIES]) at = s;
         --cnt;
         cs[at * F32_QUERIES] = cs[cnt * F32_QUERIES];
         ci[at * F32_QUERIES] = ci[cnt * F32_QUERIES];
