@@ -1182,9 +1182,30 @@ __device__ __forceinline__ uint64_t warp_sort32(uint64_t key) {
     return key;
 }
 
-// One warp per query: exact FP32 distances of its RTOTAL = 64 candidates (two
-// per lane), the 32 smallest kept by a merge-split of two sorted halves, then
-// the first k+1 written.
+// A query's list from its 64 candidates a, b (two per lane): their keys (key(id)),
+// the 32 smallest kept by a merge-split of two sorted halves, ascending over the
+// lanes. A row of more equal points than the candidates hold may lack the query
+// itself: it comes first all the same, unless a coordinate is not finite (its
+// distance to itself is then none).
+template <class Key>
+__device__ __forceinline__ uint64_t rerank_list(uint32_t a, uint32_t b, uint32_t self, Key key) {
+    const unsigned FULL = 0xFFFFFFFFu, lane = threadIdx.x & 31u;
+    const uint64_t ka = warp_sort32(key(a)), kb = warp_sort32(key(b));
+    const uint64_t kbr = __shfl_sync(FULL, kb, 31 - lane);
+    uint64_t k = ka < kbr ? ka : kbr;  // the 32 smallest, as a bitonic sequence
+    for (int stride = 16; stride > 0; stride >>= 1) {
+        const uint64_t other = __shfl_xor_sync(FULL, k, stride);
+        k = (lane & stride) == 0 ? (k < other ? k : other) : (k < other ? other : k);
+    }
+    if (!__any_sync(FULL, a == self || b == self) && key(self) == 0) {  // warp-uniform
+        const uint64_t before = __shfl_up_sync(FULL, k, 1);
+        k = lane ? before : 0;
+    }
+    return k;
+}
+
+// One warp per query: exact FP32 distances of its RTOTAL = 64 candidates, the
+// first k+1 written.
 // Queries are points q0 .. q0 + nq - 1; rows of cand_idx / out_* are local.
 __global__ void k_knn_rerank(const float* __restrict__ X, uint64_t n, uint32_t d, uint32_t k, uint64_t q0,
                              uint64_t nq, const uint32_t* __restrict__ cand_idx, uint32_t* __restrict__ out_idx,
@@ -1194,14 +1215,9 @@ __global__ void k_knn_rerank(const float* __restrict__ X, uint64_t n, uint32_t d
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t lq = warp; lq < nq; lq += nwarps) {
         const uint64_t q = q0 + lq;
-        uint64_t ka = warp_sort32(rerank_key(X, n, d, q, cand_idx[lq * RTOTAL + lane]));
-        uint64_t kb = warp_sort32(rerank_key(X, n, d, q, cand_idx[lq * RTOTAL + 32 + lane]));
-        const uint64_t kbr = __shfl_sync(0xFFFFFFFFu, kb, 31 - lane);
-        uint64_t key = ka < kbr ? ka : kbr;  // the 32 smallest, as a bitonic sequence
-        for (int stride = 16; stride > 0; stride >>= 1) {
-            const uint64_t other = __shfl_xor_sync(0xFFFFFFFFu, key, stride);
-            key = (lane & stride) == 0 ? (key < other ? key : other) : (key < other ? other : key);
-        }
+        const uint32_t* cand = cand_idx + lq * RTOTAL;
+        const uint64_t key = rerank_list(cand[lane], cand[32 + lane], (uint32_t)q,
+                                         [&](uint32_t j) { return rerank_key(X, n, d, q, j); });
         if (lane <= k) {
             const uint32_t tag = (uint32_t)key;
             const uint32_t idx = (key == ~0ull) ? 0xFFFFFFFFu : (tag == 0 ? (uint32_t)q : tag - 1u);
@@ -2375,14 +2391,8 @@ __global__ void k_knn_rerank_sorted(const float* __restrict__ Xs, uint64_t n, ui
             const uint32_t j = perm[js];
             return ((uint64_t)__float_as_uint(acc) << 32) | (j == q ? 0u : j + 1u);
         };
-        uint64_t ka = warp_sort32(key(cand_idx[r * RTOTAL + lane]));
-        uint64_t kb = warp_sort32(key(cand_idx[r * RTOTAL + 32 + lane]));
-        const uint64_t kbr = __shfl_sync(0xFFFFFFFFu, kb, 31 - lane);
-        uint64_t kk = ka < kbr ? ka : kbr;  // the 32 smallest, as a bitonic sequence
-        for (int stride = 16; stride > 0; stride >>= 1) {
-            const uint64_t other = __shfl_xor_sync(0xFFFFFFFFu, kk, stride);
-            kk = (lane & stride) == 0 ? (kk < other ? kk : other) : (kk < other ? other : kk);
-        }
+        const uint32_t* cand = cand_idx + r * RTOTAL;
+        const uint64_t kk = rerank_list(cand[lane], cand[32 + lane], (uint32_t)sq, key);
         if (lane <= k) {
             const uint32_t tag = (uint32_t)kk;
             const uint32_t idx = (kk == ~0ull) ? 0xFFFFFFFFu : (tag == 0 ? q : tag - 1u);

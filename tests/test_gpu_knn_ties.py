@@ -88,3 +88,50 @@ def test_equal_points_of_a_pruned_size(arm):
         assert sc_gpu.knn_last_stats()["clusters"] >= 16
     for i, row in zip(at, index):
         assert np.array_equal(row, np.concatenate([[i], at[at != i]])[:k + 1])
+
+
+@pytest.mark.parametrize("arm", ARMS)
+@pytest.mark.parametrize("k", [10, 24, 31])
+@pytest.mark.parametrize("kind,n,copies", [("first", 600, 50), ("first", 600, 200), ("wide", 600, 120),
+                                           ("scattered", 3000, 200), ("lattice", 2000, 0)])
+def test_every_point_heads_its_own_list(kind, n, copies, k, arm):
+    """Also a point with more equals of lower index than a row keeps candidates."""
+    X = _points(kind, n, copies, n + copies)
+    assert (_copies_before(X) >= KEPT).any()
+    index, dist = _expected(X, k)
+    r = sc_gpu.knn_gaussian(X, k, precision=arm)
+    rows = np.ones(n, bool)
+    if kind == "wide" and arm == sc_gpu.KNN_BF16:
+        rows[-1] = False  # as above
+    assert np.array_equal(r.index[:, 0], np.arange(n))
+    assert np.array_equal(r.index[rows], index[rows]) and np.array_equal(r.distances[rows], dist[rows])
+
+
+def test_every_point_heads_its_own_list_when_pruned():
+    n, k = 70_000, 15
+    X = np.random.Generator(np.random.PCG64(4)).normal(size=(n, 12)).astype(np.float32)
+    at = np.sort(np.random.Generator(np.random.PCG64(5)).permutation(n)[:200])
+    X[at] = X[at[0]]
+    r = sc_gpu.knn_gaussian(X, k)
+    assert sc_gpu.knn_last_stats()["clusters"] >= 16
+    assert np.array_equal(r.index[:, 0], np.arange(n))
+    for i in at:
+        assert np.array_equal(r.index[i], np.concatenate([[i], at[at != i]])[:k + 1])
+        assert not r.distances[i].any()
+
+
+@pytest.mark.parametrize("arm", ARMS)
+def test_a_point_that_is_not_finite_has_no_distance_to_itself(arm):
+    X = np.random.Generator(np.random.PCG64(6)).normal(size=(300, 5)).astype(np.float32)
+    X[7, 2], X[8, 0] = np.inf, np.nan
+    r = sc_gpu.knn_gaussian(X, 4, precision=arm)
+    # no distance of theirs is finite, so neither heads its list; the infinite one's
+    # 16-bit scores are -inf where the products are, and such points are listed
+    assert np.all(np.isinf(r.distances[7:9]))
+    assert 7 not in r.index[7] and np.all(r.index[8] == 0xFFFFFFFF)
+    if arm == sc_gpu.KNN_FP32:
+        assert np.all(r.index[7] == 0xFFFFFFFF)
+    else:
+        assert np.array_equal(r.index[7], np.flatnonzero(X[:, 2] > 0)[np.flatnonzero(X[:, 2] > 0) != 7][:5])
+    others = np.delete(np.arange(300), [7, 8])
+    assert np.array_equal(r.index[others, 0], others)
