@@ -165,6 +165,13 @@ sc_status sc_get_wait_limit(const sc_ctx* ctx, uint32_t* out);
  * SC_E_TIMEOUT without any copy or MMA left in flight. Off by default.
  */
 sc_status sc_test_knn_hold_tiles(sc_ctx* ctx, int32_t on);
+/*
+ * Test hook for devices that place fewer blocks in one thread-block cluster: the
+ * kernels that run small levels and the last sweeps of larger ones in one launch
+ * use at most `most` blocks (16, 8, or 0: every step has a launch of its own, as
+ * on a device that places neither). 16 by default. Labels do not depend on it.
+ */
+sc_status sc_test_team_cluster(sc_ctx* ctx, uint32_t most);
 
 /*
  * Autotuner: times the first level of `cfg` (one pass, one level: the level

@@ -9,6 +9,7 @@
 #include <chrono>
 
 #include "sc_prims.cuh"
+#include "sc_team.cuh"
 
 struct sc_ctx {
     sc::Ctx c;
@@ -266,6 +267,13 @@ sc_status sc_knn_last_stats(const sc_ctx* ctx, sc_knn_stats* out) {
 
 sc_status sc_test_knn_hold_tiles(sc_ctx* ctx, int32_t on) {
     return guarded(ctx, [&](sc::Ctx& c) { c.knn_hold_tiles = on ? 1u : 0u; });
+}
+
+sc_status sc_test_team_cluster(sc_ctx* ctx, uint32_t most) {
+    return guarded(ctx, [&](sc::Ctx& c) {
+        if (most != 0 && most != 8 && most != 16) sc::fail(SC_E_INVALID_ARGUMENT, "a team has 16, 8 or 0 blocks, not %u", most);
+        c.team_most = most;
+    });
 }
 
 sc_status sc_autotune(sc_ctx* ctx, const sc_graph* g, const sc_leiden_config* cfg, sc_tuning* chosen,
@@ -578,9 +586,11 @@ sc_status sc_leiden_batch_ex(sc_ctx* ctx, const sc_graph* const* graphs, const s
         uint64_t remaining = count;
         bool failed = false;
         sc_error_info first_err{};
+        const uint32_t team = sc::team_offer(c);
         auto worker = [&]() {
             sc::Ctx w;
             w.staged_downloads = false;
+            w.team_offered = (int32_t)team;
             sc_status st = init_ctx(w, c.device, W <= 8);
             if (st != SC_OK) {
                 std::lock_guard<std::mutex> lk(mu);

@@ -81,6 +81,11 @@ struct Ctx {
     // test hook (sc_test_knn_hold_tiles): the kNN producer issues no point
     // tiles, so the contraction's first wait runs out and the call times out
     uint32_t knn_hold_tiles = 0;
+    // thread-block cluster of the small levels' kernels (sc_team.cu): the blocks
+    // that the device can place in one (16, 8, 0: none; -1: not asked yet), and
+    // the most that may be used (test hook sc_test_team_cluster)
+    int32_t team_offered = -1;
+    uint32_t team_most = 16;
     // kNN point clusters of the pruned search (sc_set_knn_clusters): 0 picks
     // a count from n, 1 scans every tile
     uint32_t knn_clusters = 0;

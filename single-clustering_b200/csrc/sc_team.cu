@@ -1277,31 +1277,62 @@ __global__ void __launch_bounds__(TEAM_THREADS, 1) k_move_tail(const __grid_cons
 }
 
 // A launch of one cluster of `blocks` blocks with the team's shared memory.
+struct TeamLaunch {
+    cudaLaunchConfig_t config{};
+    cudaLaunchAttribute cluster{};
+    template <class K>
+    TeamLaunch(Ctx& c, K kernel, uint32_t blocks) {
+        SC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TeamSmem)));
+        SC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        config.gridDim = dim3(blocks);
+        config.blockDim = dim3(TEAM_THREADS);
+        config.dynamicSmemBytes = sizeof(TeamSmem);
+        config.stream = c.stream;
+        cluster.id = cudaLaunchAttributeClusterDimension;
+        cluster.val.clusterDim.x = blocks;
+        cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+        config.attrs = &cluster;
+        config.numAttrs = 1;
+    }
+    TeamLaunch(const TeamLaunch&) = delete;
+    TeamLaunch& operator=(const TeamLaunch&) = delete;
+};
+
 template <class K, class A>
 void launch_team(Ctx& c, K kernel, uint32_t blocks, const A& args) {
-    SC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TeamSmem)));
-    SC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    cudaLaunchConfig_t lc{};
-    lc.gridDim = dim3(blocks);
-    lc.blockDim = dim3(TEAM_THREADS);
-    lc.dynamicSmemBytes = sizeof(TeamSmem);
-    lc.stream = c.stream;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = blocks;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    lc.attrs = &at;
-    lc.numAttrs = 1;
-    SC_CUDA(cudaLaunchKernelEx(&lc, kernel, args));
+    TeamLaunch l(c, kernel, blocks);
+    SC_CUDA(cudaLaunchKernelEx(&l.config, kernel, args));
     c.launches++;
 }
 
-uint32_t team_blocks(const Ctx& c) { return c.side[0] ? TEAM_CLUSTER : TEAM_CLUSTER / 2; }
+// Half a team beside other instances' work.
+uint32_t team_blocks(Ctx& c) { return c.side[0] ? team_offer(c) : std::min(team_offer(c), TEAM_CLUSTER / 2); }
 
 }  // namespace
 
+// A cluster of 16 blocks, each with most of an SM's shared memory, needs 16 free SMs
+// that the hardware lets share one: more than the 8 every device promises, and not
+// there on every part or partition of a GPU. All of the team's kernels have the
+// same threads and shared memory (and one block an SM), so k_team answers for them.
+uint32_t team_offer(Ctx& c) {
+    if (c.team_offered < 0) {
+        c.team_offered = 0;
+        if (c.smem_optin < sizeof(TeamSmem)) return 0;
+        for (uint32_t blocks = TEAM_CLUSTER; blocks >= TEAM_CLUSTER / 2 && !c.team_offered; blocks /= 2) {
+            TeamLaunch l(c, k_team, blocks);
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, k_team, &l.config) != cudaSuccess) {
+                cudaGetLastError();  // a cluster size that the device does not have
+                clusters = 0;
+            }
+            if (clusters > 0) c.team_offered = (int32_t)blocks;
+        }
+    }
+    return std::min((uint32_t)c.team_offered, c.team_most);
+}
+
 bool team_takes(Ctx& c, const DevGraph& g, const sc_leiden_config& cfg) {
-    return g.n > 0 && g.n <= TEAM_MAX_NODES && g.E <= TEAM_MAX_ENTRIES && !cfg.has_max_community_weight && g.exact_w &&
+    return team_offer(c) && g.n > 0 && g.n <= TEAM_MAX_NODES && g.E <= TEAM_MAX_ENTRIES && !cfg.has_max_community_weight && g.exact_w &&
            g.exact_nw && g.part_max_2m == 0.0 && g.part_max_nw == 0.0 && graph_bitwise_symmetric(c, g);
 }
 
@@ -1408,7 +1439,7 @@ void team_run(Ctx& c, const DevGraph& g, uint32_t* memb, uint64_t C, const sc_le
     out.graph.reset(graph_from_contraction(c, r.n, r.E, b.ptr, b.nbr, b.w, b.node_w));
 }
 
-uint32_t tail_limit(const Ctx& c, const DevGraph& g, const sc_leiden_config& cfg) {
+uint32_t tail_limit(Ctx& c, const DevGraph& g, const sc_leiden_config& cfg) {
     if (cfg.has_max_community_weight || g.max_degree > BLOCK_DEGREE || g.E > 0xFFFFFFFFull) return 0;
     return team_blocks(c) * TAIL_NODES_PER_BLOCK;
 }

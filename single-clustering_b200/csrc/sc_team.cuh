@@ -35,6 +35,10 @@ struct TeamResult {
     uint64_t C = 0;
 };
 
+// Blocks of the largest team that the device can place: 16, 8 or 0 (asked once per
+// context, not above its team_most). With 0 every level goes a launch per step.
+uint32_t team_offer(Ctx& c);
+
 // Whether the team may take g under cfg.
 bool team_takes(Ctx& c, const DevGraph& g, const sc_leiden_config& cfg);
 
@@ -47,7 +51,7 @@ void team_run(Ctx& c, const DevGraph& g, uint32_t* memb, uint64_t C, const sc_le
 // The last sweeps of a larger level's local moving: once a sweep has at most
 // tail_limit active nodes (0: the team cannot take this level), the team runs on
 // until the level is done or a sweep outgrows it.
-uint32_t tail_limit(const Ctx& c, const DevGraph& g, const sc_leiden_config& cfg);
+uint32_t tail_limit(Ctx& c, const DevGraph& g, const sc_leiden_config& cfg);
 struct TailResult {
     bool done = false;
     bool swapped = false;  // not done: the next sweep's list is lists[1], its count counts[1]

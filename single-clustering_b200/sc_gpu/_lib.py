@@ -119,6 +119,7 @@ SIGNATURES = [
     ("sc_set_wait_limit", C.c_int, [vp, C.c_uint32]),
     ("sc_get_wait_limit", C.c_int, [vp, C.POINTER(C.c_uint32)]),
     ("sc_test_knn_hold_tiles", C.c_int, [vp, C.c_int32]),
+    ("sc_test_team_cluster", C.c_int, [vp, C.c_uint32]),
     ("sc_set_knn_clusters", C.c_int, [vp, C.c_uint32]),
     ("sc_knn_last_stats", C.c_int, [vp, C.POINTER(KnnStats)]),
     ("sc_knn_autotune", C.c_int, [vp, f32p, C.c_uint64, C.c_uint64, C.c_uint64, C.POINTER(KnnOpts),
