@@ -1516,19 +1516,23 @@ __global__ void __launch_bounds__(32 * AGG_WARPS, 8)
 // group (G <= AGG_DENSE_GROUPS): any row length, no probing, and the accumulators
 // read back in order need no sort. Members in chunks of the block's size, their
 // degrees' prefix in shared memory; each thread takes entries of the flattened
-// chunk, four gathers in flight. A row of more than AGG_DENSE_PART entries is
+// chunk, four gathers in flight. A row of more than a part (AGG_DENSE_PART) is
 // shared by several blocks, which add their accumulators to the row's slice of a
 // global array (a coarse community of a kNN graph can hold a sixth of all
 // entries: 9.9 ms in one block, 0.34 in parts). Integer fixed point, exact in this
 // regime as in k_contract_smem.
 constexpr uint64_t AGG_DENSE_GROUPS = 12288;  // 96 KB of accumulators: two blocks an SM
 constexpr uint64_t AGG_DENSE_PART = 16384;
+// Bytes of the global array at most. A row is shared only past a part's length, so
+// there are at most E / part such rows of 8 G bytes: graphs with more entries times
+// groups than this allows get longer parts (unbounded, the array reached 1.2 GB).
+constexpr uint64_t AGG_DENSE_SLICES = uint64_t(128) << 20;
 constexpr int AGG_DENSE_THREADS = 512;
 
 // Parts of every dense row: istart[i] = the parts of the rows before it, slot[i] =
 // its slice of the global array (rows of several parts), counts = {parts, slices}.
 __global__ void __launch_bounds__(1024) k_dense_parts(const uint32_t* __restrict__ rows, uint64_t nrows,
-                                                      const uint64_t* __restrict__ cap, uint32_t* istart,
+                                                      const uint64_t* __restrict__ cap, uint64_t part, uint32_t* istart,
                                                       uint32_t* slot, uint32_t* srow, uint64_t* counts) {
     __shared__ unsigned long long s_w[32];
     const unsigned FULL = 0xFFFFFFFFu, lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
@@ -1537,7 +1541,7 @@ __global__ void __launch_bounds__(1024) k_dense_parts(const uint32_t* __restrict
         const uint64_t i = base + threadIdx.x;
         unsigned long long x = 0;
         if (i < nrows) {
-            const uint64_t parts = (cap[rows[i]] + AGG_DENSE_PART - 1) / AGG_DENSE_PART;
+            const uint64_t parts = (cap[rows[i]] + part - 1) / part;
             x = parts > 1 ? parts | (1ull << 32) : 1ull;
         }
         unsigned long long incl = x;
@@ -1999,8 +2003,9 @@ DevGraph* contract_exact(Ctx& c, const DevGraph& g, const uint32_t* d_grp, uint6
         const double scale = std::ldexp(1.0, g.e0_w), inv = std::ldexp(1.0, -g.e0_w);
         DBuf<uint32_t> istart(c, nmid + 1), slot(c, nmid), srow(c, nmid);
         DBuf<uint64_t> pc(c, 2);
-        k_dense_parts<<<1, 1024, 0, c.stream>>>(mrows.get(), nmid, cap.get(), istart.get(), slot.get(), srow.get(),
-                                                pc.get());
+        const uint64_t part = std::max(AGG_DENSE_PART, g.E * G * sizeof(unsigned long long) / AGG_DENSE_SLICES);
+        k_dense_parts<<<1, 1024, 0, c.stream>>>(mrows.get(), nmid, cap.get(), part, istart.get(), slot.get(),
+                                                srow.get(), pc.get());
         SC_LAUNCH_CHECK();
         uint64_t parts[2];
         {
