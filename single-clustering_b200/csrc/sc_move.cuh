@@ -208,10 +208,6 @@ __device__ __forceinline__ bool lost(const Params& p, uint32_t x) {
     return p.has_limit && p.claim[p.tgt[x]] != claim_key<MULTI>(p, x);
 }
 
-__device__ __forceinline__ double uniform01(uint64_t seed, uint64_t a, uint64_t b) {
-    return (double)(hash3(seed ^ 0x5151515151515151ull, a, b) >> 11) * 0x1.0p-53;
-}
-
 // Refinement's randomised choice (refine.rs:110-153) draws candidate c with
 // probability exp(rel_c / theta) / sum. Gumbel-max draws from the same
 // distribution: argmax_c rel_c / theta + G_c with G_c = -log(-log U_c), U_c
