@@ -912,20 +912,20 @@ __global__ void __launch_bounds__(KNN_THREADS, 1)
 // registers; points stream through shared memory in tiles of F32_TILE (every
 // thread reads the same point: broadcast loads).
 //
-// Bound by FP32 issue: 2 DP operations a pair (DP: d rounded up to 4, a register
-// array's size). One query a thread left it bound by the broadcast loads
-// instead (a 16-byte load feeds 8 operations, and holds the SM's one load
-// pipe as long as these take): 8.7 ms at 30,011 x 50, 6.3 with two queries
-// (and two or four points at a time). The work
+// Bound by instruction issue with two warps a scheduler: 2 DP operations a pair (DP:
+// d rounded up to 4, a register array's size), and the candidate slots leave room
+// for four blocks of two warps an SM. At 30,011 x 50 the issue slots are 62% busy,
+// the FMA pipe 45%, the shared-memory pipe 29%; between issues a warp waits for
+// its own last operation or a broadcast load. One query a thread, which halves the
+// operations a 16-byte load feeds, took 8.7 ms there, two (and two or four points
+// at a time) take 6.3. The work
 // items (F32_QUERIES queries x a half of the points, the half's RCAND best in its
 // half of the candidate slots) are cut into equal runs of point tiles, one run a
 // resident block, so that a few items fill the chip too: a block per item took
 // 275 us at 1,000 x 30 points, 780 at 5,003 x 30 and 57.3 ms at 100,000 x 50, the
-// runs take 47, 500 and 53.8; at 30,011 x 50 both take 6.3 ms, bound by the load
-// pipe: a 16-byte load feeds 16 operations of a warp and four warps share the
-// pipe. More queries a thread would need more slots than shared memory holds. An
-// item that several blocks share goes through their lists in scratch
-// (k_f32_merge).
+// runs take 47, 500 and 53.8; at 30,011 x 50 both take 6.3 ms. More queries a thread
+// or more warps would need more slots than shared memory holds. An item that
+// several blocks share goes through their lists in scratch (k_f32_merge).
 //
 // A candidate is two predicated stores into the query's F32_SLOTS
 // slots; when a row of the warp is nearly full, all rows are cut back to their
