@@ -2813,10 +2813,11 @@ void knn_search_pruned(Ctx& c, const float* dX, uint64_t n, uint32_t d, uint32_t
 
 // Exact (brute-force) k+1 nearest points of the queries q0 .. q0 + nq - 1
 // among all n points of the device array dX: 64 candidates per query (the 32
-// best of each half of the candidate columns) from the BF16 or FP8 tensor-core
-// scores, or the 32 best exact FP32 distances of either half of the points from the CUDA cores, ranked
-// exactly in FP32. idx/d2 are nq x (k+1), self first, then ascending squared
-// distance, ties by lower index.
+// best of each half of the candidate columns) from the 16-bit or FP8 tensor-core
+// scores, or the 32 best exact FP32 distances of either half of the points from
+// the CUDA cores, ranked exactly in FP32. idx/d2 are nq x (k+1), self first, then
+// ascending squared distance, ties by lower index (of equal candidates that a row
+// has no room for, those of lower index stay).
 void knn_search_device(Ctx& c, const float* dX, uint64_t n, uint64_t d, uint64_t k, uint64_t q0, uint64_t nq,
                        int precision, uint32_t* idx, float* d2) {
     c.knn_stats = sc_knn_stats{};
